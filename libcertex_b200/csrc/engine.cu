@@ -4,8 +4,8 @@
 //   1 GROUPMAX pass of the tensor-core kernel over every `stride`-th stored row (the anchors, read in place through a
 //     strided TMA map)                                   -> gmax [nq, groups of 128 anchors]
 //   2 k-th largest group maximum                          -> thr [nq]   (k distinct rows are at least that close)
-//   3 SCREEN pass over all rows, keep iff acc >= thr      -> per-query candidate lists
-//   4 exact fp64 scores of the candidates + top-k by (score, id)
+//   3 SCREEN pass over all rows, keep iff acc >= thr      -> per-query candidate lists with the products
+//   4 the candidates ranked by their products, exact fp64 scores of those that can be among the k best, top-k by (score, id)
 // Queries whose candidate list overflowed, searches with a filter or labels, float / half indexes and small indexes
 // take the dense path: exact fp64 scores of all rows, then a radix selection. One stream synchronisation per search
 // call reads the overflow count.
@@ -103,11 +103,20 @@ struct ScreenShape {
   int n_stages;
 };
 
-ScreenShape shape_for(int kb)
+/// Shared memory of the resident-panel variant: panel_tiles * kb * 16 KB + n_stages * (kb * 32 KB + 1 KB) + the rest
+/// (screen_smem_bytes). The panel is what the call's query tiles split into evenly, at most 7 (kb = 1) or 2 (kb = 2) tiles;
+/// what it leaves goes to stages: a short panel is done with a stored tile soon, and the tiles in flight are what keeps
+/// the memory busy (one query over 1 M rows of 128 bytes: 27.6 us, 4.6 TB/s). Rows of more than two K blocks stream their K blocks
+/// (two query tiles per segment, stages fixed by the kernel).
+ScreenShape shape_for(int kb, int nqt)
 {
-  // shared memory: panel_tiles * kb * 16 KB + n_stages * (kb * 32 KB + 1 KB) + 9 KB must stay below 227 KB; rows of
-  // more than two K blocks stream their K blocks instead (two query tiles per segment, stages fixed by the kernel)
-  return kb == 1 ? ScreenShape{7, 3} : ScreenShape{2, 2};
+  if (kb > 2) { return ScreenShape{2, 2}; }
+  const int most     = kb == 1 ? 7 : 2;
+  const int n_panels = std::max(1, (nqt + most - 1) / most);
+  const int panel    = std::max(1, (nqt + n_panels - 1) / n_panels);
+  int stages         = 2;
+  while (stages < kMaxStages && screen_smem_bytes(kb, panel, stages + 1) <= kMaxSmem) { ++stages; }
+  return ScreenShape{panel, stages};
 }
 
 /// 3-D map (bytes of a row, column of a tile, tile) with free byte strides between columns and between tiles; box
@@ -715,26 +724,21 @@ void Index::search_dense(const Resources& res, const void* q, size_t qpitch, con
 void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32_t* thr, const void* queries,
                         size_t row_bytes, int q0, int nq, int k, double* best_s, int32_t* best_row, int32_t* ovf_list,
                         unsigned int* ovf_count, unsigned long long* stats, int* err, int64_t n, int32_t* thr2,
-                        const float* shift, const Admit& adm, std::vector<cudaEvent_t>* events) const
+                        const float* shift, const double* qq, const Admit& adm, std::vector<cudaEvent_t>* events) const
 {
   Scratch scratch(res.stream);
   const int grid          = res.sm_count;
-  const ScreenShape shape = shape_for(kb_);
   const int nqt           = static_cast<int>((nq + kQTile - 1) / kQTile);
+  const ScreenShape shape = shape_for(kb_, nqt);
   const int nt_all        = static_cast<int>((n + kTile - 1) / kTile);
   const uint32_t cap      = test_mode_ == 2 ? static_cast<uint32_t>(test_cap_) : static_cast<uint32_t>(std::max(2048, 2 * k));
-  // a record holds the survivors of one chain of 16 rows: as many records as candidate slots always suffice
-  const unsigned long long rec_cap = std::max<unsigned long long>(1ull << 20, static_cast<unsigned long long>(nq) * cap);
   uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(nq));
-  int32_t* cand        = scratch.get<int32_t>(static_cast<size_t>(nq) * cap);
-  uint64_t* rec        = scratch.get<uint64_t>(static_cast<size_t>(rec_cap));
-  auto* rec_count      = scratch.get<unsigned long long>(1);
+  Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(nq) * cap);
   const DevicePlan plan = device_plan(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
   auto* d_segs          = static_cast<ScreenSeg*>(plan.segs);
   int* d_seg_begin      = plan.begin;
   if (!d_segs) { upload_plan(scratch, plan_chunked(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_)), d_segs, d_seg_begin); }
   CERTEX_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * nq, res.stream));
-  CERTEX_CUDA(cudaMemsetAsync(rec_count, 0, sizeof(unsigned long long), res.stream));
   const size_t cp        = code_pitch_;
   const CUtensorMap tm_q = make_code_map(qcodes, cp, static_cast<uint64_t>(round_up(nq, kQTile)), cp, kQueryTile);
   const CUtensorMap tm_x = make_code_map(codes_, cp, static_cast<uint64_t>(n), cp, kBaseTile);
@@ -752,9 +756,9 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   a.init        = init_;
   a.cmax        = cmax_;
   a.thr         = thr;
-  a.rec         = rec;
-  a.rec_count   = rec_count;
-  a.rec_cap     = rec_cap;
+  a.cand        = cand;
+  a.cnt         = cnt;
+  a.cap         = cap;
   a.segs        = d_segs;
   a.seg_begin   = d_seg_begin;
   auto mark = [&] {
@@ -768,8 +772,6 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   mark();
   CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
   mark();
-  launch_expand_records(rec, rec_count, rec_cap, n, perm_, cnt, cand, cap, res.sm_count, res.stream);
-  CERTEX_CUDA(cudaGetLastError());
   Refine rf{};
   rf.thr2  = thr2;
   rf.thr   = thr;
@@ -778,22 +780,22 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   // 8-bit vectors kept in host memory: the exact stage reads the candidates' code rows, which are the vectors
   const bool from_codes = host_vectors_ && screen_kind_ == 1;
   launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, queries, row_bytes,
-                       nq, q0, cand, cnt, cap, k, adm, best_s, best_row, ovf_list, ovf_count, stats, rec_count, rec_cap, rf,
-                       res.stream, from_codes ? inv_ : nullptr, sqnorm_);
+                       nq, q0, Candidates{cand, cnt, cap, n, perm_, init_, shift, qq}, k, adm, best_s, best_row, ovf_list, ovf_count,
+                       stats, rf, res.stream, from_codes ? inv_ : nullptr, sqnorm_);
   CERTEX_CUDA(cudaGetLastError());
 }
 
-void Index::search_screened(const Resources& res, const uint8_t* qbuf, const float* shift, const void* queries,
+void Index::search_screened(const Resources& res, const uint8_t* qbuf, const float* shift, const double* qq, const void* queries,
                             size_t row_bytes, int q0, int nq, int k, double* best_s, int32_t* best_row, int32_t* ovf_list,
                             unsigned int* ovf_count, unsigned long long* stats, int* err, int anchor_stride, int64_t n,
                             int32_t* thr2, const Admit& adm, std::vector<cudaEvent_t>* events) const
 {
   // qbuf: the code rows of all queries of the call, zero padded to [round_up(total, 128), code_pitch_]; this batch is
-  // rows [q0, q0 + nq). shift (fp16 codes only): the rounding allowance of every query.
+  // rows [q0, q0 + nq). shift, qq (fp16 codes only): the rounding allowance and |q|^2 of every query.
   Scratch scratch(res.stream);
   const int grid          = res.sm_count;
-  const ScreenShape shape = shape_for(kb_);
   const int nqt           = static_cast<int>((nq + kQTile - 1) / kQTile);
+  const ScreenShape shape = shape_for(kb_, nqt);
   // anchors: sorted rows 0, stride, 2 stride, ...; only whole tiles of 256 anchors take part
   const int nt_anchor     = static_cast<int>(n / (static_cast<int64_t>(anchor_stride) * kTile));
   const int n_groups      = nt_anchor * (kBaseTile / kGroupRows);
@@ -876,7 +878,7 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
   if (screen_kind_ == 2) { launch_finish_thr_f16(thr, shift + q0, nq, 1, res.stream); }
   CERTEX_CUDA(cudaGetLastError());
   // 3 screen over all rows, 4 exact scores of the candidates and the k best
-  screen_pass(res, qb, thr, queries, row_bytes, q0, nq, k, best_s, best_row, ovf_list, ovf_count, stats, err, n, thr2, shift,
+  screen_pass(res, qb, thr, queries, row_bytes, q0, nq, k, best_s, best_row, ovf_list, ovf_count, stats, err, n, thr2, shift, qq,
               adm, events);
 }
 
@@ -1008,7 +1010,9 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
       ++r1;
     }
     const int grid          = res.sm_count;
-    const ScreenShape shape = shape_for(kb_);
+    int most_qt             = 1;  // query tiles of the label with the most queries
+    for (size_t r = r0; r < r1; ++r) { most_qt = std::max(most_qt, static_cast<int>((routed[r].queries.size() + kQTile - 1) / kQTile)); }
+    const ScreenShape shape = shape_for(kb_, most_qt);
     std::vector<ScreenSeg> segs;
     std::vector<int> col0, seg_begin;
     r1 = r0 + plan_routed(routed, r0, r1, q_tile0, shape.panel_tiles, grid, 64, segs, col0, seg_begin);
@@ -1063,7 +1067,6 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     const size_t cp      = code_pitch_;
     const int n_groups   = static_cast<int>(max_tiles) * per_tile;
     const int64_t ld_g   = round_up(n_groups, 8);
-    const unsigned long long rec_cap = std::max<unsigned long long>(1ull << 20, static_cast<unsigned long long>(ns) * cap);
     // the host's tables of the pass, sent in one copy (segs_g ...: the threshold pass over the leading tiles of every label)
     const std::vector<std::pair<const void*, size_t>> tables = {
       {slot_query.data(), slot_query.size() * 4},      {slot_ng.data(), slot_ng.size() * 4},
@@ -1086,19 +1089,17 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     uint8_t* q_rows      = scratch.get<uint8_t>(static_cast<size_t>(ns) * (f16 ? qpitch : cp));  // the queries in slot order
     uint8_t* q_codes     = f16 ? scratch.get<uint8_t>(static_cast<size_t>(ns) * cp) : q_rows;
     float* shift         = f16 ? scratch.get<float>(static_cast<size_t>(ns)) : nullptr;
+    double* qq           = f16 && params_.metric != kL2 ? scratch.get<double>(static_cast<size_t>(ns)) : nullptr;
     int32_t* gmax        = scratch.get<int32_t>(static_cast<size_t>(ns) * ld_g);
     int32_t* thr         = scratch.get<int32_t>(static_cast<size_t>(ns));
     uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(ns));
-    int32_t* cand        = scratch.get<int32_t>(static_cast<size_t>(ns) * cap);
-    uint64_t* rec        = scratch.get<uint64_t>(static_cast<size_t>(rec_cap));
-    auto* rec_count      = scratch.get<unsigned long long>(1);
+    Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(ns) * cap);
     double* slot_s       = scratch.get<double>(static_cast<size_t>(ns) * k);
     int32_t* slot_row    = scratch.get<int32_t>(static_cast<size_t>(ns) * k);
     int32_t* ovf_list    = scratch.get<int32_t>(static_cast<size_t>(ns));
     unsigned int* d_flag = scratch.get<unsigned int>(4);  // [0] overflowed slots, [1] error code, [2] fp16 overflow
     auto* d_stats        = scratch.get<unsigned long long>(2);
     CERTEX_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * ns, res.stream));
-    CERTEX_CUDA(cudaMemsetAsync(rec_count, 0, sizeof(unsigned long long), res.stream));
     CERTEX_CUDA(cudaMemsetAsync(d_flag, 0, 4 * sizeof(unsigned int), res.stream));
     CERTEX_CUDA(cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned long long), res.stream));
     // queries in slot order (8-bit vectors: zero padded to code rows, which the verification reads as well)
@@ -1107,6 +1108,7 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     if (f16) {
       launch_encode_f16_queries(q_rows, qpitch, dtype_, static_cast<int>(dim_), ns, q_codes, cp, n1max_, n2max_, emax_, shift,
                                 d_flag + 2, res.stream);
+      if (qq) { launch_query_sqnorms(q_rows, qpitch, dtype_, static_cast<int>(dim_), ns, qq, res.stream); }
     }
     CERTEX_CUDA(cudaGetLastError());
     const CUtensorMap tm_q = make_code_map(q_codes, cp, static_cast<uint64_t>(ns), cp, kQueryTile);
@@ -1159,22 +1161,21 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     a.seg_step  = nullptr;
     a.cmax      = lcmax_;
     a.thr       = thr;
-    a.rec       = rec;
-    a.rec_count = rec_count;
-    a.rec_cap   = rec_cap;
+    a.cand      = cand;
+    a.cnt       = cnt;
+    a.cap       = cap;
     mark();
     CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
     mark();
-    launch_expand_records(rec, rec_count, rec_cap, n_lrows_, lperm_, cnt, cand, cap, res.sm_count, res.stream);
     Admit plain{};
     plain.removed = removed_;
     const bool from_codes = host_vectors_ && screen_kind_ == 1;
     launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, q_rows,
-                         q_rows_pitch, ns, 0, cand, cnt, cap, k, plain, slot_s, slot_row, ovf_list, d_flag, d_stats, rec_count,
-                         rec_cap, Refine{}, res.stream, from_codes ? inv_ : nullptr, sqnorm_);
+                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, n_lrows_, lperm_, linit_, shift, qq}, k, plain, slot_s, slot_row,
+                         ovf_list, d_flag, d_stats, Refine{}, res.stream, from_codes ? inv_ : nullptr, sqnorm_);
     launch_scatter_best(slot_s, slot_row, d_slot_q, ns, k, best_s, best_row, res.stream);
     CERTEX_CUDA(cudaGetLastError());
-    st->launches += f16 ? 10 : 8;
+    st->launches += f16 ? (qq ? 10 : 9) : 7;
     unsigned int h_flag[4]        = {0, 0, 0, 0};
     unsigned long long h_stats[2] = {0, 0};
     std::vector<int32_t> h_ovf;
@@ -1197,7 +1198,8 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     for (cudaEvent_t e : events) { cudaEventDestroy(e); }
     CERTEX_EXPECTS(h_flag[1] == 0, "certex: the screening pass gave up on a wait (code " + std::to_string(h_flag[1]) + ")");
     st->routed_queries += static_cast<unsigned long long>(ns);
-    pairs += h_stats[0];  // pairs the routed screen kept and the verification scored
+    pairs += h_stats[0];  // pairs the routed screen kept
+    st->verified += h_stats[1];
     // slots whose list overflowed (every real slot, when a query coordinate did not fit fp16) go to the dense groups
     std::vector<char> again(static_cast<size_t>(ns), h_flag[2] != 0 ? 1 : 0);
     for (unsigned int i = 0; i < h_flag[0] && i < static_cast<unsigned int>(ns); ++i) { again[static_cast<size_t>(h_ovf[i])] = 1; }
@@ -1338,6 +1340,7 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
       wave_blocks += grouped_blocks(nqg, n_cols);
       wave_max_cols = std::max(wave_max_cols, n_cols);
       pairs += static_cast<unsigned long long>(nqg) * static_cast<unsigned long long>(n_cols);
+      st->verified += static_cast<unsigned long long>(nqg) * static_cast<unsigned long long>(n_cols);
       a += nqg;
     }
     i = j;
@@ -1388,6 +1391,7 @@ struct Index::Pending {
   bool screened     = false;  // the tensor-core screen ran: the counters decide whether the outputs stand
   uint8_t* qbuf     = nullptr;
   float* shift      = nullptr;
+  double* qq        = nullptr;
   unsigned int* q_ovf = nullptr;
   int32_t* ovf_list = nullptr;
   int32_t* thr2     = nullptr;
@@ -1460,7 +1464,6 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
   local.queries      = static_cast<unsigned long long>(nq);
   if (filter.query_labels && !filter.words && n_part_ > 0 && test_mode_ != 1) {
     local.survivors = search_by_labels(res, queries, row_bytes, static_cast<int>(nq), k, adm, best_s, best_row, n, &local);
-    local.verified  = local.survivors;
   } else if (screened) {
     P.screened           = true;
     const int64_t nq_pad = round_up(nq, kQTile);
@@ -1478,8 +1481,10 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
     CERTEX_CUDA(cudaMemsetAsync(counters, 0, sizeof(HostCounters), res.stream));
     if (screen_kind_ == 2) {
       shift = scratch.get<float>(static_cast<size_t>(nq));
+      P.qq  = params_.metric != kL2 ? scratch.get<double>(static_cast<size_t>(nq)) : nullptr;
       CERTEX_CUDA(cudaMemsetAsync(qbuf + static_cast<size_t>(nq) * code_pitch_, 0, static_cast<size_t>(nq_pad - nq) * code_pitch_, res.stream));
       launch_encode_f16_queries(queries, row_bytes, dtype_, d, nq, qbuf, code_pitch_, n1max_, n2max_, emax_, shift, q_ovf, res.stream);
+      if (P.qq) { launch_query_sqnorms(queries, row_bytes, dtype_, d, nq, P.qq, res.stream); }
       CERTEX_CUDA(cudaGetLastError());
     } else {
       if (row_bytes != code_pitch_ || nq_pad != nq) {
@@ -1494,9 +1499,9 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
     P.d_stats = d_stats, P.batch = batch;
     for (int64_t q0 = 0; q0 < nq; q0 += batch) {
       const int nb = static_cast<int>(std::min<int64_t>(batch, nq - q0));
-      search_screened(res, qbuf, shift, queries, row_bytes, static_cast<int>(q0), nb, k, best_s, best_row, ovf_list, d_count,
+      search_screened(res, qbuf, shift, P.qq, queries, row_bytes, static_cast<int>(q0), nb, k, best_s, best_row, ovf_list, d_count,
                       d_stats, reinterpret_cast<int*>(d_count + 1), stride, n, thr2, adm, stats_sink ? &P.events : nullptr);
-      local.launches += screen_kind_ == 2 ? 7 : 6;  // gather_init, GROUPMAX, kth_largest (+ thresholds), SCREEN, expand, verify
+      local.launches += screen_kind_ == 2 ? 6 : 5;  // gather_init, GROUPMAX, kth_largest (+ thresholds), SCREEN, verify
     }
     // The outputs are written now, as if no list had overflowed; the counters follow them to the host and search_end
     // looks at them once the caller has enqueued what it wanted behind the search.
@@ -1580,19 +1585,23 @@ bool Index::search_end(Pending* raw, bool refinish) const
       uint8_t* qcodes2       = scratch.get<uint8_t>(static_cast<size_t>(pad) * code_pitch_);
       uint8_t* queries2      = scratch.get<uint8_t>(static_cast<size_t>(n_ovf) * P.row_bytes);
       float* shift2          = scratch.get<float>(static_cast<size_t>(n_ovf));
+      double* qq2            = scratch.get<double>(static_cast<size_t>(n_ovf));
       double* best2_s        = scratch.get<double>(static_cast<size_t>(n_ovf) * k);
       int32_t* best2_row     = scratch.get<int32_t>(static_cast<size_t>(n_ovf) * k);
       int32_t* ovf2          = scratch.get<int32_t>(static_cast<size_t>(n_ovf));
       launch_gather_rows(P.qbuf, code_pitch_, P.ovf_list, n_ovf, pad, qcodes2, code_pitch_, code_pitch_, res.stream);
       launch_gather_rows(P.queries, P.row_bytes, P.ovf_list, n_ovf, n_ovf, queries2, P.row_bytes, P.row_bytes, res.stream);
-      if (P.shift) { launch_gather_rows(P.shift, 4, P.ovf_list, n_ovf, n_ovf, shift2, 4, 4, res.stream); }
+      if (P.shift) {
+        launch_gather_rows(P.shift, 4, P.ovf_list, n_ovf, n_ovf, shift2, 4, 4, res.stream);
+        if (P.qq) { launch_gather_rows(P.qq, 8, P.ovf_list, n_ovf, n_ovf, qq2, 8, 8, res.stream); }
+      }
       CERTEX_CUDA(cudaGetLastError());
       for (int b0 = 0; b0 < n_ovf; b0 += static_cast<int>(P.batch)) {
         const int nb = std::min<int>(static_cast<int>(P.batch), n_ovf - b0);
         screen_pass(res, qcodes2 + static_cast<size_t>(b0) * code_pitch_, P.thr2 + b0, queries2, P.row_bytes, b0, nb, k, best2_s,
                     best2_row, ovf2, P.d_count + 2, P.d_stats, reinterpret_cast<int*>(P.d_count + 1), n, nullptr,
-                    P.shift ? shift2 : nullptr, P.adm, stats_sink ? &P.events : nullptr);
-        local.launches += 3;
+                    P.shift ? shift2 : nullptr, P.qq ? qq2 : nullptr, P.adm, stats_sink ? &P.events : nullptr);
+        local.launches += 2;
       }
       launch_scatter_best(best2_s, best2_row, P.ovf_list, n_ovf, k, P.best_s, P.best_row, res.stream);
       launch_compose(ovf2, P.d_count + 2, n_ovf, P.ovf_list, res.stream);
@@ -1869,7 +1878,8 @@ std::unique_ptr<Index> Index::from_blocks(const Resources& res, const IndexParam
     CERTEX_CUDA(cudaMemcpyAsync(idx->removed_, host.data(), static_cast<size_t>(n), cudaMemcpyHostToDevice, res.stream));
     res.sync();
     idx->n_removed_ = n_rem;
-    if (idx->screen_kind_ && n_rem > 0) {  // removed rows must never pass the screen
+    if (idx->screen_kind_ && std::any_of(host.begin(), host.begin() + n, [](char f) { return f != 0; })) {
+      // removed rows must never pass the screen
       Scratch scratch(res.stream);
       int64_t* ids     = scratch.get<int64_t>(static_cast<size_t>(n));
       auto* counter    = scratch.get<unsigned long long>(1);
@@ -1991,9 +2001,9 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   const bool is_signed = code_kind == 1, f16 = code_kind == 2;
   Scratch scratch(res.stream);
   const int kb            = static_cast<int>(code_len / 128);
-  const ScreenShape shape = shape_for(kb);
   const int grid          = res.sm_count;
   const int nqt           = static_cast<int>((nq + kQTile - 1) / kQTile);
+  const ScreenShape shape = shape_for(kb, nqt);
   const int nt            = static_cast<int>((n + kTile - 1) / kTile);
   const ChunkedPlan plan  = plan_chunked(nqt, nt, shape.panel_tiles, grid, chunk_tiles_for(static_cast<size_t>(code_len)));
   ScreenSeg* d_segs       = scratch.get<ScreenSeg>(plan.segs.size());
@@ -2042,19 +2052,21 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
     launch_chain_max(init_pad, 0, n_pad / kChainRows, cmax, f16, res.stream);
   }
   CERTEX_CUDA(cudaGetLastError());
-  const unsigned long long rec_cap = std::max<unsigned long long>(1ull << 20, static_cast<unsigned long long>(nq) * 1024ull);
-  uint64_t* rec   = scratch.get<uint64_t>(static_cast<size_t>(rec_cap));
-  auto* rec_count = scratch.get<unsigned long long>(1);
-  CERTEX_CUDA(cudaMemsetAsync(rec_count, 0, sizeof(unsigned long long), res.stream));
+  // lists of chains, which become the caller's lists of rows
+  const uint32_t n_chains  = static_cast<uint32_t>((n + kChainRows - 1) / kChainRows);
+  const uint32_t chain_cap = mode == kModeScreen ? std::min(std::max<uint32_t>(cap, 2048), n_chains) : 0;
+  Candidate* chains        = scratch.get<Candidate>(static_cast<size_t>(nq) * chain_cap);
+  uint32_t* chain_cnt      = scratch.get<uint32_t>(static_cast<size_t>(nq));
+  CERTEX_CUDA(cudaMemsetAsync(chain_cnt, 0, static_cast<size_t>(nq) * 4, res.stream));
   ScreenArgs a{};
   a.init        = init_pad;
   a.cmax        = cmax;
   a.thr         = thr;
   a.gmax        = gmax;
   a.ld_gmax     = ld;
-  a.rec         = rec;
-  a.rec_count   = rec_count;
-  a.rec_cap     = rec_cap;
+  a.cand        = chains;
+  a.cnt         = chain_cnt;
+  a.cap         = chain_cap;
   a.nq          = static_cast<int>(nq);
   a.kb          = kb;
   a.panel_tiles = shape.panel_tiles;
@@ -2074,12 +2086,12 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   const cudaError_t le = screen_i8_launch(tm_q, tm_x, a, grid, res.stream);
   CERTEX_CUDA(cudaEventRecord(e1, res.stream));
   if (mode == kModeScreen && le == cudaSuccess) {
-    launch_expand_records(rec, rec_count, rec_cap, n, nullptr, cnt, cand, cap, res.sm_count, res.stream);
+    launch_candidate_rows(chains, chain_cnt, chain_cap, static_cast<int>(nq), n, cnt, cand, cap, res.stream);
   }
-  int h_err                  = 0;
-  unsigned long long h_count = 0;
+  int h_err = 0;
+  std::vector<uint32_t> h_cnt(static_cast<size_t>(nq), 0u);
   CERTEX_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, res.stream));
-  CERTEX_CUDA(cudaMemcpyAsync(&h_count, rec_count, sizeof(h_count), cudaMemcpyDeviceToHost, res.stream));
+  CERTEX_CUDA(cudaMemcpyAsync(h_cnt.data(), chain_cnt, h_cnt.size() * 4, cudaMemcpyDeviceToHost, res.stream));
   const cudaError_t se = cudaStreamSynchronize(res.stream);
   float ms             = 0;
   if (se == cudaSuccess) { cudaEventElapsedTime(&ms, e0, e1); }
@@ -2088,7 +2100,10 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   CERTEX_CUDA(le);
   CERTEX_CUDA(se);
   CERTEX_EXPECTS(h_err == 0, "certex: the screening pass gave up on a wait (code " + std::to_string(h_err) + ")");
-  CERTEX_EXPECTS(h_count <= rec_cap, "certex: the survivor record buffer overflowed");
+  if (mode == kModeScreen) {
+    const uint32_t most = *std::max_element(h_cnt.begin(), h_cnt.end());
+    CERTEX_EXPECTS(most <= chain_cap, "certex: a list of kept chains overflowed");
+  }
   if (elapsed_ms) { *elapsed_ms = ms; }
 }
 

@@ -593,6 +593,41 @@ __global__ void encode_f16_queries_kernel(const uint8_t* queries, size_t qpitch,
   }
 }
 
+// qq[q] = |q|^2 in the order of the exact scores (coordinate 0 to d - 1, every operation rounded on its own): a chain of d
+// dependent additions per query. Made by one thread of the verification it kept a whole block waiting; here 32 queries share
+// a warp, their coordinates come through shared memory in pieces of 32, and the chains run side by side.
+template <typename T>
+__global__ void __launch_bounds__(32) query_sqnorm_kernel(const uint8_t* queries, size_t qpitch, int d, int64_t nq, double* qq)
+{
+  __shared__ float tile[32][33];
+  const int lane   = threadIdx.x;
+  const int64_t q0 = static_cast<int64_t>(blockIdx.x) * 32;
+  const int n      = static_cast<int>(min(static_cast<int64_t>(32), nq - q0));
+  double a         = 0;
+  float next[32];  // the piece after this one, on its way while this one is summed
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const T* row = reinterpret_cast<const T*>(queries + static_cast<size_t>(q0 + i) * qpitch);
+      next[i]      = i < n && t + lane < d ? static_cast<float>(row[t + lane]) : 0.f;
+    }
+  };
+  fetch(0);
+  for (int t0 = 0; t0 < d; t0 += 32) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) { tile[i][lane] = next[i]; }
+    __syncwarp();
+    if (t0 + 32 < d) { fetch(t0 + 32); }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {  // beyond the last coordinate zeros are added, which leave the sum as it is
+      const double v = static_cast<double>(tile[lane][i]);
+      a              = __dadd_rn(a, __dmul_rn(v, v));
+    }
+  }
+  if (lane < n) { qq[q0 + lane] = a; }
+}
+
 // fp16 codes, in two steps around the optional exchange of thresholds between shards. Step 0: thr[q] = the key of the
 // k-th largest group maximum (see float_key in the screen kernel) -> the key of value - shift[q] / 2, a score that k
 // rows of this index certainly reach in exact arithmetic. Step 1: such a key -> float bits of the screen's
@@ -617,24 +652,18 @@ __global__ void chain_max_f32_kernel(const float* init, int64_t c0, int64_t n, f
   cmax[c0 + i] = m;
 }
 
-// Survivor records -> per-query candidate lists. One thread per record; the appends of a query go through cnt[q].
-__global__ void expand_records_kernel(const uint64_t* rec, const unsigned long long* rec_count, unsigned long long rec_cap,
-                                      int64_t n_rows, const int32_t* perm, uint32_t* cnt, int32_t* cand, uint32_t cap)
+// The rows of candidate lists, one thread per chain.
+__global__ void candidate_rows_kernel(const Candidate* cand, const uint32_t* cnt, uint32_t cap, int64_t n_rows,
+                                      uint32_t* row_cnt, int32_t* rows, uint32_t row_cap)
 {
-  const unsigned long long n = min(*rec_count, rec_cap);
-  for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-    const uint64_t r     = rec[i];
-    const uint32_t q     = static_cast<uint32_t>(r >> 48);
-    const int64_t row0   = static_cast<int64_t>((r >> 16) & 0xffffffffull) * 16;
-    uint32_t mask        = static_cast<uint32_t>(r & 0xffffu);
-    while (mask) {
-      const int b = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int32_t id = row0 + b < n_rows ? (perm ? perm[row0 + b] : static_cast<int32_t>(row0 + b)) : -1;
-      if (id >= 0) {  // rows beyond the last one and padding rows of a label's block have no id
-        const uint32_t pos = atomicAdd(cnt + q, 1u);
-        if (pos < cap) { cand[static_cast<size_t>(q) * cap + pos] = id; }
+  const uint32_t n = min(cnt[blockIdx.x], cap);
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const Candidate c = cand[static_cast<size_t>(blockIdx.x) * cap + i];
+    for (uint32_t mask = c.mask; mask; mask &= mask - 1) {
+      const int64_t r = static_cast<int64_t>(c.chain) * kChainRows + __ffs(mask) - 1;
+      if (r < n_rows) {
+        const uint32_t at = atomicAdd(row_cnt + blockIdx.x, 1u);
+        if (at < row_cap) { rows[static_cast<size_t>(blockIdx.x) * row_cap + at] = static_cast<int32_t>(r); }
       }
     }
   }
@@ -935,51 +964,158 @@ __device__ __forceinline__ void int_row_scores(const uint8_t* vectors, size_t pi
   }
 }
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
+// Every thread of the block: the k-th largest of n keys in shared memory, 1 <= k <= number of keys that are not 0 (0: no
+// key). Up to 512 keys: one warp holds them in registers and finds the largest threshold that k of them reach bit by bit,
+// without a step of the whole block in between. More: a most-significant-digit radix walk that starts at the highest byte in
+// which the keys differ. `scratch`: 260 words.
+__device__ uint32_t block_kth_largest(const uint32_t* key, int n, int k, uint32_t* scratch)
 {
+  const int n_threads = blockDim.x;
+  constexpr int kHeld = 16;
+  if (n <= 32 * kHeld) {
+    if (threadIdx.x < 32) {
+      uint32_t u[kHeld];
+      uint32_t hi = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long other = __shfl_xor_sync(0xffffffffu, v, o);
-    v                              = other < v ? other : v;
+      for (int i = 0; i < kHeld; ++i) {
+        const int at = threadIdx.x + i * 32;
+        u[i]         = at < n ? key[at] : 0u;
+        hi           = max(hi, u[i]);
+      }
+      hi         = __reduce_max_sync(0xffffffffu, hi);
+      uint32_t t = 0;
+      bool exact = false;
+      for (int bit = 31 - __clz(hi); bit >= 0 && !exact; --bit) {
+        const uint32_t next = t | (1u << bit);
+        int reach           = 0;
+#pragma unroll
+        for (int i = 0; i < kHeld; ++i) { reach += u[i] >= next ? 1 : 0; }
+        reach = __reduce_add_sync(0xffffffffu, reach);
+        if (reach >= k) { t = next; }
+        exact = reach == k;
+      }
+      uint32_t least = 0xffffffffu;  // the smallest key that reaches t
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) { least = u[i] >= t && u[i] != 0u ? min(least, u[i]) : least; }
+      least = __reduce_min_sync(0xffffffffu, least);
+      if (threadIdx.x == 0) { scratch[256] = least; }
+    }
+    __syncthreads();
+    return scratch[256];
   }
-  return v;
+  uint32_t lo = 0xffffffffu, hi = 0u;
+  for (int i = threadIdx.x; i < n; i += n_threads) {
+    const uint32_t v = key[i];
+    if (v != 0u) { lo = min(lo, v), hi = max(hi, v); }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (threadIdx.x == 0) { scratch[257] = 0xffffffffu, scratch[258] = 0u; }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(scratch + 257, lo);
+    atomicMax(scratch + 258, hi);
+  }
+  __syncthreads();
+  const uint32_t base  = scratch[257];
+  const uint32_t range = scratch[258] - base;
+  const int top        = range == 0u ? 0 : 32 - __clz(range);
+  uint32_t prefix = 0, mask = 0, remaining = static_cast<uint32_t>(k);
+  for (int shift = ((top + 7) / 8 - 1) * 8; shift >= 0; shift -= 8) {
+    for (int i = threadIdx.x; i < 256; i += n_threads) { scratch[i] = 0; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += n_threads) {
+      const uint32_t v = key[i];
+      if (v != 0u && ((v - base) & mask) == prefix) { atomicAdd(&scratch[((v - base) >> shift) & 255u], 1u); }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int lane = threadIdx.x;
+      uint32_t c[8], sum = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        c[i] = scratch[255 - (lane * 8 + i)];
+        sum += c[i];
+      }
+      uint32_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) { incl += v; }
+      }
+      const uint32_t before = incl - sum;
+      if (before < remaining && incl >= remaining) {
+        uint32_t cum = before;
+        int i        = 0;
+        for (; i < 7; ++i) {
+          if (cum + c[i] >= remaining) { break; }
+          cum += c[i];
+        }
+        scratch[257] = prefix | (static_cast<uint32_t>(255 - (lane * 8 + i)) << shift);
+        scratch[258] = remaining - cum;
+      }
+    }
+    __syncthreads();
+    prefix    = scratch[257];
+    remaining = scratch[258];
+    mask |= 0xffu << shift;
+  }
+  __syncthreads();
+  return prefix + base;
 }
 
-// The k smallest of n2 distinct 64-bit keys in shared memory (~0 = none), ascending into out [k], for small k and a
-// block of at most kSelectWarps warps: every warp draws the k smallest of its share of the keys by k rounds of a warp
-// minimum, then the first warp draws the k smallest of those lists the same way. No key moves in shared memory.
-constexpr int kSelectWarps = 4;
-constexpr int kSelectMaxK  = 32;
-__device__ void select_smallest_keys(const unsigned long long* key, int n2, int k, unsigned long long* lists,
-                                     unsigned long long* out)
+// Sorts m entries in shared memory by (score, id), ascending, in place. Up to one entry per thread: every entry's place
+// is the number of entries before it (the ids are distinct); more: bitonic, the tail up to next_pow2(m) filled up.
+template <typename IdT>
+__device__ void sort_pairs(double* s, IdT* id, int m)
 {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  unsigned long long lo = 0;  // keys below lo are taken already
-  for (int r = 0; r < k; ++r) {
-    unsigned long long best = ~0ull;
-    for (int j = warp * 32 + lane; j < n2; j += n_warps * 32) {
-      const unsigned long long v = key[j];
-      if (v >= lo && v < best) { best = v; }
-    }
-    best = warp_min_u64(best);
-    if (lane == 0) { lists[warp * kSelectMaxK + r] = best; }
-    lo = best == ~0ull ? best : best + 1;
-  }
   __syncthreads();
-  if (warp == 0) {
-    lo = 0;
-    for (int r = 0; r < k; ++r) {
-      unsigned long long best = ~0ull;
-      for (int j = lane; j < n_warps * kSelectMaxK; j += 32) {
-        const unsigned long long v = (j % kSelectMaxK) < k ? lists[j] : ~0ull;
-        if (v >= lo && v < best) { best = v; }
-      }
-      best = warp_min_u64(best);
-      if (lane == 0) { out[r] = best; }
-      lo = best == ~0ull ? best : best + 1;
+  if (m <= static_cast<int>(blockDim.x)) {
+    double x = 0;
+    IdT xi   = 0;
+    int place = 0;
+    const bool mine = static_cast<int>(threadIdx.x) < m;
+    if (mine) {
+      x  = s[threadIdx.x];
+      xi = id[threadIdx.x];
+      for (int j = 0; j < m; ++j) { place += pair_less(s[j], id[j], x, xi) ? 1 : 0; }
     }
+    __syncthreads();
+    if (mine) {
+      s[place]  = x;
+      id[place] = xi;
+    }
+    __syncthreads();
+    return;
   }
+  const int n2 = next_pow2(m);
+  for (int i = m + threadIdx.x; i < n2; i += blockDim.x) {
+    s[i]  = CUDART_INF;
+    id[i] = static_cast<IdT>(0x7fffffff);
+  }
+  bitonic_sort(s, id, n2);
+}
+
+// The same for distinct 64-bit keys.
+__device__ void sort_keys(unsigned long long* key, int m)
+{
   __syncthreads();
+  if (m <= static_cast<int>(blockDim.x)) {
+    unsigned long long x = 0;
+    int place            = 0;
+    const bool mine      = static_cast<int>(threadIdx.x) < m;
+    if (mine) {
+      x = key[threadIdx.x];
+      for (int j = 0; j < m; ++j) { place += key[j] < x ? 1 : 0; }
+    }
+    __syncthreads();
+    if (mine) { key[place] = x; }
+    __syncthreads();
+    return;
+  }
+  const int n2 = next_pow2(m);
+  for (int i = m + threadIdx.x; i < n2; i += blockDim.x) { key[i] = ~0ull; }
+  bitonic_sort_keys(key, n2);
 }
 
 // ------------------------------------------------------------------------------------------- stored |x|^2 (cosine)
@@ -1034,66 +1170,159 @@ __device__ __forceinline__ uint8_t* stage_of(void* after_the_arrays)
 {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(after_the_arrays) + 15) & ~static_cast<uintptr_t>(15));
 }
-// Dynamic shared memory: qd [d] doubles | sc [n2] doubles | id [n2] int32, n2 = next_pow2(cap); for 8-bit rows
-// the query's bytes (in the space of qd) | n2 64-bit keys.
-// Blocks of 128 threads for 8-bit rows (64 registers: 8 blocks per SM), of 256 threads for float rows (80 registers,
-// which the fetch of the next slab during the walk of this one needs: 3 blocks per SM, as many as the shared memory allows).
+// Block per query. A candidate chain comes with its largest product, so the candidates are ranked before a vector is read.
+// With value = product + e of the row (what the thresholds are made of), a chain whose kept rows may all be returned has a
+// row of value >= product + the smallest e of them; a row of it has a value <= product + its own e (the same number when
+// the chain kept one row, as nearly all do). Let v_k be the k-th largest of the former over the chains (rows of k
+// different chains reach it). Only rows whose latter can still belong to the k nearest are scored in fp64:
+//   8-bit vectors  those >= v_k. Values are exact but for the bit that e = -floor(|x|^2 / 2) drops: 2 value - 1 or 2 value
+//                  is the exact term, and twice a value below v_k lies below 2 v_k - 1, which k rows reach.
+//   fp16 codes     those >= v_k - shift, shift = twice the most a value may be off (see encode_f16_queries_kernel): k rows
+//                  certainly reach v_k - shift / 2, and a row that does has a value of at least v_k - shift.
+// Reading and scoring rows is what bounds the kernel (d coordinates of a gathered row per candidate, each with two or
+// three fp64 operations), and the screen keeps several times k candidates; after the ranking about k are left:
+// 10 000 queries, k = 100, 1 M x 768 float coordinates: 220 of 619 rows, 5.96 -> 2.27 ms; 777 queries, k = 33, 1.2 M x 100
+// bytes with a bitset: 34 of 1017 rows, 138 + 67 us (the launch that made lists of rows) -> 64 us; 1000 queries, k = 10,
+// 100 000 x 128 floats: 14 of 209 rows, 69 + 12 -> 25 us.
+// Dynamic shared memory: the query (doubles, or bytes) | sc [n2] doubles | id [n2] int32, n2 = next_pow2(cap); for 8-bit
+// rows n2 64-bit keys in place of sc. Before the scores are made the space of sc holds the rows' values and ids, and the
+// space of id what the chains reach.
 template <typename T>
 constexpr bool kByteRows = std::is_same<T, int8_t>::value || std::is_same<T, uint8_t>::value;
 template <typename T, int METRIC, bool STORED_XX = false>
 __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 3) verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* queries, size_t qpitch,
-                                     int q0, const int32_t* cand, const uint32_t* cnt, uint32_t cap, int n2max, int k,
+                                     int q0, Candidates cd, int n2max, int k,
                                      Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list,
-                                     unsigned int* ovf_count, unsigned long long* stats,
-                                     const unsigned long long* rec_count, unsigned long long rec_cap, Refine rf,
+                                     unsigned int* ovf_count, unsigned long long* stats, Refine rf,
                                      const int32_t* where, const double* sqnorm)
 {
   extern __shared__ double sh[];
   __shared__ double s_qq;
-  const int q       = q0 + blockIdx.x;  // number of the query in the call; cand / cnt are those of its batch
-  const uint32_t c0 = cnt[blockIdx.x];
-  // a candidate list that overflowed, or a survivor record buffer that did (then no list of the batch is complete):
-  // the query is reported in ovf_list. What its list holds are still rows at or above its threshold, and the k-th best
-  // exact score among them bounds the k-th neighbour: a tighter threshold for a second pass (rf).
-  const bool over   = c0 > cap || (rec_count && *rec_count > rec_cap);
-  if (over && rf.thr2 == nullptr) {
+  __shared__ uint32_t s_scratch[260];
+  __shared__ int s_rows, s_sure, s_seen, s_kept;
+  constexpr bool kBytes = kByteRows<T>;
+  const int q           = q0 + blockIdx.x;  // number of the query in the call; the candidates are those of its batch
+  const uint32_t c0     = cd.cnt[blockIdx.x];
+  // A candidate list that overflowed (or more rows in it than the block holds): the query is reported in ovf_list. What the
+  // block has are still rows at or above the query's threshold, and the k-th best exact score among them bounds the k-th
+  // neighbour: a tighter threshold for a second pass (rf).
+  const bool listed_all = c0 <= cd.cap;
+  if (!listed_all && rf.thr2 == nullptr) {
     if (threadIdx.x == 0) { ovf_list[atomicAdd(ovf_count, 1u)] = q; }
     return;
   }
-  const uint32_t c = min(c0, cap);
+  const int c  = static_cast<int>(min(c0, cd.cap));
   double* qd   = sh;
-  double* sc   = sh + d;
+  double* sc   = kBytes ? sh + (d + 15) / 16 * 2 : sh + d;
   int32_t* ids = reinterpret_cast<int32_t*>(sc + n2max);
-  const int64_t qi = q;
-  constexpr bool kBytes = std::is_same<T, int8_t>::value || std::is_same<T, uint8_t>::value;
+  if (c == 0) {  // no candidate (a slot without a query, or nothing that the query may return)
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+      best_s[static_cast<size_t>(q) * k + t]   = CUDART_INF;
+      best_row[static_cast<size_t>(q) * k + t] = -1;
+    }
+    return;
+  }
   __shared__ long long s_qq_int;
+  if (threadIdx.x == 0) { s_rows = 0, s_sure = 0, s_seen = 0, s_kept = 0; }
   if constexpr (kBytes) {
     // the query's bytes, zero padded to whole 16-byte vectors, in the space of qd; |q|^2 as an integer
     uint8_t* qbytes    = reinterpret_cast<uint8_t*>(qd);
     const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
     const int padded   = (d + 15) / 16 * 16;
     for (int t = threadIdx.x; t < padded; t += blockDim.x) { qbytes[t] = t < d ? src[t] : 0; }
-    __syncthreads();
+  } else {
+    // the query as doubles; |q|^2 in coordinate order comes with the query's code, where the metric has a use for it
+    const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
+    for (int t = threadIdx.x; t < d; t += blockDim.x) { qd[t] = Elems<T>::one(src, t); }
+    if (threadIdx.x == 0) { s_qq = METRIC == kL2 ? 0.0 : cd.qq[q]; }
+  }
+  __syncthreads();
+  if constexpr (kBytes) {
     if (threadIdx.x < 32) {  // |q|^2: 255^2 * 4096 < 2^31
-      int a = 0;
-      for (int t = threadIdx.x; t < padded / 4; t += 32) {
-        const uint32_t w = reinterpret_cast<const uint32_t*>(qbytes)[t];
+      const uint32_t* qw = reinterpret_cast<const uint32_t*>(qd);
+      int a              = 0;
+      for (int t = threadIdx.x; t < (d + 15) / 16 * 4; t += 32) {
+        const uint32_t w = qw[t];
         a = std::is_same<T, int8_t>::value ? __dp4a(static_cast<int>(w), static_cast<int>(w), a)
                                            : static_cast<int>(__dp4a(w, w, static_cast<unsigned>(a)));
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); }
+      a = __reduce_add_sync(0xffffffffu, a);
       if (threadIdx.x == 0) {
         s_qq_int = a;
         s_qq     = __ll2double_rn(static_cast<long long>(a));
       }
     }
-    __syncthreads();
-  } else {
-    load_queries<T>(queries, qpitch, &qi, 1, d, qd, d, &s_qq);
   }
-  const int n2 = max(next_pow2(static_cast<int>(c)), 2);
-  const int32_t* mine = cand + static_cast<size_t>(blockIdx.x) * cap;
+  // ---- values as unsigned keys in their order: of the rows that may be returned, and what every chain reaches (0: nothing)
+  const Candidate* mine = cd.cand + static_cast<size_t>(blockIdx.x) * cd.cap;
+  uint32_t* vkey        = reinterpret_cast<uint32_t*>(sc);
+  int32_t* vid          = reinterpret_cast<int32_t*>(sc) + n2max;
+  uint32_t* reached     = reinterpret_cast<uint32_t*>(ids);
+  auto key_of = [](int32_t product, int32_t e) {
+    if constexpr (kBytes) {
+      return static_cast<uint32_t>(product + e) ^ 0x80000000u;
+    } else {
+      const uint32_t f = __float_as_uint(__int_as_float(product) + __int_as_float(e));
+      return f ^ ((f >> 31) ? 0xffffffffu : 0x80000000u);
+    }
+  };
+  // Without a bitset the ids are looked up for the rows that are scored only: removed rows and padding have e = never.
+  constexpr int32_t kNever = kBytes ? kNeverInit : static_cast<int32_t>(0xff800000u);
+  const bool late          = adm.bits == nullptr && adm.row_labels == nullptr;
+  int sure = 0, seen = 0;
+  for (int i = threadIdx.x; i < c; i += blockDim.x) {
+    const uint4 cv     = __ldg(reinterpret_cast<const uint4*>(mine) + i);  // chain, mask, product
+    const int32_t prod = static_cast<int32_t>(cv.z);
+    uint32_t least     = 0xffffffffu;
+    bool all           = true;
+    for (uint32_t mask = cv.y; mask; mask &= mask - 1) {
+      const int64_t r  = static_cast<int64_t>(cv.x) * kChainRows + __ffs(mask) - 1;
+      const int32_t e  = r < cd.n_rows ? __ldg(cd.init + r) : kNever;
+      int32_t id       = static_cast<int32_t>(r);
+      bool may         = e != kNever;
+      if (may && !late) {
+        id  = __ldg(cd.perm + r);
+        may = admitted(adm, q, id);
+      }
+      ++seen;
+      if (may) {
+        const uint32_t key = key_of(prod, e);
+        const int at       = atomicAdd(&s_rows, 1);
+        least              = min(least, key);
+        if (at < n2max) { vkey[at] = key, vid[at] = id; }
+      } else {
+        all = false;
+      }
+    }
+    reached[i] = all ? least : 0u;
+    sure += all ? 1 : 0;
+  }
+  sure = __reduce_add_sync(0xffffffffu, sure);
+  seen = __reduce_add_sync(0xffffffffu, seen);
+  if ((threadIdx.x & 31) == 0) { atomicAdd(&s_sure, sure), atomicAdd(&s_seen, seen); }
+  __syncthreads();
+  const int rows  = min(s_rows, n2max);
+  const bool over = listed_all ? s_rows > n2max : true;
+  if (over && rf.thr2 == nullptr) {
+    if (threadIdx.x == 0) { ovf_list[atomicAdd(ovf_count, 1u)] = q; }
+    return;
+  }
+  uint32_t lowest = 1;
+  if (s_sure >= k && s_rows > k) {
+    lowest = block_kth_largest(reached, c, k, s_scratch);
+    if constexpr (!kBytes) {
+      const uint32_t f = lowest ^ ((lowest >> 31) ? 0x80000000u : 0xffffffffu);
+      const float v    = __fadd_rd(__uint_as_float(f), -cd.shift[q]);
+      const uint32_t g = __float_as_uint(v);
+      lowest           = max(1u, g ^ ((g >> 31) ? 0xffffffffu : 0x80000000u));
+    }
+  }
+  __syncthreads();  // the space of `reached` becomes the list of the rows to score
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+    if (vkey[i] >= lowest) { ids[atomicAdd(&s_kept, 1)] = late ? __ldg(cd.perm + vid[i]) : vid[i]; }
+  }
+  __syncthreads();
+  const int m = s_kept;
   // One thread reports an overflowed query with the tighter threshold that the k-th best exact score `kth` among the
   // listed candidates gives (+inf: fewer than k).
   auto report_overflow = [&](double kth) {
@@ -1103,7 +1332,11 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
     if (kth < CUDART_INF) {
       // the screen's value of a row as good as the k-th: <q, x> - |x|^2 / 2 (L2), <q, x> (inner product),
       // <q, x / |x|> (cosine)
-      const double value = METRIC == kCos ? sqrt(s_qq) * (1.0 - 0.5 * kth) : 0.5 * (s_qq - kth);
+      double qq = s_qq;
+      if (!kBytes && METRIC == kL2) {  // the scores had no use for it
+        for (int i = 0; i < d; ++i) { qq = __dadd_rn(qq, __dmul_rn(qd[i], qd[i])); }
+      }
+      const double value = METRIC == kCos ? sqrt(qq) * (1.0 - 0.5 * kth) : 0.5 * (qq - kth);
       if (rf.kind == 1) {  // integer values: e = -floor(|x|^2 / 2) only raises a row's value
         const double cv  = ceil(value);
         const int32_t tv = cv >= 2147483647.0 ? 0x7fffffff : cv <= -2147483648.0 ? static_cast<int32_t>(0x80000000u)
@@ -1120,23 +1353,18 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
   if constexpr (kBytes) {
     // integer scores (below 2^31 in magnitude) and ids sort as one 64-bit key: (score + 2^31) << 32 | id
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(sc);
-    __shared__ unsigned long long s_lists[kSelectWarps * kSelectMaxK], s_best[kSelectMaxK];
     constexpr int kGroups = 32 / kRowLanes;  // rows a warp's load covers
     const int sub         = threadIdx.x & (kRowLanes - 1);
     const int group       = (threadIdx.x >> 5) * kGroups + ((threadIdx.x & 31) / kRowLanes);
     const int n_groups    = (blockDim.x >> 5) * kGroups;
-    for (int i = static_cast<int>(c) + threadIdx.x; i < n2; i += blockDim.x) { keys[i] = ~0ull; }
-    for (int i0 = 0; i0 < static_cast<int>(c); i0 += n_groups * kRowUnroll) {  // the same trips for every lane of a warp
+    for (int i0 = 0; i0 < m; i0 += n_groups * kRowUnroll) {  // the same trips for every lane of a warp
       int32_t row[kRowUnroll];
-      bool ok[kRowUnroll];
       long long v[kRowUnroll];
 #pragma unroll
       for (int u = 0; u < kRowUnroll; ++u) {
         const int i = i0 + u * n_groups + group;
-        row[u]      = i < static_cast<int>(c) ? mine[i] : -1;
+        row[u]      = i < m ? ids[i] : -1;
       }
-#pragma unroll
-      for (int u = 0; u < kRowUnroll; ++u) { ok[u] = row[u] >= 0 && admitted(adm, q, row[u]); }
       if (where) {  // `vectors` is not in id order: row `where[id]` of it holds the vector with that id
         int32_t at[kRowUnroll];
 #pragma unroll
@@ -1149,37 +1377,23 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
       for (int u = 0; u < kRowUnroll; ++u) {
         const int i = i0 + u * n_groups + group;
         if (sub == 0 && row[u] >= 0) {
-          keys[i] = ok[u] ? (static_cast<unsigned long long>(v[u] + 2147483648ll) << 32) | static_cast<uint32_t>(row[u]) : ~0ull;
+          keys[i] = (static_cast<unsigned long long>(v[u] + 2147483648ll) << 32) | static_cast<uint32_t>(row[u]);
         }
       }
     }
-    const bool small = k <= kSelectMaxK && n2 <= 512 && blockDim.x <= kSelectWarps * 32;
-    __syncthreads();
-    if (small) {
-      select_smallest_keys(keys, n2, k, s_lists, s_best);
-    } else {
-      bitonic_sort_keys(keys, n2);
-    }
-    // entry t of the ranking, t < k: straight from the keys
-    auto entry = [&](int t) { return small ? s_best[t] : (t < n2 ? keys[t] : ~0ull); };
+    sort_keys(keys, m);
     if (over) {
       if (threadIdx.x == 0) {
-        const unsigned long long kk = entry(k - 1);
-        report_overflow(kk != ~0ull ? __ll2double_rn(static_cast<long long>(kk >> 32) - 2147483648ll) : CUDART_INF);
+        report_overflow(k <= m ? __ll2double_rn(static_cast<long long>(keys[k - 1] >> 32) - 2147483648ll) : CUDART_INF);
       }
       return;
     }
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
-      const unsigned long long key             = entry(t);
-      const bool have                          = key != ~0ull;
+      const bool have                          = t < m;
+      const unsigned long long key             = have ? keys[t] : 0ull;
       best_s[static_cast<size_t>(q) * k + t]   = have ? __ll2double_rn(static_cast<long long>(key >> 32) - 2147483648ll) : CUDART_INF;
       best_row[static_cast<size_t>(q) * k + t] = have ? static_cast<int32_t>(key & 0xffffffffull) : -1;
     }
-    if (threadIdx.x == 0 && stats) {
-      atomicAdd(stats + 0, static_cast<unsigned long long>(c));  // survivors of the screen
-      atomicAdd(stats + 1, static_cast<unsigned long long>(c));  // exact scores computed
-    }
-    return;
   } else {
     // Float rows: a thread sums its candidate's coordinates in order (the order of the fp64 reference loop), but the
     // rows come through shared memory: a warp fetches a 128-byte slab of 32 candidate rows with eight loads that each
@@ -1191,86 +1405,76 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
     const int n_pieces    = static_cast<int>((static_cast<size_t>(d) * sizeof(T) + 15) / 16);  // rows are zero padded to the pitch
     uint8_t* tile         = stage_of(ids + n2max) + static_cast<size_t>(warp) * 32 * kStageStride;
     const int piece       = lane & 7, row_in_load = lane >> 3;
-    for (int g = warp; g * 32 < n2; g += n_warps) {
-      const int i   = g * 32 + lane;
-      int32_t row   = 0x7fffffff;
-      bool ok       = false;
-      if (i < static_cast<int>(c)) {
-        row = mine[i];
-        ok  = admitted(adm, q, row);
-      }
+    for (int g = warp; g * 32 < m; g += n_warps) {
+      const int i       = g * 32 + lane;
+      const bool ok     = i < m;
+      const int32_t row = ok ? ids[i] : -1;
       Acc<METRIC, 1, STORED_XX> acc;
       acc.clear();
       if constexpr (STORED_XX) {
         if (ok) { acc.xx = __ldg(sqnorm + row); }
       }
-      if (g * 32 < static_cast<int>(c)) {  // the same for every lane of the warp
-        int32_t from[8];  // the rows this lane fetches pieces of
+      int32_t from[8];  // the rows this lane fetches pieces of
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { from[j] = __shfl_sync(0xffffffffu, ok ? row : -1, 4 * j + row_in_load); }
-        // The loads of the next slab are issued as soon as this slab's registers have been parked in the tile, so that
-        // they are in flight while the lanes walk the tile (a warp alone then overlaps its memory latency with its sums).
-        uint4 w[8];
-        auto fetch = [&](int p0) {
+      for (int j = 0; j < 8; ++j) { from[j] = __shfl_sync(0xffffffffu, row, 4 * j + row_in_load); }
+      // The loads of the next slab are issued as soon as this slab's registers have been parked in the tile, so that
+      // they are in flight while the lanes walk the tile (a warp alone then overlaps its memory latency with its sums).
+      uint4 w[8];
+      auto fetch = [&](int p0) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            w[j] = (from[j] >= 0 && p0 + piece < n_pieces)
-                     ? __ldg(reinterpret_cast<const uint4*>(vectors + static_cast<size_t>(from[j]) * pitch) + p0 + piece)
-                     : make_uint4(0, 0, 0, 0);
-          }
-        };
-        fetch(0);
-        for (int p0 = 0; p0 < n_pieces; p0 += 8) {
-          __syncwarp();  // every lane is done with the slab before
+        for (int j = 0; j < 8; ++j) {
+          w[j] = (from[j] >= 0 && p0 + piece < n_pieces)
+                   ? __ldg(reinterpret_cast<const uint4*>(vectors + static_cast<size_t>(from[j]) * pitch) + p0 + piece)
+                   : make_uint4(0, 0, 0, 0);
+        }
+      };
+      fetch(0);
+      for (int p0 = 0; p0 < n_pieces; p0 += 8) {
+        __syncwarp();  // every lane is done with the slab before
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            *reinterpret_cast<uint4*>(tile + (4 * j + row_in_load) * kStageStride + piece * 16) = w[j];
-          }
-          __syncwarp();
-          if (p0 + 8 < n_pieces) { fetch(p0 + 8); }
-          if (ok) {
-            const int np = min(8, n_pieces - p0);
-            for (int p = 0; p < np; ++p) {
-              const uint4 x4 = *reinterpret_cast<const uint4*>(tile + lane * kStageStride + p * 16);
-              double x[V];
-              Elems<T>::unpack_finite(x4, x);  // screened rows are finite
-              const int t0 = (p0 + p) * V;
-              if (t0 + V <= d) {
-                // the query's doubles two at a time (t0 is a multiple of V, qd is 16-byte aligned): half the
-                // shared-memory instructions of the walk
+        for (int j = 0; j < 8; ++j) {
+          *reinterpret_cast<uint4*>(tile + (4 * j + row_in_load) * kStageStride + piece * 16) = w[j];
+        }
+        __syncwarp();
+        if (p0 + 8 < n_pieces) { fetch(p0 + 8); }
+        if (ok) {
+          const int np = min(8, n_pieces - p0);
+          for (int p = 0; p < np; ++p) {
+            const uint4 x4 = *reinterpret_cast<const uint4*>(tile + lane * kStageStride + p * 16);
+            double x[V];
+            Elems<T>::unpack_finite(x4, x);  // screened rows are finite
+            const int t0 = (p0 + p) * V;
+            if (t0 + V <= d) {
+              // the query's doubles two at a time (t0 is a multiple of V, qd is 16-byte aligned): half the
+              // shared-memory instructions of the walk
 #pragma unroll
-                for (int e = 0; e < V; e += 2) {
-                  const double2 a = *reinterpret_cast<const double2*>(qd + t0 + e);
-                  acc.add1(x[e], a.x);
-                  acc.add1(x[e + 1], a.y);
-                }
-              } else {
-                for (int e = 0; e < V && t0 + e < d; ++e) { acc.add(x[e], qd, d, t0 + e); }
+              for (int e = 0; e < V; e += 2) {
+                const double2 a = *reinterpret_cast<const double2*>(qd + t0 + e);
+                acc.add1(x[e], a.x);
+                acc.add1(x[e + 1], a.y);
               }
+            } else {
+              for (int e = 0; e < V && t0 + e < d; ++e) { acc.add(x[e], qd, d, t0 + e); }
             }
           }
         }
       }
-      if (i < n2) {
-        sc[i]  = ok ? acc.result(0, s_qq) : CUDART_INF;
-        ids[i] = row;
-      }
+      if (ok) { sc[i] = acc.result(0, s_qq); }
     }
-    bitonic_sort(sc, ids, n2);
-  }
-  if (over) {
-    __syncthreads();
-    if (threadIdx.x == 0) { report_overflow(k <= n2 ? sc[k - 1] : CUDART_INF); }
-    return;
-  }
-  for (int t = threadIdx.x; t < k; t += blockDim.x) {
-    const bool have                         = t < n2 && sc[t] < CUDART_INF;
-    best_s[static_cast<size_t>(q) * k + t]   = have ? sc[t] : CUDART_INF;
-    best_row[static_cast<size_t>(q) * k + t] = have ? ids[t] : -1;
+    sort_pairs(sc, ids, m);
+    if (over) {
+      if (threadIdx.x == 0) { report_overflow(k <= m ? sc[k - 1] : CUDART_INF); }
+      return;
+    }
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+      const bool have                         = t < m;
+      best_s[static_cast<size_t>(q) * k + t]   = have ? sc[t] : CUDART_INF;
+      best_row[static_cast<size_t>(q) * k + t] = have ? ids[t] : -1;
+    }
   }
   if (threadIdx.x == 0 && stats) {
-    atomicAdd(stats + 0, static_cast<unsigned long long>(c));  // survivors of the screen
-    atomicAdd(stats + 1, static_cast<unsigned long long>(c));  // exact scores computed
+    atomicAdd(stats + 0, static_cast<unsigned long long>(s_seen));  // rows the screen kept
+    atomicAdd(stats + 1, static_cast<unsigned long long>(m));  // exact scores computed
   }
 }
 
@@ -1737,11 +1941,10 @@ void launch_gather_chain_min(const int32_t* init, int64_t stride_w, int64_t stri
                                                                                  is_float ? 1 : 0);
 }
 
-void launch_expand_records(const uint64_t* rec, const unsigned long long* rec_count, unsigned long long rec_cap,
-                           int64_t n_rows, const int32_t* perm, uint32_t* cnt, int32_t* cand, uint32_t cap, int sm_count,
-                           cudaStream_t s)
+void launch_candidate_rows(const Candidate* cand, const uint32_t* cnt, uint32_t cap, int nq, int64_t n_rows, uint32_t* row_cnt,
+                           int32_t* rows, uint32_t row_cap, cudaStream_t s)
 {
-  expand_records_kernel<<<sm_count * 8, 256, 0, s>>>(rec, rec_count, rec_cap, n_rows, perm, cnt, cand, cap);
+  if (nq > 0) { candidate_rows_kernel<<<nq, 128, 0, s>>>(cand, cnt, cap, n_rows, row_cnt, rows, row_cap); }
 }
 
 void launch_chain_max(const int32_t* init, int64_t c0, int64_t n, int32_t* cmax, bool is_float, cudaStream_t s)
@@ -1789,6 +1992,17 @@ void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, in
   } else {
     encode_f16_queries_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq,
                                                            static_cast<uint8_t*>(codes), code_pitch, n1max, n2max, emax, shift, overflow);
+  }
+}
+
+void launch_query_sqnorms(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, double* qq, cudaStream_t s)
+{
+  if (nq <= 0) { return; }
+  const auto grid = static_cast<unsigned>((nq + 31) / 32);
+  if (dtype == kF32) {
+    query_sqnorm_kernel<float><<<grid, 32, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq, qq);
+  } else {
+    query_sqnorm_kernel<__half><<<grid, 32, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq, qq);
   }
 }
 
@@ -1870,28 +2084,25 @@ void launch_remove(const int64_t* ids, int64_t n_ids, int64_t size, uint8_t* rem
 }
 
 void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, int metric, const void* queries,
-                          size_t qpitch, int nq, int q0, const int32_t* cand, const uint32_t* cnt, uint32_t cap, int k,
+                          size_t qpitch, int nq, int q0, const Candidates& cd, int k,
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
-                          unsigned long long* stats, const unsigned long long* rec_count, unsigned long long rec_cap,
-                          Refine rf, cudaStream_t s, const int32_t* where, const double* sqnorm)
+                          unsigned long long* stats, Refine rf, cudaStream_t s, const int32_t* where, const double* sqnorm)
 {
   if (nq <= 0) { return; }
-  const int n2max   = next_pow2(static_cast<int>(cap));
-  const bool bytes  = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys: no separate id array
-  // float rows: a warp scores 32 candidates at a time, so a query with a few hundred candidates keeps 8 warps busy;
-  // larger blocks leave warps idle at the barrier before the sort (measured on 768-dimensional rows with 153 and 664
-  // candidates per query and on 128-dimensional keys with 2 394: 256 threads beat 128, 512 and 1024 in all three)
-  const int threads = (dtype == kF32 || dtype == kF16) ? 256 : 128;
+  const int n2max   = next_pow2(static_cast<int>(cd.cap));
+  const bool bytes  = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys
+  // a warp of float rows scores 32 rows at a time, and about k to 2 k are left to score
+  const int threads = !bytes && k > 32 ? 256 : 128;
   // float rows: + 16 bytes of alignment and one staging tile per warp
-  const size_t smem = sizeof(double) * (static_cast<size_t>(d) + n2max) +
-                      (bytes ? 0 : sizeof(int32_t) * n2max + 16 + static_cast<size_t>(threads / 32) * 32 * kStageStride);
+  const size_t smem = (bytes ? static_cast<size_t>((d + 15) / 16 * 16) : sizeof(double) * static_cast<size_t>(d)) +
+                      (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2max) +
+                      (bytes ? 0 : 16 + static_cast<size_t>(threads / 32) * 32 * kStageStride);
   by_dtype(dtype, [&](auto tag) {
     using T   = decltype(tag);
     auto go   = [&](auto kernel) {
       allow_smem(kernel, smem);
-      kernel<<<nq, threads, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch, q0, cand, cnt, cap,
-                                   n2max, k, adm, best_s, best_row, ovf_list, ovf_count, stats, rec_count, rec_cap, rf,
-                                   where, sqnorm);
+      kernel<<<nq, threads, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch, q0, cd, n2max, k, adm,
+                                       best_s, best_row, ovf_list, ovf_count, stats, rf, where, sqnorm);
     };
     if (metric == kL2) {
       go(verify_select_kernel<T, kL2>);

@@ -53,6 +53,9 @@ void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, in
                                size_t code_pitch, float n1max, float n2max, float emax, float* shift,
                                unsigned int* overflow, cudaStream_t s);
 
+/// qq [nq] = |q|^2 of float queries as the exact scores sum it (coordinates in order, fp64, every operation rounded).
+void launch_query_sqnorms(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, double* qq, cudaStream_t s);
+
 /// thr [nq] of fp16 codes. step 0: float keys of the k-th largest group maxima -> keys of (value - shift / 2), scores
 /// that k rows certainly reach; step 1: such keys -> float bits of the screen's threshold (bound - shift / 2).
 void launch_finish_thr_f16(int32_t* thr, const float* shift, int nq, int step, cudaStream_t s, int per = 1);
@@ -69,11 +72,26 @@ void launch_sort_batch(const int32_t* e, int64_t n, int32_t id0, int64_t row0, c
                        int metric, bool is_float, uint32_t* keys_in, uint32_t* keys_out, int32_t* ids_in, int32_t* ids_out,
                        void* temp, size_t temp_bytes, void* codes, int32_t* perm, int32_t* inv, int32_t* init, cudaStream_t s);
 
-/// Survivor records of the screen (see make_record) -> cnt [nq] / cand [nq, cap]; rows >= n_rows are dropped, rows are
-/// translated to ids through perm (when not null).
-void launch_expand_records(const uint64_t* rec, const unsigned long long* rec_count, unsigned long long rec_cap,
-                           int64_t n_rows, const int32_t* perm, uint32_t* cnt, int32_t* cand, uint32_t cap, int sm_count,
-                           cudaStream_t s);
+/// What a screen kept: cand [nq, cap] chains per query (see Candidate in screen_i8.cuh), cnt [nq] how many (more than cap:
+/// the list overflowed), and what turns a row of a chain into an id and the value the thresholds are made of: perm [n_rows]
+/// the id of a code row, init [n_rows] its e (int32, or float bits with fp16 codes; never: a removed row, or no row). fp16
+/// codes also, indexed like the queries: shift (see launch_encode_f16_queries) and, but for the L2 metric, qq (see
+/// launch_query_sqnorms).
+struct Candidate;
+struct Candidates {
+  const Candidate* cand;
+  const uint32_t* cnt;
+  uint32_t cap;
+  int64_t n_rows;
+  const int32_t* perm;
+  const int32_t* init;
+  const float* shift;
+  const double* qq;
+};
+
+/// The rows of the candidate lists (row numbers below n_rows): row_cnt [nq] += how many, rows [nq, row_cap] the first of them.
+void launch_candidate_rows(const Candidate* cand, const uint32_t* cnt, uint32_t cap, int nq, int64_t n_rows, uint32_t* row_cnt,
+                           int32_t* rows, uint32_t row_cap, cudaStream_t s);
 
 /// thr[q] = k-th largest of gmax[q, 0:ng]  (INT_MIN when ng < k). With ng_rows [nq] every row has its own length
 /// (at most ng); a negative length gives thr[q] = never. With topk [nq, k] the k largest values of every row are
@@ -125,18 +143,17 @@ void launch_scatter_best(const double* s2, const int32_t* row2, const int32_t* s
 void launch_compose(int32_t* list, const unsigned int* n, int n_max, const int32_t* sel, cudaStream_t s);
 
 /**
- * Exact fp64 scores of every query's candidate rows, then its k best by (score, row). One block per query.
- * cand [nq, cap] rows, cnt [nq] how many (a query with cnt > cap is skipped and its index appended to ovf_list;
- * so is every query when *rec_count > rec_cap, i.e. when the screen's survivor records did not all fit).
- * best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates exist).
- * `where` (8-bit rows only, optional): `vectors` is not in id order, row where[id] of it holds the vector with that id
- * (the norm-sorted code rows of an index whose vectors live in host memory).
+ * The k best of every query's candidates by (exact fp64 score, id). One block per query: the candidates are ranked by the
+ * screen's own values, and those that can belong to the k best are scored. A query with cnt > cap chains, or more than
+ * next_pow2(cap) rows in them, is appended to ovf_list and not answered. best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates exist). `where`
+ * (8-bit rows only, optional): `vectors` is not in id order, row where[id] of it holds the vector with that id (the
+ * norm-sorted code rows of an index whose vectors live in host memory).
  */
 void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, int metric, const void* queries,
-                          size_t qpitch, int nq, int q0, const int32_t* cand, const uint32_t* cnt, uint32_t cap, int k,
+                          size_t qpitch, int nq, int q0, const Candidates& cd, int k,
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
-                          unsigned long long* stats, const unsigned long long* rec_count, unsigned long long rec_cap,
-                          Refine rf, cudaStream_t s, const int32_t* where = nullptr, const double* sqnorm = nullptr);
+                          unsigned long long* stats, Refine rf, cudaStream_t s, const int32_t* where = nullptr,
+                          const double* sqnorm = nullptr);
 
 /// out[r] = |x_r|^2 of n float32 / float16 rows, summed over the coordinates in order in fp64 with every product and sum
 /// rounded on its own: the sum the cosine verification makes per candidate. With it (sqnorm of launch_verify_select,

@@ -18,9 +18,11 @@
 // an instruction per element) and tests  max + cmax[chain] >= thr  with cmax = max of e over the chain. That test
 // never rejects a pair that should be kept. Only in a chain that passes it (rare) the columns are looked at one by
 // one, still with cmax in place of their own e: what is kept is a superset of the pairs at or above the threshold,
-// larger by the few rows whose e is below their chain's maximum, and the exact scores of the verification sort those
-// out. The kept columns of a chain form one record (query, chain, 16-bit mask) in the warp's staging buffer in shared
-// memory, and a half-full buffer goes to global memory with one atomic add for the whole batch.
+// larger by the few rows whose e is below their chain's maximum, and the verification sorts those
+// out. The kept columns of a chain are staged in the warp's buffer in shared memory as one entry (query, chain, 16-bit mask,
+// largest product), and a half-full buffer goes straight into the queries' candidate lists: a lane takes an entry, an atomic
+// add on the query's counter gives its place. The product lets the verification rank the candidates before it reads a
+// single vector.
 // GROUPMAX writes gmax[q][group] = max over 64 anchors of value (exact, e is staged in shared memory with the tile);
 // the k-th largest group maximum of a query is its threshold: k distinct stored rows are at least that close. The
 // anchors of one tile are spread over the whole sorted set (column c of tile t is anchor c * n_tiles + t), so that the
@@ -63,7 +65,7 @@ constexpr int kThreads    = 32 * (2 + kEpiWarps);
 // The two single-thread roles sit in the last two warps; warps 0..15 are the epilogue (TMEM lane quarter = warp % 4).
 constexpr int kTmaWarp    = kEpiWarps;
 constexpr int kMmaWarp    = kEpiWarps + 1;
-constexpr int kRecBuf     = 64;                // staged survivor records per epilogue warp (flushed when half full)
+constexpr int kRecBuf     = 64;                // staged candidates per epilogue warp (sent to the lists when half full)
 constexpr int kWideStage  = 2 * kQTileBytes + kBTileBytes;  // WIDE: one K block of two query tiles and a base tile
 constexpr int kWideStages = 3;
 constexpr int kERing      = 4;                 // WIDE: tiles whose e values may be in flight
@@ -100,7 +102,7 @@ struct SharedCtl {
 
   uint32_t tmem_base;
   int abort_flag;
-  int rec_n[kEpiWarps];         // fill counts of the warps' record staging buffers
+  int rec_n[kEpiWarps];         // fill counts of the warps' staging buffers
 };
 
 __device__ __forceinline__ int max3(int a, int b, int c) { return __vimax3_s32(a, b, c); }
@@ -234,7 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
   const uint32_t init_off  = stage_off + (WIDE ? static_cast<uint32_t>(kWideStages * kWideStage)
                                                : static_cast<uint32_t>(ns) * kb * kBTileBytes);
   const uint32_t rec_off   = init_off + static_cast<uint32_t>(WIDE ? kERing : ns) * kBaseTile * 4;
-  const uint32_t ctl_off   = rec_off + kEpiWarps * kRecBuf * 8;
+  const uint32_t recm_off  = rec_off + kEpiWarps * kRecBuf * 8;
+  const uint32_t ctl_off   = recm_off + kEpiWarps * kRecBuf * 4;
   SharedCtl* ctl           = reinterpret_cast<SharedCtl*>(gen_base + ctl_off);
   const int32_t* init_smem = reinterpret_cast<const int32_t*>(gen_base + init_off);
   volatile int* abort_flag = &ctl->abort_flag;
@@ -501,30 +504,37 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
     const int quarter        = warp & 3;  // the TMEM lane quarter this warp may access
     const int row            = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    uint64_t* rec_buf        = reinterpret_cast<uint64_t*>(gen_base + rec_off) + ew * kRecBuf;
-    volatile int* rec_n      = &ctl->rec_n[ew];  // staged records of this warp
+    // Staged candidates of this warp. key: bits 63..48 query (inside the batch), bits 47..16 chain, bits 15..0 mask; max: the
+    // chain's largest product.
+    uint64_t* st_key    = reinterpret_cast<uint64_t*>(gen_base + rec_off) + ew * kRecBuf;
+    int32_t* st_max     = reinterpret_cast<int32_t*>(gen_base + recm_off) + ew * kRecBuf;
+    volatile int* rec_n = &ctl->rec_n[ew];
 
     uint32_t gu = 0;  // units of this CTA so far: slot = gu & 1, the slot's use number = gu >> 1
     bool ok     = true;
 
-    // Staged records -> global memory: one atomic add reserves the range, the lanes copy.
-    auto flush = [&](int n_rec) {
-      unsigned long long at = 0;
-      if (lane == 0) { at = atomicAdd(p.rec_count, static_cast<unsigned long long>(n_rec)); }
-      at = __shfl_sync(0xffffffffu, at, 0);
-      for (int i = lane; i < n_rec; i += 32) {
-        if (at + i < p.rec_cap) { p.rec[at + i] = rec_buf[i]; }
+    // A candidate into its query's list.
+    auto append = [&](uint64_t key, int32_t product) {
+      const uint32_t q  = static_cast<uint32_t>(key >> 48);
+      const uint32_t at = atomicAdd(p.cnt + q, 1u);
+      if (at < p.cap) {
+        reinterpret_cast<uint4*>(p.cand)[static_cast<size_t>(q) * p.cap + at] =
+          make_uint4(static_cast<uint32_t>(key >> 16), static_cast<uint32_t>(key & 0xffffu), static_cast<uint32_t>(product), 0u);
       }
+    };
+    // The staged candidates -> the lists: the lanes' atomic adds are in flight together.
+    auto flush = [&](int n) {
+      for (int i = lane; i < n; i += 32) { append(st_key[i], st_max[i]); }
       __syncwarp();
       if (lane == 0) { *rec_n = 0; }
       __syncwarp();
     };
-    // A chain of 16 columns whose maximum reached the query's threshold with the chain's largest e: the columns that
-    // reach it with that same e form one record. (Rows are kept sorted by norm, so e is almost constant over a chain
-    // and hardly any row is kept that the exact e would drop; the exact scores sort that out.) The record is staged
-    // through the warp's buffer in shared memory, whose fill count is a shared-memory atomic: the few threads that get
-    // here need no warp-wide step.
-    auto record = [&](const int32_t* v, int thr, int ce, int q, int64_t row0) {
+    // A chain of 16 columns whose largest product m reached the query's threshold with the chain's largest e: the columns
+    // that reach it with that same e are kept, as one entry. (Rows are kept sorted by norm, so e is almost constant over a
+    // chain and hardly any row is kept that its own e would drop; the verification sorts that out.) The entry is staged
+    // through the warp's buffer in shared memory, whose fill count is a shared-memory atomic: the few threads that get here
+    // need no warp-wide step.
+    auto record = [&](const int32_t* v, int m, int thr, int ce, int q, int64_t row0) {
       uint32_t mask = 0;
       if (F16) {
         const float tf = __int_as_float(thr), cf = __int_as_float(ce);
@@ -535,21 +545,21 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
 #pragma unroll
         for (int i = 0; i < 16; ++i) { mask |= (v[i] >= t ? 1u : 0u) << i; }
       }
-      const uint64_t r = make_record(static_cast<uint32_t>(q), static_cast<uint32_t>(row0 / kChainRows), mask);
-      const int pos    = atomicAdd(const_cast<int*>(rec_n), 1);
+      const uint64_t key = (static_cast<uint64_t>(q) << 48) | (static_cast<uint64_t>(row0 / kChainRows) << 16) | mask;
+      const int pos      = atomicAdd(const_cast<int*>(rec_n), 1);
       if (pos < kRecBuf) {
-        rec_buf[pos] = r;
-      } else {  // the staging buffer is full: straight to global memory
-        const unsigned long long at = atomicAdd(p.rec_count, 1ull);
-        if (at < p.rec_cap) { p.rec[at] = r; }
+        st_key[pos] = key;
+        st_max[pos] = m;
+      } else {  // the staging buffer is full: straight to the list
+        append(key, m);
       }
     };
 
     // An epilogue warp is one serial stream of instructions per unit, and the pass is as fast as that stream (the MMAs
     // of a unit of a 128-byte row take about 610 cycles; a hundred dependent instructions of a warp that shares its
     // scheduler with four others take more). So the loops are plain nested loops over the segment's tiles and query
-    // tiles with pointers that are bumped, nothing is recomputed per unit that is known per tile or per segment, and
-    // warp-wide steps (the check of the record buffer) happen once per tile. Everything between a unit's completion and
+    // tiles with pointers that are bumped, and nothing is recomputed per unit that is known per tile or per segment.
+    // Everything between a unit's completion and
     // the release of its slot also sits on the other path that bounds the pass (two slots: the MMAs of the next unit but
     // one wait for the release): the threshold and the chain maxima of e are loaded before the wait and not touched
     // until the slot is released, and the release follows tcgen05.wait::ld directly (it is warp-wide: when lane 0 is
@@ -622,17 +632,20 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
           // 32 columns (two chains) of a SCREEN piece: v = a or b, c0 / c1 their chain maxima of e
           auto screen32 = [&](const int32_t* v, int c0, int c1, int64_t r0) {
             bool h0, h1;
+            int m0, m1;
             if (F16) {
-              const float tf = __int_as_float(thr);
-              h0 = max16f(v) + __int_as_float(c0) >= tf;
-              h1 = max16f(v + 16) + __int_as_float(c1) >= tf;
+              const float tf = __int_as_float(thr), f0 = max16f(v), f1 = max16f(v + 16);
+              h0 = f0 + __int_as_float(c0) >= tf;
+              h1 = f1 + __int_as_float(c1) >= tf;
+              m0 = __float_as_int(f0), m1 = __float_as_int(f1);
             } else {
-              h0 = max16(v) + c0 >= thr;
-              h1 = max16(v + 16) + c1 >= thr;
+              m0 = max16(v), m1 = max16(v + 16);
+              h0 = m0 + c0 >= thr;
+              h1 = m1 + c1 >= thr;
             }
-            if (h0 | h1) {  // rare: the lanes that kept something stage their records, nobody else waits
-              if (h0) { record(v, thr, c0, q, r0); }
-              if (h1) { record(v + 16, thr, c1, q, r0 + 16); }
+            if (h0 | h1) {  // rare: the lanes that kept something stage it, nobody else waits
+              if (h0) { record(v, m0, thr, c0, q, r0); }
+              if (h1) { record(v + 16, m1, thr, c1, q, r0 + 16); }
               kept = true;
             }
           };
@@ -730,8 +743,8 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
           TRACE_AT(tr_w, gu, 7);
         }
         if (!ok) { break; }
-        // the tile is done: staged records go out once the buffer is half full (records beyond its end go straight to
-        // global memory meanwhile), and the tile's e values are released (GROUPMAX)
+        // the tile is done: staged candidates go out once the buffer is half full (those beyond its end go straight to the
+        // lists meanwhile), and the tile's e values are released (GROUPMAX)
         if (MODE == kModeScreen && __any_sync(0xffffffffu, kept)) {
           const int staged = min(*rec_n, kRecBuf);
           if (staged > kRecBuf / 2) { flush(staged); }
@@ -759,16 +772,12 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
 
 }  // namespace
 
-size_t screen_smem_bytes_wide()
-{
-  return 1024 + static_cast<size_t>(kWideStages) * kWideStage + static_cast<size_t>(kERing) * kBaseTile * 4 +
-         kEpiWarps * kRecBuf * 8 + sizeof(SharedCtl) + 64;
-}
-
 size_t screen_smem_bytes(int kb, int panel_tiles, int n_stages)
 {
-  return 1024 + static_cast<size_t>(panel_tiles) * kb * kQTileBytes + static_cast<size_t>(n_stages) * kb * kBTileBytes +
-         static_cast<size_t>(n_stages) * kBaseTile * 4 + kEpiWarps * kRecBuf * 8 + sizeof(SharedCtl) + 64;
+  const size_t tiles = kb > 2 ? static_cast<size_t>(kWideStages) * kWideStage + static_cast<size_t>(kERing) * kBaseTile * 4
+                              : static_cast<size_t>(panel_tiles) * kb * kQTileBytes +
+                                  static_cast<size_t>(n_stages) * (kb * kBTileBytes + kBaseTile * 4);
+  return 1024 + tiles + kEpiWarps * kRecBuf * 12 + sizeof(SharedCtl) + 64;
 }
 
 namespace {
@@ -784,7 +793,7 @@ cudaError_t screen_i8_launch(const CUtensorMap& tm_q, const CUtensorMap& tm_x, c
   ScreenArgs args  = args_in;
   args.trace       = g_trace;
   args.trace_units = g_trace_units;
-  const size_t smem = args.wide ? screen_smem_bytes_wide() : screen_smem_bytes(args.kb, args.panel_tiles, args.n_stages);
+  const size_t smem = screen_smem_bytes(args.kb, args.panel_tiles, args.n_stages);
   // opt-in to large dynamic shared memory (cheap; set on every launch so that every device of the process has it)
   if (!args.wide && args.kb != 1 && args.kb != 2) { return cudaErrorInvalidValue; }
   const bool kb2 = args.kb == 2;

@@ -25,7 +25,7 @@ enum : int { kModeScreen = 0, kModeGroupMax = 1, kModeRate = 2, kModeGroupBound 
 /// Init value of a column that must never pass a threshold (removed rows, padding beyond the last row).
 constexpr int32_t kNeverInit = -(1 << 30);
 
-constexpr int kChainRows = 16;  // rows per chain: the unit of the conservative threshold test and of a survivor record
+constexpr int kChainRows = 16;  // rows per chain: the unit of the conservative threshold test
 
 /// One contiguous piece of work of a CTA: query tiles [q_tile0, q_tile0 + n_qtiles) against base tiles [t0, t1)
 /// (query tiles of 128 queries, base tiles of 256 rows).
@@ -36,12 +36,13 @@ struct ScreenSeg {
   int t1;
 };
 
-/// A survivor record: bits 63..48 query (inside the batch), bits 47..16 chunk = row / 16, bits 15..0 one bit per row
-/// of the chunk that reached the query's threshold.
-__host__ __device__ inline uint64_t make_record(uint32_t q, uint32_t chunk, uint32_t mask16)
-{
-  return (static_cast<uint64_t>(q) << 48) | (static_cast<uint64_t>(chunk) << 16) | mask16;
-}
+/// An entry of a query's candidate list: the rows of one chain that reached the query's threshold.
+struct __align__(16) Candidate {
+  uint32_t chain;   // rows 16 chain .. 16 chain + 15 of the code rows the pass read
+  uint32_t mask;    // one bit per row of the chain
+  int32_t product;  // the largest <q, x> of the chain (int32, or the bits of a float): a row in the mask has it
+  uint32_t unused;
+};
 
 struct ScreenArgs {
   const int32_t* init;            // [n_tiles * 256] per-row term e[x] added to <q, x> (kNeverInit: removed / padding)
@@ -49,9 +50,9 @@ struct ScreenArgs {
   const int32_t* thr;             // SCREEN: [nq] keep iff <q, x> + e[x] >= thr[q]
   int32_t* gmax;                  // GROUPMAX: [nq, ld_gmax] maximum of <q, x> + e[x] over every group of 64 rows
   int64_t ld_gmax;
-  uint64_t* rec;                  // SCREEN: survivor records
-  unsigned long long* rec_count;  // SCREEN: records appended (may exceed rec_cap: overflow, the excess is not written)
-  unsigned long long rec_cap;
+  Candidate* cand;                // SCREEN: [nq, cap] the chains kept per query, in no order
+  uint32_t* cnt;                  // SCREEN: [nq] chains kept (may exceed cap: overflow, the excess is not written)
+  uint32_t cap;
   int nq;
   int kb;                         // K blocks of 128 bytes per row
   int panel_tiles;                // query tiles resident in shared memory
@@ -72,8 +73,10 @@ struct ScreenArgs {
   int trace_units;
 };
 
+constexpr size_t kMaxSmem = 227 * 1024;  // dynamic shared memory a block may have
+
+/// What a launch needs of it.
 size_t screen_smem_bytes(int kb, int panel_tiles, int n_stages);
-size_t screen_smem_bytes_wide();
 
 /// Profiling aid, effective only in a library built with -DCERTEX_SCREEN_TRACE=1 (make trace): CTA 0 of every later
 /// pass writes SM clock stamps of its first `units` accumulator units to the device buffer `trace` ([units, 12] int64;
