@@ -36,6 +36,12 @@ constexpr int64_t kQTile = kQueryTile;
 constexpr int64_t kMaxCodeBytes = 4096;  // longest code row the tensor-core pass takes (32 K blocks)
 
 inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
+inline int next_pow2(uint32_t v)
+{
+  int p = 1;
+  while (static_cast<uint32_t>(p) < v) { p <<= 1; }
+  return p;
+}
 
 // ------------------------------------------------------------------ stream-ordered scratch memory
 struct Scratch {
@@ -733,7 +739,9 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   const int nt_all        = static_cast<int>((n + kTile - 1) / kTile);
   const uint32_t cap      = test_mode_ == 2 ? static_cast<uint32_t>(test_cap_) : static_cast<uint32_t>(std::max(2048, 2 * k));
   uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(nq));
-  Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(nq) * cap);
+  const int ld_cand    = next_pow2(cap);
+  Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(nq) * ld_cand);
+  int32_t* kept        = scratch.get<int32_t>(static_cast<size_t>(nq));
   const DevicePlan plan = device_plan(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
   auto* d_segs          = static_cast<ScreenSeg*>(plan.segs);
   int* d_seg_begin      = plan.begin;
@@ -759,6 +767,7 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   a.cand        = cand;
   a.cnt         = cnt;
   a.cap         = cap;
+  a.ld_cand     = static_cast<uint32_t>(ld_cand);
   a.segs        = d_segs;
   a.seg_begin   = d_seg_begin;
   auto mark = [&] {
@@ -780,8 +789,8 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   // 8-bit vectors kept in host memory: the exact stage reads the candidates' code rows, which are the vectors
   const bool from_codes = host_vectors_ && screen_kind_ == 1;
   launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, queries, row_bytes,
-                       nq, q0, Candidates{cand, cnt, cap, n, perm_, init_, shift, qq}, k, adm, best_s, best_row, ovf_list, ovf_count,
-                       stats, rf, res.stream, from_codes ? inv_ : nullptr, sqnorm_);
+                       nq, q0, Candidates{cand, cnt, cap, ld_cand, n, perm_, init_, shift, qq}, k, adm, best_s, best_row, ovf_list, ovf_count,
+                       stats, rf, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
   CERTEX_CUDA(cudaGetLastError());
 }
 
@@ -1093,7 +1102,9 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     int32_t* gmax        = scratch.get<int32_t>(static_cast<size_t>(ns) * ld_g);
     int32_t* thr         = scratch.get<int32_t>(static_cast<size_t>(ns));
     uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(ns));
-    Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(ns) * cap);
+    const int ld_cand    = next_pow2(cap);
+    Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(ns) * ld_cand);
+    int32_t* kept        = scratch.get<int32_t>(static_cast<size_t>(ns));
     double* slot_s       = scratch.get<double>(static_cast<size_t>(ns) * k);
     int32_t* slot_row    = scratch.get<int32_t>(static_cast<size_t>(ns) * k);
     int32_t* ovf_list    = scratch.get<int32_t>(static_cast<size_t>(ns));
@@ -1164,6 +1175,7 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     a.cand      = cand;
     a.cnt       = cnt;
     a.cap       = cap;
+    a.ld_cand   = static_cast<uint32_t>(ld_cand);
     mark();
     CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
     mark();
@@ -1171,8 +1183,8 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     plain.removed = removed_;
     const bool from_codes = host_vectors_ && screen_kind_ == 1;
     launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, q_rows,
-                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, n_lrows_, lperm_, linit_, shift, qq}, k, plain, slot_s, slot_row,
-                         ovf_list, d_flag, d_stats, Refine{}, res.stream, from_codes ? inv_ : nullptr, sqnorm_);
+                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq}, k, plain, slot_s, slot_row,
+                         ovf_list, d_flag, d_stats, Refine{}, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
     launch_scatter_best(slot_s, slot_row, d_slot_q, ns, k, best_s, best_row, res.stream);
     CERTEX_CUDA(cudaGetLastError());
     st->launches += f16 ? (qq ? 10 : 9) : 7;
@@ -2067,6 +2079,7 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   a.cand        = chains;
   a.cnt         = chain_cnt;
   a.cap         = chain_cap;
+  a.ld_cand     = chain_cap;
   a.nq          = static_cast<int>(nq);
   a.kb          = kb;
   a.panel_tiles = shape.panel_tiles;

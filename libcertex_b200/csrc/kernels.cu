@@ -1189,62 +1189,150 @@ __device__ __forceinline__ uint8_t* stage_of(void* after_the_arrays)
 // space of id what the chains reach.
 template <typename T>
 constexpr bool kByteRows = std::is_same<T, int8_t>::value || std::is_same<T, uint8_t>::value;
-template <typename T, int METRIC, bool STORED_XX = false>
-__global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 3) verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* queries, size_t qpitch,
-                                     int q0, Candidates cd, int n2max, int k,
-                                     Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list,
-                                     unsigned int* ovf_count, unsigned long long* stats, Refine rf,
-                                     const int32_t* where, const double* sqnorm)
+// |q|^2 as the scores have it, by one thread.
+template <typename T>
+__device__ double query_sqnorm(const Candidates& cd, const void* queries, size_t qpitch, int d, int q)
+{
+  if constexpr (kByteRows<T>) {
+    const T* src = reinterpret_cast<const T*>(static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch);
+    int a        = 0;
+    for (int t = 0; t < d; ++t) { a += static_cast<int>(src[t]) * static_cast<int>(src[t]); }
+    return a;
+  } else {
+    return cd.qq[q];
+  }
+}
+
+// One thread reports an overflowed query with the tighter threshold that the k-th best exact score `kth` among the listed
+// candidates gives (+inf: fewer than k). qq: |q|^2, where the metric's scores have a use for it.
+template <typename T, int METRIC>
+__device__ void report_overflow(const Refine& rf, int q, int qb, const void* queries, size_t qpitch, int d, double qq, double kth,
+                                int32_t* ovf_list, unsigned int* ovf_count)
+{
+  const unsigned int pos = atomicAdd(ovf_count, 1u);
+  ovf_list[pos]          = q;
+  int32_t t              = rf.thr[qb];
+  if (kth < CUDART_INF) {
+    // the screen's value of a row as good as the k-th: <q, x> - |x|^2 / 2 (L2), <q, x> (inner product),
+    // <q, x / |x|> (cosine)
+    
+    if (!kByteRows<T> && METRIC == kL2) {  // the scores had no use for it
+      const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
+      for (int i = 0; i < d; ++i) {
+        const double v = Elems<T>::one(src, i);
+        qq             = __dadd_rn(qq, __dmul_rn(v, v));
+      }
+    }
+    const double value = METRIC == kCos ? sqrt(qq) * (1.0 - 0.5 * kth) : 0.5 * (qq - kth);
+    if (rf.kind == 1) {  // integer values: e = -floor(|x|^2 / 2) only raises a row's value
+      const double cv  = ceil(value);
+      const int32_t tv = cv >= 2147483647.0 ? 0x7fffffff : cv <= -2147483648.0 ? static_cast<int32_t>(0x80000000u)
+                                                                                  : static_cast<int32_t>(cv);
+      t = max(t, tv);
+    } else {             // fp16 codes: the value the pass computes may be lower by half the query's allowance
+      float f = __double2float_rd(value - 0.5 * static_cast<double>(rf.shift[q]));
+      f       = nextafterf(f, -CUDART_INF_F);
+      t       = __float_as_int(fmaxf(f, __int_as_float(t)));
+    }
+  }
+  rf.thr2[pos] = t;
+}
+
+// The three steps (rank, score, sort) are one launch when a block's warps can score a query's rows side by side. With
+// longer lists (k > kSplitK) they are three: then scoring takes a block as many turns as lists are long, the blocks of a few
+// hundred queries fill the GPU unevenly (1.15 waves of them for 512 queries) and those of a few queries leave it idle, so the
+// rows to score are dealt out over the whole grid, 128 to a block, and the lists are sorted by blocks of 1024 threads
+// (sort_lists_kernel). The list of a query and its scores then lie in the memory of its candidates, which are no longer needed.
+// 512 queries, k = 2048, 1 M x 128 halves (2402 rows a query): one launch 341 us; rank 38, score 97, sort 44 us.
+enum : int { kFused = 0, kRank = 1, kScore = 2 };
+constexpr int kSplitK    = 256;
+constexpr int kScoreRows = 128;  // rows a block of the scoring step takes
+template <typename T, int METRIC, bool STORED_XX, int PART>
+__global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 3)
+verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* queries, size_t qpitch, int q0, Candidates cd,
+                     int n2max, int k, Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
+                     unsigned long long* stats, Refine rf, const int32_t* where, const double* sqnorm, int32_t* kept)
 {
   extern __shared__ double sh[];
   __shared__ double s_qq;
   __shared__ uint32_t s_scratch[260];
   __shared__ int s_rows, s_sure, s_seen, s_kept;
+  __shared__ long long s_qq_int;
   constexpr bool kBytes = kByteRows<T>;
-  const int q           = q0 + blockIdx.x;  // number of the query in the call; the candidates are those of its batch
-  const uint32_t c0     = cd.cnt[blockIdx.x];
-  // A candidate list that overflowed (or more rows in it than the block holds): the query is reported in ovf_list. What the
-  // block has are still rows at or above the query's threshold, and the k-th best exact score among them bounds the k-th
-  // neighbour: a tighter threshold for a second pass (rf).
-  const bool listed_all = c0 <= cd.cap;
-  if (!listed_all && rf.thr2 == nullptr) {
-    if (threadIdx.x == 0) { ovf_list[atomicAdd(ovf_count, 1u)] = q; }
-    return;
-  }
-  const int c  = static_cast<int>(min(c0, cd.cap));
+  const int qb          = PART == kScore ? blockIdx.y : blockIdx.x;  // the query's number in its batch
+  const int q           = q0 + qb;                                   // and in the call
+  const Candidate* mine = cd.cand + static_cast<size_t>(qb) * cd.ld;
+  // split: the query's list and scores in the memory of its candidates (ld = n2max entries of 16 bytes)
+  double* far_s    = reinterpret_cast<double*>(const_cast<Candidate*>(mine));
+  int32_t* far_ids = reinterpret_cast<int32_t*>(far_s + n2max);
   double* qd   = sh;
-  double* sc   = kBytes ? sh + (d + 15) / 16 * 2 : sh + d;
+  double* sc   = kBytes ? sh + (d + 15) / 16 * 2 : sh + d;  // fused: the scores and ids in shared memory
   int32_t* ids = reinterpret_cast<int32_t*>(sc + n2max);
-  if (c == 0) {  // no candidate (a slot without a query, or nothing that the query may return)
+  bool over    = false;
+  int m        = 0;
+  auto nothing = [&] {  // no candidate (a slot without a query, or nothing that the query may return)
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
       best_s[static_cast<size_t>(q) * k + t]   = CUDART_INF;
       best_row[static_cast<size_t>(q) * k + t] = -1;
     }
-    return;
+  };
+  auto give_up = [&] {
+    if (threadIdx.x == 0) {
+      ovf_list[atomicAdd(ovf_count, 1u)] = q;
+      if (PART == kRank) { kept[qb] = -1; }
+    }
+  };
+  if constexpr (PART == kScore) {
+    const int32_t w = kept[qb];  // how many rows are scored; negative: the query was given up; bit 30: its list overflowed
+    const int at    = static_cast<int>(blockIdx.x) * kScoreRows;
+    m               = min(kScoreRows, (w < 0 ? 0 : w & 0x3fffffff) - at);
+    if (m <= 0) { return; }
+    sc  = far_s + at;
+    ids = far_ids + at;
   }
-  __shared__ long long s_qq_int;
-  if (threadIdx.x == 0) { s_rows = 0, s_sure = 0, s_seen = 0, s_kept = 0; }
-  if constexpr (kBytes) {
-    // the query's bytes, zero padded to whole 16-byte vectors, in the space of qd; |q|^2 as an integer
-    uint8_t* qbytes    = reinterpret_cast<uint8_t*>(qd);
+  // A candidate list that overflowed (or more rows in it than the block holds): the query is reported in ovf_list. What the
+  // block has are still rows at or above the query's threshold, and the k-th best exact score among them bounds the k-th
+  // neighbour: a tighter threshold for a second pass (rf).
+  const uint32_t c0     = PART == kFused || PART == kRank ? cd.cnt[qb] : 0u;
+  const bool listed_all = c0 <= cd.cap;
+  const int c           = static_cast<int>(min(c0, cd.cap));
+  if constexpr (PART == kFused || PART == kRank) {
+    if (!listed_all && rf.thr2 == nullptr) {
+      give_up();
+      return;
+    }
+    if (c == 0) {
+      if (PART == kFused) {
+        nothing();
+      } else if (threadIdx.x == 0) {
+        kept[qb] = 0;
+      }
+      return;
+    }
+    if (threadIdx.x == 0) { s_rows = 0, s_sure = 0, s_seen = 0, s_kept = 0; }
+  }
+  if constexpr (PART == kFused || PART == kScore) {
     const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
-    const int padded   = (d + 15) / 16 * 16;
-    for (int t = threadIdx.x; t < padded; t += blockDim.x) { qbytes[t] = t < d ? src[t] : 0; }
-  } else {
-    // the query as doubles; |q|^2 in coordinate order comes with the query's code, where the metric has a use for it
-    const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
-    for (int t = threadIdx.x; t < d; t += blockDim.x) { qd[t] = Elems<T>::one(src, t); }
+    if constexpr (kBytes) {
+      // the query's bytes, zero padded to whole 16-byte vectors, in the space of qd
+      uint8_t* qbytes  = reinterpret_cast<uint8_t*>(qd);
+      const int padded = (d + 15) / 16 * 16;
+      for (int t = threadIdx.x; t < padded; t += blockDim.x) { qbytes[t] = t < d ? src[t] : 0; }
+    } else {
+      for (int t = threadIdx.x; t < d; t += blockDim.x) { qd[t] = Elems<T>::one(src, t); }
+    }
+  }
+  if constexpr (!kBytes && PART != kRank) {  // |q|^2 in coordinate order, where the metric's scores have a use for it
     if (threadIdx.x == 0) { s_qq = METRIC == kL2 ? 0.0 : cd.qq[q]; }
   }
   __syncthreads();
-  if constexpr (kBytes) {
-    if (threadIdx.x < 32) {  // |q|^2: 255^2 * 4096 < 2^31
-      const uint32_t* qw = reinterpret_cast<const uint32_t*>(qd);
+  if constexpr (kBytes && PART != kRank) {
+    if (threadIdx.x < 32) {  // |q|^2 as an integer: 255^2 * 4096 < 2^31
+      const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
       int a              = 0;
-      for (int t = threadIdx.x; t < (d + 15) / 16 * 4; t += 32) {
-        const uint32_t w = qw[t];
-        a = std::is_same<T, int8_t>::value ? __dp4a(static_cast<int>(w), static_cast<int>(w), a)
-                                           : static_cast<int>(__dp4a(w, w, static_cast<unsigned>(a)));
+      for (int t = threadIdx.x; t < d; t += 32) {
+        const int v = static_cast<int>(reinterpret_cast<const T*>(src)[t]);
+        a += v * v;
       }
       a = __reduce_add_sync(0xffffffffu, a);
       if (threadIdx.x == 0) {
@@ -1252,139 +1340,127 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
         s_qq     = __ll2double_rn(static_cast<long long>(a));
       }
     }
+    if (PART != kFused) { __syncthreads(); }
   }
-  // ---- values as unsigned keys in their order: of the rows that may be returned, and what every chain reaches (0: nothing)
-  const Candidate* mine = cd.cand + static_cast<size_t>(blockIdx.x) * cd.cap;
-  uint32_t* vkey        = reinterpret_cast<uint32_t*>(sc);
-  int32_t* vid          = reinterpret_cast<int32_t*>(sc) + n2max;
-  uint32_t* reached     = reinterpret_cast<uint32_t*>(ids);
-  auto key_of = [](int32_t product, int32_t e) {
-    if constexpr (kBytes) {
-      return static_cast<uint32_t>(product + e) ^ 0x80000000u;
-    } else {
-      const uint32_t f = __float_as_uint(__int_as_float(product) + __int_as_float(e));
-      return f ^ ((f >> 31) ? 0xffffffffu : 0x80000000u);
-    }
-  };
-  // Without a bitset the ids are looked up for the rows that are scored only: removed rows and padding have e = never.
-  constexpr int32_t kNever = kBytes ? kNeverInit : static_cast<int32_t>(0xff800000u);
-  const bool late          = adm.bits == nullptr && adm.row_labels == nullptr;
-  int sure = 0, seen = 0;
-  for (int i = threadIdx.x; i < c; i += blockDim.x) {
-    const uint4 cv     = __ldg(reinterpret_cast<const uint4*>(mine) + i);  // chain, mask, product
-    const int32_t prod = static_cast<int32_t>(cv.z);
-    uint32_t least     = 0xffffffffu;
-    bool all           = true;
-    for (uint32_t mask = cv.y; mask; mask &= mask - 1) {
-      const int64_t r  = static_cast<int64_t>(cv.x) * kChainRows + __ffs(mask) - 1;
-      const int32_t e  = r < cd.n_rows ? __ldg(cd.init + r) : kNever;
-      int32_t id       = static_cast<int32_t>(r);
-      bool may         = e != kNever;
-      if (may && !late) {
-        id  = __ldg(cd.perm + r);
-        may = admitted(adm, q, id);
-      }
-      ++seen;
-      if (may) {
-        const uint32_t key = key_of(prod, e);
-        const int at       = atomicAdd(&s_rows, 1);
-        least              = min(least, key);
-        if (at < n2max) { vkey[at] = key, vid[at] = id; }
+  if constexpr (PART == kFused || PART == kRank) {
+    // ---- values as unsigned keys in their order: of the rows that may be returned, and what every chain reaches (0: nothing)
+    uint32_t* vkey    = PART == kRank ? reinterpret_cast<uint32_t*>(sh) : reinterpret_cast<uint32_t*>(sc);
+    int32_t* vid      = reinterpret_cast<int32_t*>(vkey) + n2max;
+    uint32_t* reached = PART == kRank ? vkey + 2 * n2max : reinterpret_cast<uint32_t*>(ids);
+    auto key_of = [](int32_t product, int32_t e) {
+      if constexpr (kBytes) {
+        return static_cast<uint32_t>(product + e) ^ 0x80000000u;
       } else {
-        all = false;
+        const uint32_t f = __float_as_uint(__int_as_float(product) + __int_as_float(e));
+        return f ^ ((f >> 31) ? 0xffffffffu : 0x80000000u);
+      }
+    };
+    // Without a bitset the ids are looked up for the rows that are scored only: removed rows and padding have e = never.
+    constexpr int32_t kNever = kBytes ? kNeverInit : static_cast<int32_t>(0xff800000u);
+    const bool late          = adm.bits == nullptr && adm.row_labels == nullptr;
+    int sure = 0, seen = 0;
+    for (int i = threadIdx.x; i < c; i += blockDim.x) {
+      const uint4 cv     = reinterpret_cast<const uint4*>(mine)[i];  // chain, mask, product
+      const int32_t prod = static_cast<int32_t>(cv.z);
+      uint32_t least     = 0xffffffffu;
+      bool all           = true;
+      for (uint32_t mask = cv.y; mask; mask &= mask - 1) {
+        const int64_t r  = static_cast<int64_t>(cv.x) * kChainRows + __ffs(mask) - 1;
+        const int32_t e  = r < cd.n_rows ? __ldg(cd.init + r) : kNever;
+        int32_t id       = static_cast<int32_t>(r);
+        bool may         = e != kNever;
+        if (may && !late) {
+          id  = __ldg(cd.perm + r);
+          may = admitted(adm, q, id);
+        }
+        ++seen;
+        if (may) {
+          const uint32_t key = key_of(prod, e);
+          const int at       = atomicAdd(&s_rows, 1);
+          least              = min(least, key);
+          if (at < n2max) { vkey[at] = key, vid[at] = id; }
+        } else {
+          all = false;
+        }
+      }
+      reached[i] = all ? least : 0u;
+      sure += all ? 1 : 0;
+    }
+    sure = __reduce_add_sync(0xffffffffu, sure);
+    seen = __reduce_add_sync(0xffffffffu, seen);
+    if ((threadIdx.x & 31) == 0) { atomicAdd(&s_sure, sure), atomicAdd(&s_seen, seen); }
+    __syncthreads();
+    const int rows  = min(s_rows, n2max);
+    over            = !listed_all || s_rows > n2max;
+    if (over && rf.thr2 == nullptr) {
+      give_up();
+      return;
+    }
+    uint32_t lowest = 1;
+    if (s_sure >= k && s_rows > k) {
+      lowest = block_kth_largest(reached, c, k, s_scratch);
+      if constexpr (!kBytes) {
+        const uint32_t f = lowest ^ ((lowest >> 31) ? 0x80000000u : 0xffffffffu);
+        const float v    = __fadd_rd(__uint_as_float(f), -cd.shift[q]);
+        const uint32_t g = __float_as_uint(v);
+        lowest           = max(1u, g ^ ((g >> 31) ? 0xffffffffu : 0x80000000u));
       }
     }
-    reached[i] = all ? least : 0u;
-    sure += all ? 1 : 0;
-  }
-  sure = __reduce_add_sync(0xffffffffu, sure);
-  seen = __reduce_add_sync(0xffffffffu, seen);
-  if ((threadIdx.x & 31) == 0) { atomicAdd(&s_sure, sure), atomicAdd(&s_seen, seen); }
-  __syncthreads();
-  const int rows  = min(s_rows, n2max);
-  const bool over = listed_all ? s_rows > n2max : true;
-  if (over && rf.thr2 == nullptr) {
-    if (threadIdx.x == 0) { ovf_list[atomicAdd(ovf_count, 1u)] = q; }
-    return;
-  }
-  uint32_t lowest = 1;
-  if (s_sure >= k && s_rows > k) {
-    lowest = block_kth_largest(reached, c, k, s_scratch);
-    if constexpr (!kBytes) {
-      const uint32_t f = lowest ^ ((lowest >> 31) ? 0x80000000u : 0xffffffffu);
-      const float v    = __fadd_rd(__uint_as_float(f), -cd.shift[q]);
-      const uint32_t g = __float_as_uint(v);
-      lowest           = max(1u, g ^ ((g >> 31) ? 0xffffffffu : 0x80000000u));
-    }
-  }
-  __syncthreads();  // the space of `reached` becomes the list of the rows to score
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-    if (vkey[i] >= lowest) { ids[atomicAdd(&s_kept, 1)] = late ? __ldg(cd.perm + vid[i]) : vid[i]; }
-  }
-  __syncthreads();
-  const int m = s_kept;
-  // One thread reports an overflowed query with the tighter threshold that the k-th best exact score `kth` among the
-  // listed candidates gives (+inf: fewer than k).
-  auto report_overflow = [&](double kth) {
-    const unsigned int pos = atomicAdd(ovf_count, 1u);
-    ovf_list[pos]          = q;
-    int32_t t              = rf.thr[blockIdx.x];
-    if (kth < CUDART_INF) {
-      // the screen's value of a row as good as the k-th: <q, x> - |x|^2 / 2 (L2), <q, x> (inner product),
-      // <q, x / |x|> (cosine)
-      double qq = s_qq;
-      if (!kBytes && METRIC == kL2) {  // the scores had no use for it
-        for (int i = 0; i < d; ++i) { qq = __dadd_rn(qq, __dmul_rn(qd[i], qd[i])); }
-      }
-      const double value = METRIC == kCos ? sqrt(qq) * (1.0 - 0.5 * kth) : 0.5 * (qq - kth);
-      if (rf.kind == 1) {  // integer values: e = -floor(|x|^2 / 2) only raises a row's value
-        const double cv  = ceil(value);
-        const int32_t tv = cv >= 2147483647.0 ? 0x7fffffff : cv <= -2147483648.0 ? static_cast<int32_t>(0x80000000u)
-                                                                                    : static_cast<int32_t>(cv);
-        t = max(t, tv);
-      } else {             // fp16 codes: the value the pass computes may be lower by half the query's allowance
-        float f = __double2float_rd(value - 0.5 * static_cast<double>(rf.shift[q]));
-        f       = nextafterf(f, -CUDART_INF_F);
-        t       = __float_as_int(fmaxf(f, __int_as_float(t)));
+    __syncthreads();  // the space of `reached` becomes the list of the rows to score
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+      if (vkey[i] >= lowest) {
+        (PART == kRank ? far_ids : ids)[atomicAdd(&s_kept, 1)] = late ? __ldg(cd.perm + vid[i]) : vid[i];
       }
     }
-    rf.thr2[pos] = t;
-  };
+    __syncthreads();
+    m = s_kept;
+    if (threadIdx.x == 0 && stats) {
+      atomicAdd(stats + 0, static_cast<unsigned long long>(s_seen));  // rows the screen kept
+      atomicAdd(stats + 1, static_cast<unsigned long long>(m));       // exact scores computed
+    }
+    if (PART == kRank) {
+      if (threadIdx.x == 0) { kept[qb] = m | (over ? 1 << 30 : 0); }
+      return;
+    }
+  }
   if constexpr (kBytes) {
-    // integer scores (below 2^31 in magnitude) and ids sort as one 64-bit key: (score + 2^31) << 32 | id
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(sc);
-    constexpr int kGroups = 32 / kRowLanes;  // rows a warp's load covers
-    const int sub         = threadIdx.x & (kRowLanes - 1);
-    const int group       = (threadIdx.x >> 5) * kGroups + ((threadIdx.x & 31) / kRowLanes);
-    const int n_groups    = (blockDim.x >> 5) * kGroups;
-    for (int i0 = 0; i0 < m; i0 += n_groups * kRowUnroll) {  // the same trips for every lane of a warp
-      int32_t row[kRowUnroll];
-      long long v[kRowUnroll];
+    {
+      // integer scores (below 2^31 in magnitude) and ids sort as one 64-bit key: (score + 2^31) << 32 | id
+      constexpr int kGroups = 32 / kRowLanes;  // rows a warp's load covers
+      const int sub         = threadIdx.x & (kRowLanes - 1);
+      const int group       = (threadIdx.x >> 5) * kGroups + ((threadIdx.x & 31) / kRowLanes);
+      const int n_groups    = (blockDim.x >> 5) * kGroups;
+      for (int i0 = 0; i0 < m; i0 += n_groups * kRowUnroll) {  // the same trips for every lane of a warp
+        int32_t row[kRowUnroll];
+        long long v[kRowUnroll];
 #pragma unroll
-      for (int u = 0; u < kRowUnroll; ++u) {
-        const int i = i0 + u * n_groups + group;
-        row[u]      = i < m ? ids[i] : -1;
-      }
-      if (where) {  // `vectors` is not in id order: row `where[id]` of it holds the vector with that id
-        int32_t at[kRowUnroll];
+        for (int u = 0; u < kRowUnroll; ++u) {
+          const int i = i0 + u * n_groups + group;
+          row[u]      = i < m ? ids[i] : -1;
+        }
+        if (where) {  // `vectors` is not in id order: row `where[id]` of it holds the vector with that id
+          int32_t at[kRowUnroll];
 #pragma unroll
-        for (int u = 0; u < kRowUnroll; ++u) { at[u] = row[u] >= 0 ? __ldg(where + row[u]) : -1; }
-        int_row_scores<T, METRIC>(vectors, pitch, at, d, reinterpret_cast<const uint4*>(qd), s_qq_int, sub, v);
-      } else {
-        int_row_scores<T, METRIC>(vectors, pitch, row, d, reinterpret_cast<const uint4*>(qd), s_qq_int, sub, v);
-      }
+          for (int u = 0; u < kRowUnroll; ++u) { at[u] = row[u] >= 0 ? __ldg(where + row[u]) : -1; }
+          int_row_scores<T, METRIC>(vectors, pitch, at, d, reinterpret_cast<const uint4*>(qd), s_qq_int, sub, v);
+        } else {
+          int_row_scores<T, METRIC>(vectors, pitch, row, d, reinterpret_cast<const uint4*>(qd), s_qq_int, sub, v);
+        }
 #pragma unroll
-      for (int u = 0; u < kRowUnroll; ++u) {
-        const int i = i0 + u * n_groups + group;
-        if (sub == 0 && row[u] >= 0) {
-          keys[i] = (static_cast<unsigned long long>(v[u] + 2147483648ll) << 32) | static_cast<uint32_t>(row[u]);
+        for (int u = 0; u < kRowUnroll; ++u) {
+          const int i = i0 + u * n_groups + group;
+          if (sub == 0 && row[u] >= 0) {
+            keys[i] = (static_cast<unsigned long long>(v[u] + 2147483648ll) << 32) | static_cast<uint32_t>(row[u]);
+          }
         }
       }
     }
+    if (PART == kScore) { return; }
     sort_keys(keys, m);
     if (over) {
       if (threadIdx.x == 0) {
-        report_overflow(k <= m ? __ll2double_rn(static_cast<long long>(keys[k - 1] >> 32) - 2147483648ll) : CUDART_INF);
+        report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, s_qq, k <= m ? __ll2double_rn(static_cast<long long>(keys[k - 1] >> 32) - 2147483648ll) : CUDART_INF, ovf_list, ovf_count);
       }
       return;
     }
@@ -1395,75 +1471,78 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
       best_row[static_cast<size_t>(q) * k + t] = have ? static_cast<int32_t>(key & 0xffffffffull) : -1;
     }
   } else {
-    // Float rows: a thread sums its candidate's coordinates in order (the order of the fp64 reference loop), but the
-    // rows come through shared memory: a warp fetches a 128-byte slab of 32 candidate rows with eight loads that each
-    // cover four whole lines (eight lanes per row), parks it in its tile, and every lane then walks its own row's slab.
-    // Per 512 bytes that is 4 + 4 + 4 memory wavefronts instead of the 32 of a warp whose lanes each load 16 bytes of
-    // a different row.
-    constexpr int V       = Elems<T>::kPerVec;  // coordinates per 16-byte piece
-    const int lane        = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    const int n_pieces    = static_cast<int>((static_cast<size_t>(d) * sizeof(T) + 15) / 16);  // rows are zero padded to the pitch
-    uint8_t* tile         = stage_of(ids + n2max) + static_cast<size_t>(warp) * 32 * kStageStride;
-    const int piece       = lane & 7, row_in_load = lane >> 3;
-    for (int g = warp; g * 32 < m; g += n_warps) {
-      const int i       = g * 32 + lane;
-      const bool ok     = i < m;
-      const int32_t row = ok ? ids[i] : -1;
-      Acc<METRIC, 1, STORED_XX> acc;
-      acc.clear();
-      if constexpr (STORED_XX) {
-        if (ok) { acc.xx = __ldg(sqnorm + row); }
-      }
-      int32_t from[8];  // the rows this lane fetches pieces of
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { from[j] = __shfl_sync(0xffffffffu, row, 4 * j + row_in_load); }
-      // The loads of the next slab are issued as soon as this slab's registers have been parked in the tile, so that
-      // they are in flight while the lanes walk the tile (a warp alone then overlaps its memory latency with its sums).
-      uint4 w[8];
-      auto fetch = [&](int p0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          w[j] = (from[j] >= 0 && p0 + piece < n_pieces)
-                   ? __ldg(reinterpret_cast<const uint4*>(vectors + static_cast<size_t>(from[j]) * pitch) + p0 + piece)
-                   : make_uint4(0, 0, 0, 0);
+    {
+      // Float rows: a thread sums its candidate's coordinates in order (the order of the fp64 reference loop), but the
+      // rows come through shared memory: a warp fetches a 128-byte slab of 32 candidate rows with eight loads that each
+      // cover four whole lines (eight lanes per row), parks it in its tile, and every lane then walks its own row's slab.
+      // Per 512 bytes that is 4 + 4 + 4 memory wavefronts instead of the 32 of a warp whose lanes each load 16 bytes of
+      // a different row.
+      constexpr int V       = Elems<T>::kPerVec;  // coordinates per 16-byte piece
+      const int lane        = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+      const int n_pieces    = static_cast<int>((static_cast<size_t>(d) * sizeof(T) + 15) / 16);  // rows are zero padded to the pitch
+      uint8_t* tile         = stage_of(PART == kFused ? static_cast<void*>(ids + n2max) : static_cast<void*>(qd + d)) + static_cast<size_t>(warp) * 32 * kStageStride;
+      const int piece       = lane & 7, row_in_load = lane >> 3;
+      for (int g = warp; g * 32 < m; g += n_warps) {
+        const int i       = g * 32 + lane;
+        const bool ok     = i < m;
+        const int32_t row = ok ? ids[i] : -1;
+        Acc<METRIC, 1, STORED_XX> acc;
+        acc.clear();
+        if constexpr (STORED_XX) {
+          if (ok) { acc.xx = __ldg(sqnorm + row); }
         }
-      };
-      fetch(0);
-      for (int p0 = 0; p0 < n_pieces; p0 += 8) {
-        __syncwarp();  // every lane is done with the slab before
+        int32_t from[8];  // the rows this lane fetches pieces of
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          *reinterpret_cast<uint4*>(tile + (4 * j + row_in_load) * kStageStride + piece * 16) = w[j];
-        }
-        __syncwarp();
-        if (p0 + 8 < n_pieces) { fetch(p0 + 8); }
-        if (ok) {
-          const int np = min(8, n_pieces - p0);
-          for (int p = 0; p < np; ++p) {
-            const uint4 x4 = *reinterpret_cast<const uint4*>(tile + lane * kStageStride + p * 16);
-            double x[V];
-            Elems<T>::unpack_finite(x4, x);  // screened rows are finite
-            const int t0 = (p0 + p) * V;
-            if (t0 + V <= d) {
-              // the query's doubles two at a time (t0 is a multiple of V, qd is 16-byte aligned): half the
-              // shared-memory instructions of the walk
+        for (int j = 0; j < 8; ++j) { from[j] = __shfl_sync(0xffffffffu, row, 4 * j + row_in_load); }
+        // The loads of the next slab are issued as soon as this slab's registers have been parked in the tile, so that
+        // they are in flight while the lanes walk the tile (a warp alone then overlaps its memory latency with its sums).
+        uint4 w[8];
+        auto fetch = [&](int p0) {
 #pragma unroll
-              for (int e = 0; e < V; e += 2) {
-                const double2 a = *reinterpret_cast<const double2*>(qd + t0 + e);
-                acc.add1(x[e], a.x);
-                acc.add1(x[e + 1], a.y);
+          for (int j = 0; j < 8; ++j) {
+            w[j] = (from[j] >= 0 && p0 + piece < n_pieces)
+                     ? __ldg(reinterpret_cast<const uint4*>(vectors + static_cast<size_t>(from[j]) * pitch) + p0 + piece)
+                     : make_uint4(0, 0, 0, 0);
+          }
+        };
+        fetch(0);
+        for (int p0 = 0; p0 < n_pieces; p0 += 8) {
+          __syncwarp();  // every lane is done with the slab before
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            *reinterpret_cast<uint4*>(tile + (4 * j + row_in_load) * kStageStride + piece * 16) = w[j];
+          }
+          __syncwarp();
+          if (p0 + 8 < n_pieces) { fetch(p0 + 8); }
+          if (ok) {
+            const int np = min(8, n_pieces - p0);
+            for (int p = 0; p < np; ++p) {
+              const uint4 x4 = *reinterpret_cast<const uint4*>(tile + lane * kStageStride + p * 16);
+              double x[V];
+              Elems<T>::unpack_finite(x4, x);  // screened rows are finite
+              const int t0 = (p0 + p) * V;
+              if (t0 + V <= d) {
+                // the query's doubles two at a time (t0 is a multiple of V, qd is 16-byte aligned): half the
+                // shared-memory instructions of the walk
+#pragma unroll
+                for (int e = 0; e < V; e += 2) {
+                  const double2 a = *reinterpret_cast<const double2*>(qd + t0 + e);
+                  acc.add1(x[e], a.x);
+                  acc.add1(x[e + 1], a.y);
+                }
+              } else {
+                for (int e = 0; e < V && t0 + e < d; ++e) { acc.add(x[e], qd, d, t0 + e); }
               }
-            } else {
-              for (int e = 0; e < V && t0 + e < d; ++e) { acc.add(x[e], qd, d, t0 + e); }
             }
           }
         }
+        if (ok) { sc[i] = acc.result(0, s_qq); }
       }
-      if (ok) { sc[i] = acc.result(0, s_qq); }
     }
+    if (PART == kScore) { return; }
     sort_pairs(sc, ids, m);
     if (over) {
-      if (threadIdx.x == 0) { report_overflow(k <= m ? sc[k - 1] : CUDART_INF); }
+      if (threadIdx.x == 0) { report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, s_qq, k <= m ? sc[k - 1] : CUDART_INF, ovf_list, ovf_count); }
       return;
     }
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
@@ -1472,9 +1551,144 @@ __global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 
       best_row[static_cast<size_t>(q) * k + t] = have ? ids[t] : -1;
     }
   }
-  if (threadIdx.x == 0 && stats) {
-    atomicAdd(stats + 0, static_cast<unsigned long long>(s_seen));  // rows the screen kept
-    atomicAdd(stats + 1, static_cast<unsigned long long>(m));  // exact scores computed
+}
+
+// The third step of a split verification, block per query: its k best by (score, id). The scores are spread over kBuckets
+// equal intervals between the smallest and the largest, the buckets are laid out one after the other in shared memory, and a
+// row's place is the beginning of its bucket plus the rows of the bucket that come before it. A bitonic sort of 4096 pairs
+// moves 12 bytes a row 78 times through shared memory, which bounds it: 217 us for 512 lists of 2400 rows; this one takes
+// 44 us. (With most scores in one interval a row is compared with all others, which is as slow as the bitonic sort.)
+constexpr int kSortThreads = 1024;
+constexpr int kSortHeld    = 4;     // rows a thread holds: lists of at most 4096 rows
+constexpr int kBuckets     = 4096;
+template <typename T, int METRIC>
+__global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
+                                                                  int n2max, int k, double* best_s, int32_t* best_row,
+                                                                  int32_t* ovf_list, unsigned int* ovf_count, Refine rf,
+                                                                  const int32_t* kept)
+{
+  extern __shared__ double sh[];  // s [n2max] | id [n2max] | start [kBuckets + 1]
+  __shared__ double s_lo[32], s_hi[32];
+  __shared__ int s_sum[32];
+  double* s           = sh;
+  int32_t* id         = reinterpret_cast<int32_t*>(s + n2max);
+  int32_t* start      = reinterpret_cast<int32_t*>(stage_of(id + n2max));  // 16-byte aligned
+  const int qb        = blockIdx.x, q = q0 + qb;
+  const int lane      = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t w     = kept[qb];
+  if (w < 0) { return; }  // given up
+  const bool over     = (w >> 30) != 0;
+  const int m         = w & 0x3fffffff;
+  const double* far_s = reinterpret_cast<const double*>(cd.cand + static_cast<size_t>(qb) * cd.ld);
+  double x[kSortHeld];
+  int32_t xi[kSortHeld];
+  double lo = CUDART_INF, hi = -CUDART_INF;
+#pragma unroll
+  for (int i = 0; i < kSortHeld; ++i) {
+    const int at = threadIdx.x + i * kSortThreads;
+    x[i]         = CUDART_INF;
+    xi[i]        = 0x7fffffff;
+    if (at < m) {
+      if constexpr (kByteRows<T>) {
+        const unsigned long long key = reinterpret_cast<const unsigned long long*>(far_s)[at];
+        x[i]                         = __ll2double_rn(static_cast<long long>(key >> 32) - 2147483648ll);
+        xi[i]                        = static_cast<int32_t>(key & 0xffffffffull);
+      } else {
+        x[i]  = far_s[at];
+        xi[i] = reinterpret_cast<const int32_t*>(far_s + n2max)[at];
+      }
+      lo = fmin(lo, x[i]);
+      hi = fmax(hi, x[i]);
+    }
+  }
+  for (int i = threadIdx.x; i <= kBuckets; i += kSortThreads) { start[i] = 0; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) { s_lo[warp] = lo, s_hi[warp] = hi; }
+  __syncthreads();
+  lo = s_lo[lane], hi = s_hi[lane];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  // a larger score never has a smaller bucket: the difference and the product round monotonically
+  const double scale = hi > lo ? kBuckets / (hi - lo) : 0.0;
+  auto bucket        = [&](double v) { return min(max(static_cast<int>((v - lo) * scale), 0), kBuckets - 1); };
+  int b[kSortHeld], nth[kSortHeld];
+#pragma unroll
+  for (int i = 0; i < kSortHeld; ++i) {
+    b[i] = -1;
+    if (threadIdx.x + i * kSortThreads < m) {
+      b[i]   = bucket(x[i]);
+      nth[i] = atomicAdd(&start[b[i]], 1);
+    }
+  }
+  __syncthreads();
+  // counts -> first places: four buckets per thread
+  static_assert(kBuckets == 4 * kSortThreads, "one scan step");
+  int4 c        = reinterpret_cast<int4*>(start)[threadIdx.x];
+  const int sum = c.x + c.y + c.z + c.w;
+  int incl      = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) { incl += v; }
+  }
+  if (lane == 31) { s_sum[warp] = incl; }
+  __syncthreads();
+  if (warp == 0) {
+    int t = s_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) { t += v; }
+    }
+    s_sum[lane] = t;
+  }
+  __syncthreads();
+  const int before = incl - sum + (warp > 0 ? s_sum[warp - 1] : 0);
+  reinterpret_cast<int4*>(start)[threadIdx.x] = make_int4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
+  if (threadIdx.x == 0) { start[kBuckets] = m; }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSortHeld; ++i) {
+    if (b[i] >= 0) {
+      const int at = start[b[i]] + nth[i];
+      s[at]        = x[i];
+      id[at]       = xi[i];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSortHeld; ++i) {
+    if (b[i] >= 0) {
+      const int first = start[b[i]], last = start[b[i] + 1];
+      int place       = first;
+      if (first < k) {
+        for (int j = first; j < last; ++j) { place += pair_less(s[j], id[j], x[i], xi[i]) ? 1 : 0; }
+      }
+      if (place < k && !over) {
+        best_s[static_cast<size_t>(q) * k + place]   = x[i];
+        best_row[static_cast<size_t>(q) * k + place] = xi[i];
+      }
+      if (place == k - 1 && over) {
+        report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, METRIC == kL2 && !kByteRows<T> ? 0.0 : query_sqnorm<T>(cd, queries, qpitch, d, q), x[i], ovf_list, ovf_count);
+      }
+    }
+  }
+  if (over) {
+    if (threadIdx.x == 0 && m < k) {
+      report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, 0.0, CUDART_INF, ovf_list, ovf_count);
+    }
+    return;
+  }
+  for (int t = m + threadIdx.x; t < k; t += kSortThreads) {
+    best_s[static_cast<size_t>(q) * k + t]   = CUDART_INF;
+    best_row[static_cast<size_t>(q) * k + t] = -1;
   }
 }
 
@@ -2086,32 +2300,49 @@ void launch_remove(const int64_t* ids, int64_t n_ids, int64_t size, uint8_t* rem
 void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, int metric, const void* queries,
                           size_t qpitch, int nq, int q0, const Candidates& cd, int k,
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
-                          unsigned long long* stats, Refine rf, cudaStream_t s, const int32_t* where, const double* sqnorm)
+                          unsigned long long* stats, Refine rf, cudaStream_t s, int32_t* kept, const int32_t* where, const double* sqnorm)
 {
   if (nq <= 0) { return; }
-  const int n2max   = next_pow2(static_cast<int>(cd.cap));
-  const bool bytes  = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys
-  // a warp of float rows scores 32 rows at a time, and about k to 2 k are left to score
-  const int threads = !bytes && k > 32 ? 256 : 128;
-  // float rows: + 16 bytes of alignment and one staging tile per warp
-  const size_t smem = (bytes ? static_cast<size_t>((d + 15) / 16 * 16) : sizeof(double) * static_cast<size_t>(d)) +
-                      (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2max) +
-                      (bytes ? 0 : 16 + static_cast<size_t>(threads / 32) * 32 * kStageStride);
+  const int n2max  = cd.ld;
+  const bool bytes = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys
+  const bool split = k > kSplitK;
+  const size_t q_bytes = bytes ? static_cast<size_t>((d + 15) / 16 * 16) : sizeof(double) * static_cast<size_t>(d);
+  const size_t pairs   = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2max);
+  // float rows: one staging tile per warp, + 16 bytes of alignment
+  auto tiles = [&](int threads) { return bytes ? size_t(0) : 16 + static_cast<size_t>(threads / 32) * 32 * kStageStride; };
   by_dtype(dtype, [&](auto tag) {
-    using T   = decltype(tag);
-    auto go   = [&](auto kernel) {
+    using T = decltype(tag);
+    auto go = [&](auto kernel, dim3 grid, int threads, size_t smem) {
       allow_smem(kernel, smem);
-      kernel<<<nq, threads, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch, q0, cd, n2max, k, adm,
-                                       best_s, best_row, ovf_list, ovf_count, stats, rf, where, sqnorm);
+      kernel<<<grid, threads, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch, q0, cd, n2max, k, adm,
+                                         best_s, best_row, ovf_list, ovf_count, stats, rf, where, sqnorm, kept);
     };
+    auto all = [&](auto metric, auto stored) {
+      constexpr int M  = decltype(metric)::value;
+      constexpr bool S = decltype(stored)::value;
+      if (!split) {
+        // a warp of float rows scores 32 rows at a time, and about k to 2 k are left to score
+        const int threads = !bytes && k > 32 ? 256 : 128;
+        go(verify_select_kernel<T, M, S, kFused>, dim3(nq), threads, q_bytes + pairs + tiles(threads));
+        return;
+      }
+      go(verify_select_kernel<T, M, S, kRank>, dim3(nq), 256, pairs);
+      // (a batch has at most 32 768 queries: the second grid dimension takes them)
+      go(verify_select_kernel<T, M, S, kScore>, dim3((n2max + kScoreRows - 1) / kScoreRows, nq), 128, q_bytes + tiles(128));
+      const size_t smem = pairs + (kBuckets + 8) * sizeof(int32_t);
+      allow_smem(sort_lists_kernel<T, M>, smem);
+      sort_lists_kernel<T, M><<<nq, kSortThreads, smem, s>>>(queries, qpitch, d, q0, cd, n2max, k, best_s, best_row, ovf_list,
+                                                             ovf_count, rf, kept);
+    };
+    using std::integral_constant;
     if (metric == kL2) {
-      go(verify_select_kernel<T, kL2>);
+      all(integral_constant<int, kL2>{}, std::false_type{});
     } else if (metric == kIP) {
-      go(verify_select_kernel<T, kIP>);
+      all(integral_constant<int, kIP>{}, std::false_type{});
     } else if (sqnorm != nullptr && !bytes) {
-      go(verify_select_kernel<T, kCos, true>);
+      all(integral_constant<int, kCos>{}, std::true_type{});
     } else {
-      go(verify_select_kernel<T, kCos>);
+      all(integral_constant<int, kCos>{}, std::false_type{});
     }
   });
 }

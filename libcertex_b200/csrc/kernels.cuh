@@ -72,8 +72,8 @@ void launch_sort_batch(const int32_t* e, int64_t n, int32_t id0, int64_t row0, c
                        int metric, bool is_float, uint32_t* keys_in, uint32_t* keys_out, int32_t* ids_in, int32_t* ids_out,
                        void* temp, size_t temp_bytes, void* codes, int32_t* perm, int32_t* inv, int32_t* init, cudaStream_t s);
 
-/// What a screen kept: cand [nq, cap] chains per query (see Candidate in screen_i8.cuh), cnt [nq] how many (more than cap:
-/// the list overflowed), and what turns a row of a chain into an id and the value the thresholds are made of: perm [n_rows]
+/// What a screen kept: cand [nq, ld] chains per query (see Candidate in screen_i8.cuh; ld a power of two, at least cap), cnt
+/// [nq] how many (more than cap: the list overflowed), and what turns a row of a chain into an id and the value the thresholds are made of: perm [n_rows]
 /// the id of a code row, init [n_rows] its e (int32, or float bits with fp16 codes; never: a removed row, or no row). fp16
 /// codes also, indexed like the queries: shift (see launch_encode_f16_queries) and, but for the L2 metric, qq (see
 /// launch_query_sqnorms).
@@ -82,6 +82,7 @@ struct Candidates {
   const Candidate* cand;
   const uint32_t* cnt;
   uint32_t cap;
+  int ld;
   int64_t n_rows;
   const int32_t* perm;
   const int32_t* init;
@@ -145,14 +146,15 @@ void launch_compose(int32_t* list, const unsigned int* n, int n_max, const int32
 /**
  * The k best of every query's candidates by (exact fp64 score, id). One block per query: the candidates are ranked by the
  * screen's own values, and those that can belong to the k best are scored. A query with cnt > cap chains, or more than
- * next_pow2(cap) rows in them, is appended to ovf_list and not answered. best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates exist). `where`
+ * ld rows in them, is appended to ovf_list and not answered. best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates exist). `where`
  * (8-bit rows only, optional): `vectors` is not in id order, row where[id] of it holds the vector with that id (the
- * norm-sorted code rows of an index whose vectors live in host memory).
+ * norm-sorted code rows of an index whose vectors live in host memory). kept: scratch of nq ints; the candidates are
+ * overwritten.
  */
 void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, int metric, const void* queries,
                           size_t qpitch, int nq, int q0, const Candidates& cd, int k,
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
-                          unsigned long long* stats, Refine rf, cudaStream_t s, const int32_t* where = nullptr,
+                          unsigned long long* stats, Refine rf, cudaStream_t s, int32_t* kept, const int32_t* where = nullptr,
                           const double* sqnorm = nullptr);
 
 /// out[r] = |x_r|^2 of n float32 / float16 rows, summed over the coordinates in order in fp64 with every product and sum

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
       const uint32_t q  = static_cast<uint32_t>(key >> 48);
       const uint32_t at = atomicAdd(p.cnt + q, 1u);
       if (at < p.cap) {
-        reinterpret_cast<uint4*>(p.cand)[static_cast<size_t>(q) * p.cap + at] =
+        reinterpret_cast<uint4*>(p.cand)[static_cast<size_t>(q) * p.ld_cand + at] =
           make_uint4(static_cast<uint32_t>(key >> 16), static_cast<uint32_t>(key & 0xffffu), static_cast<uint32_t>(product), 0u);
       }
     };

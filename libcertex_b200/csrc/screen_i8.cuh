@@ -50,9 +50,10 @@ struct ScreenArgs {
   const int32_t* thr;             // SCREEN: [nq] keep iff <q, x> + e[x] >= thr[q]
   int32_t* gmax;                  // GROUPMAX: [nq, ld_gmax] maximum of <q, x> + e[x] over every group of 64 rows
   int64_t ld_gmax;
-  Candidate* cand;                // SCREEN: [nq, cap] the chains kept per query, in no order
+  Candidate* cand;                // SCREEN: [nq, ld_cand] the chains kept per query, in no order
   uint32_t* cnt;                  // SCREEN: [nq] chains kept (may exceed cap: overflow, the excess is not written)
   uint32_t cap;
+  uint32_t ld_cand;
   int nq;
   int kb;                         // K blocks of 128 bytes per row
   int panel_tiles;                // query tiles resident in shared memory
