@@ -312,6 +312,10 @@ CERTEX_B200_EXPORT cuvsError_t certexB200ScreenTrace(void* trace, int32_t units)
 CERTEX_B200_EXPORT cuvsError_t certexB200PlanSegments(int32_t n_query_tiles, int32_t n_base_tiles, int32_t panel_tiles,
                                                       int32_t grid, int32_t* out);
 
+/** Filter words of a mask of n bytes in device memory (non-zero: keep): bit j of words[i] = entry 32 i + j, (n + 31) / 32
+ *  words, bits beyond n are 0. Enqueued on the resources' stream. */
+CERTEX_B200_EXPORT cuvsError_t certexB200PackMask(cuvsResources_t res, const uint8_t* mask, int64_t n, uint32_t* words);
+
 /** Test hook (host only): how a search by labels groups its queries: order [n] = 0 .. n - 1 sorted by labels[i], equal
  *  labels in ascending order. */
 CERTEX_B200_EXPORT cuvsError_t certexB200OrderByLabel(const int32_t* labels, int64_t n, int32_t* order);

@@ -569,6 +569,16 @@ cuvsError_t certexB200ScreenRaw(cuvsResources_t res, const void* q_codes, int64_
   });
 }
 
+cuvsError_t certexB200PackMask(cuvsResources_t res, const uint8_t* mask, int64_t n, uint32_t* words)
+{
+  return translate([=] {
+    CERTEX_EXPECTS(n >= 0 && (n == 0 || (mask != nullptr && words != nullptr)), "certex: null argument");
+    CERTEX_EXPECTS(n < (int64_t(1) << 43), "certex: the mask is too long");
+    launch_pack_mask(mask, n, words, as_res(res).stream);
+    CERTEX_CUDA(cudaGetLastError());
+  });
+}
+
 cuvsError_t certexB200ScreenTrace(void* trace, int32_t units)
 {
   return translate([=] {

@@ -137,6 +137,8 @@ struct Refine {
 /// entry: a zero row); rows n .. n_pad - 1 are zeros.
 void launch_gather_rows(const void* in, size_t in_pitch, const int32_t* sel, int64_t n, int64_t n_pad, void* out,
                         size_t out_pitch, size_t row_bytes, cudaStream_t s);
+/// words [(n + 31) / 32]: bit j of word i = entry 32 i + j of the byte mask (non-zero: set); bits beyond n are 0.
+void launch_pack_mask(const uint8_t* mask, int64_t n, uint32_t* words, cudaStream_t s);
 /// best_s / best_row rows sel[i] = rows i of s2 / row2, i < n (negative sel[i]: skipped).
 void launch_scatter_best(const double* s2, const int32_t* row2, const int32_t* sel, int n, int k, double* best_s,
                          int32_t* best_row, cudaStream_t s);

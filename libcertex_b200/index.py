@@ -66,10 +66,10 @@ def _to_dtype(t, dtype):
 
 def pack_mask(mask):
     """Boolean mask (flattened row-major) as uint32 filter words: bit j of word i is entry 32 i + j."""
-    b = mask.reshape(-1).to(device="cuda", dtype=torch.int64)
-    b = torch.nn.functional.pad(b, (0, (-b.numel()) % 32)).view(-1, 32)
-    w = (b << torch.arange(32, device=b.device)).sum(1)
-    return torch.where(w >= 2**31, w - 2**32, w).to(torch.int32).contiguous()
+    b = mask.reshape(-1).to(device="cuda", dtype=torch.bool).contiguous()
+    words = torch.empty(((b.numel() + 31) // 32,), dtype=torch.int32, device="cuda")
+    L.check(L.lib().certexB200PackMask(L.resources(), b.data_ptr(), b.numel(), words.data_ptr()))
+    return words
 
 
 class search_stats:
