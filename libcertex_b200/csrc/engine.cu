@@ -789,7 +789,7 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   // 8-bit vectors kept in host memory: the exact stage reads the candidates' code rows, which are the vectors
   const bool from_codes = host_vectors_ && screen_kind_ == 1;
   launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, queries, row_bytes,
-                       nq, q0, Candidates{cand, cnt, cap, ld_cand, n, perm_, init_, shift, qq}, k, adm, best_s, best_row, ovf_list, ovf_count,
+                       nq, q0, Candidates{cand, cnt, cap, ld_cand, n, perm_, init_, shift, qq, 0, 0}, k, adm, best_s, best_row, ovf_list, ovf_count,
                        stats, rf, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
   CERTEX_CUDA(cudaGetLastError());
 }
@@ -928,6 +928,7 @@ std::vector<int32_t> order_by_label(const std::vector<int32_t>& lab)
 
 /// The queries of one label in a search by labels.
 struct LabelRun {
+  int32_t label     = 0;
   int64_t part_off  = 0;  // the label's entries in the partition
   int64_t n_in_part = 0;
   int64_t tile0     = 0;  // its first tile in the label-ordered copy of the screen's rows
@@ -994,7 +995,7 @@ size_t plan_routed(const std::vector<LabelRun>& runs, size_t r0, size_t r1, cons
 // One class of routed runs (groups of 64 rows, or with `fine` of 16): passes of at most 32 768 query slots. Returns the
 // pairs the screens kept; runs' queries whose candidate list overflowed are appended to `dense`.
 unsigned long long Index::search_routed(const Resources& res, const void* q, size_t qpitch, int k,
-                                        std::vector<LabelRun>& routed, const bool fine, double* best_s, int32_t* best_row,
+                                        std::vector<LabelRun>& routed, const bool fine, int64_t n_tail, double* best_s, int32_t* best_row,
                                         SearchStats* st, std::vector<LabelRun>& dense) const
 {
   unsigned long long pairs = 0;
@@ -1077,12 +1078,20 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     const int n_groups   = static_cast<int>(max_tiles) * per_tile;
     const int64_t ld_g   = round_up(n_groups, 8);
     // the host's tables of the pass, sent in one copy (segs_g ...: the threshold pass over the leading tiles of every label)
+    // the queries of every label, for the rows that are newer than the partition
+    std::vector<int32_t> run_label, run_slot0, run_slots;
+    for (size_t r = r0; r < r1 && n_tail > 0; ++r) {
+      run_label.push_back(routed[r].label);
+      run_slot0.push_back(q_tile0[r - r0] * static_cast<int32_t>(kQTile));
+      run_slots.push_back(static_cast<int32_t>(routed[r].queries.size()));
+    }
     const std::vector<std::pair<const void*, size_t>> tables = {
       {slot_query.data(), slot_query.size() * 4},      {slot_ng.data(), slot_ng.size() * 4},
       {segs.data(), segs.size() * sizeof(ScreenSeg)},  {col0.data(), col0.size() * sizeof(int)},
       {seg_begin.data(), seg_begin.size() * sizeof(int)}, {segs_g.data(), segs_g.size() * sizeof(ScreenSeg)},
       {col0_g.data(), col0_g.size() * sizeof(int)},    {seg_begin_g.data(), seg_begin_g.size() * sizeof(int)},
-      {step_g.data(), step_g.size() * sizeof(int)}};
+      {step_g.data(), step_g.size() * sizeof(int)},    {run_label.data(), run_label.size() * 4},
+      {run_slot0.data(), run_slot0.size() * 4},        {run_slots.data(), run_slots.size() * 4}};
     uint8_t* d_tables = scratch.get<uint8_t>(Resources::upload_bytes(tables));
     std::vector<size_t> at;
     res.upload(tables, d_tables, at);
@@ -1179,11 +1188,18 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     mark();
     CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
     mark();
+    if (n_tail > 0) {
+      const TailRows tail{labels_, removed_, inv_, static_cast<const uint8_t*>(codes_), init_, cp, f16 ? 2 : dtype_ == kI8 ? 1 : 0,
+                          static_cast<int32_t>(n_part_), static_cast<int32_t>(n_tail), n_lrows_};
+      launch_tail(tail, q_codes, thr, reinterpret_cast<int32_t*>(d_tables + at[9]), reinterpret_cast<int32_t*>(d_tables + at[10]),
+                  reinterpret_cast<int32_t*>(d_tables + at[11]), static_cast<int>(r1 - r0), cand, cnt, cap, ld_cand, res.stream);
+      st->launches += 1;
+    }
     Admit plain{};
     plain.removed = removed_;
     const bool from_codes = host_vectors_ && screen_kind_ == 1;
     launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, q_rows,
-                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq}, k, plain, slot_s, slot_row,
+                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq, static_cast<int32_t>(n_part_), static_cast<int32_t>(n_tail)}, k, plain, slot_s, slot_row,
                          ovf_list, d_flag, d_stats, Refine{}, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
     launch_scatter_best(slot_s, slot_row, d_slot_q, ns, k, best_s, best_row, res.stream);
     CERTEX_CUDA(cudaGetLastError());
@@ -1239,7 +1255,7 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   // The one host decision of the path: which queries share a label. Their labels come to the host and the queries are
   // ordered by label. A label with enough rows for a threshold (2k groups of 64) is screened on the tensor cores
   // against its block of the label-ordered copy of the code rows (routed pass); the other labels, the queries whose
-  // candidate list overflowed, and every label when rows were added after the partition, are scored densely: every
+  // candidate list overflowed, and every label when the partition is far out of date, are scored densely: every
   // label becomes a group (queries x that label's partition entries + the rows added since), and the groups are
   // scored, selected from and translated to ids in waves of bounded score memory, three launches per wave.
   std::vector<int32_t> lab(static_cast<size_t>(nq));
@@ -1248,13 +1264,16 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   const std::vector<int32_t> order = order_by_label(lab);  // the device waits for the host here: no comparison sort
 
   const int64_t n_tail = n - n_part_;
-  const bool can_route = lcodes_ != nullptr && screen_kind_ != 0 && !code_overflow_ && n_tail == 0 && test_mode_ != 3;
+  // Rows that are newer than the partition are screened one by one against the queries of their label (tail_kernel), with the
+  // thresholds of the partition's rows. With a tail longer than half the partition those would keep too much of it.
+  const bool can_route = lcodes_ != nullptr && screen_kind_ != 0 && !code_overflow_ && 2 * n_tail <= n_part_ && test_mode_ != 3;
   std::vector<LabelRun> routed, routed_fine, dense;
   for (int i = 0; i < nq;) {
     const int32_t l = lab[order[static_cast<size_t>(i)]];
     int j           = i;
     while (j < nq && lab[order[static_cast<size_t>(j)]] == l) { ++j; }
     LabelRun run;
+    run.label     = l;
     const auto it = std::lower_bound(part_labels_.begin(), part_labels_.end(), l);
     if (l >= 0 && it != part_labels_.end() && *it == l) {
       const size_t at = static_cast<size_t>(it - part_labels_.begin());
@@ -1278,8 +1297,8 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   unsigned long long pairs = 0;
 
   // ------------------------------------------------------------------ routed passes
-  pairs += search_routed(res, q, qpitch, k, routed, false, best_s, best_row, st, dense);
-  pairs += search_routed(res, q, qpitch, k, routed_fine, true, best_s, best_row, st, dense);
+  pairs += search_routed(res, q, qpitch, k, routed, false, n_tail, best_s, best_row, st, dense);
+  pairs += search_routed(res, q, qpitch, k, routed_fine, true, n_tail, best_s, best_row, st, dense);
 
   // ------------------------------------------------------------------ dense groups
   std::vector<int32_t> dorder;

@@ -286,7 +286,7 @@ class Index {
                                       double* best_s, int32_t* best_row, int64_t n, SearchStats* st) const;
   /// The routed (screened) part of a search by labels for one class of labels; see engine.cu.
   unsigned long long search_routed(const Resources& res, const void* q, size_t qpitch, int k, std::vector<LabelRun>& routed,
-                                   bool fine, double* best_s, int32_t* best_row, SearchStats* st,
+                                   bool fine, int64_t n_tail, double* best_s, int32_t* best_row, SearchStats* st,
                                    std::vector<LabelRun>& dense) const;
 
   IndexParams params_;

@@ -669,6 +669,82 @@ __global__ void candidate_rows_kernel(const Candidate* cand, const uint32_t* cnt
   }
 }
 
+// A warp per row of the tail. Its code stays in the lanes' registers as far as it fits (16 bytes a lane: 512 bytes) while the
+// queries of its label pass by; their codes come from L2. The sum of a float pair is made of 32 partial sums and a tree, far
+// inside the bound of the tensor cores' sums that the thresholds allow for.
+template <int KIND>
+__global__ void tail_kernel(TailRows t, const uint8_t* q_codes, const int32_t* thr, const int32_t* label, const int32_t* slot0,
+                            const int32_t* n_slots, int n_runs, Candidate* cand, uint32_t* cnt, uint32_t cap, int ld)
+{
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < t.n_tail; i += warps) {
+    const int32_t id = t.tail_id0 + i;
+    if (t.removed[id]) { continue; }
+    const int32_t l = t.row_labels[id];
+    int lo = 0, hi = n_runs - 1;  // first run whose label is not below l
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (label[mid] < l) {
+        lo = mid + 1;
+      } else {
+        hi = mid;
+      }
+    }
+    if (l < 0 || label[lo] != l) { continue; }
+    const int32_t row  = t.inv[id];
+    const int32_t e    = t.init[row];
+    const uint4* x     = reinterpret_cast<const uint4*>(t.codes + static_cast<size_t>(row) * t.code_pitch);
+    const int n_vec    = static_cast<int>(t.code_pitch / 16);
+    const uint4 zero   = make_uint4(0, 0, 0, 0);
+    const uint4 x0     = lane < n_vec ? __ldg(x + lane) : zero;
+    auto add = [](const uint4& a, const uint4& b, int& isum, float& fsum) {
+      const uint32_t u[4] = {a.x, a.y, a.z, a.w}, v[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (KIND == 2) {
+          const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&u[j]));
+          const float2 q = __half22float2(*reinterpret_cast<const __half2*>(&v[j]));
+          fsum           = fmaf(p.x, q.x, fsum);
+          fsum           = fmaf(p.y, q.y, fsum);
+        } else if constexpr (KIND == 1) {
+          isum = __dp4a(static_cast<int>(u[j]), static_cast<int>(v[j]), isum);
+        } else {
+          isum = static_cast<int>(__dp4a(u[j], v[j], static_cast<unsigned>(isum)));
+        }
+      }
+    };
+    const int s1 = slot0[lo] + n_slots[lo];
+    for (int s = slot0[lo]; s < s1; ++s) {
+      const uint4* q = reinterpret_cast<const uint4*>(q_codes + static_cast<size_t>(s) * t.code_pitch);
+      int isum       = 0;
+      float fsum     = 0;
+      if (lane < n_vec) { add(x0, __ldg(q + lane), isum, fsum); }
+      for (int c = lane + 32; c < n_vec; c += 32) { add(__ldg(x + c), __ldg(q + c), isum, fsum); }
+      int32_t value;
+      bool hit;
+      if constexpr (KIND == 2) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) { fsum += __shfl_xor_sync(0xffffffffu, fsum, o); }
+        const float v = fsum + __int_as_float(e);
+        value         = __float_as_int(v);
+        hit           = v >= __int_as_float(thr[s]);
+      } else {
+        value = __reduce_add_sync(0xffffffffu, isum) + e;
+        hit   = value >= thr[s];
+      }
+      if (lane == 0 && hit) {
+        const uint32_t at = atomicAdd(cnt + s, 1u);
+        if (at < cap) {
+          const int64_t r = t.n_rows + i;  // n_rows is a multiple of the chain length
+          reinterpret_cast<uint4*>(cand)[static_cast<size_t>(s) * ld + at] =
+            make_uint4(static_cast<uint32_t>(r / kChainRows), 1u << (r % kChainRows), static_cast<uint32_t>(value), 0u);
+        }
+      }
+    }
+  }
+}
+
 // rows [q, 0 : n_parts * k] = the lists parts[p, q, 0:k] of every part side by side.
 __global__ void union_rows_kernel(const int32_t* parts, int n_parts, int nq, int k, int32_t* rows, int64_t ld)
 {
@@ -1347,6 +1423,7 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
     uint32_t* vkey    = PART == kRank ? reinterpret_cast<uint32_t*>(sh) : reinterpret_cast<uint32_t*>(sc);
     int32_t* vid      = reinterpret_cast<int32_t*>(vkey) + n2max;
     uint32_t* reached = PART == kRank ? vkey + 2 * n2max : reinterpret_cast<uint32_t*>(ids);
+    auto id_of = [&](int64_t r) { return r < cd.n_rows ? __ldg(cd.perm + r) : cd.tail_id0 + static_cast<int32_t>(r - cd.n_rows); };
     auto key_of = [](int32_t product, int32_t e) {
       if constexpr (kBytes) {
         return static_cast<uint32_t>(product + e) ^ 0x80000000u;
@@ -1366,11 +1443,11 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
       bool all           = true;
       for (uint32_t mask = cv.y; mask; mask &= mask - 1) {
         const int64_t r  = static_cast<int64_t>(cv.x) * kChainRows + __ffs(mask) - 1;
-        const int32_t e  = r < cd.n_rows ? __ldg(cd.init + r) : kNever;
+        const int32_t e  = r < cd.n_rows ? __ldg(cd.init + r) : r < cd.n_rows + cd.n_tail ? 0 : kNever;
         int32_t id       = static_cast<int32_t>(r);
         bool may         = e != kNever;
         if (may && !late) {
-          id  = __ldg(cd.perm + r);
+          id  = id_of(r);
           may = admitted(adm, q, id);
         }
         ++seen;
@@ -1409,7 +1486,7 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
     __syncthreads();  // the space of `reached` becomes the list of the rows to score
     for (int i = threadIdx.x; i < rows; i += blockDim.x) {
       if (vkey[i] >= lowest) {
-        (PART == kRank ? far_ids : ids)[atomicAdd(&s_kept, 1)] = late ? __ldg(cd.perm + vid[i]) : vid[i];
+        (PART == kRank ? far_ids : ids)[atomicAdd(&s_kept, 1)] = late ? id_of(vid[i]) : vid[i];
       }
     }
     __syncthreads();
@@ -2184,6 +2261,15 @@ void launch_candidate_rows(const Candidate* cand, const uint32_t* cnt, uint32_t 
                            int32_t* rows, uint32_t row_cap, cudaStream_t s)
 {
   if (nq > 0) { candidate_rows_kernel<<<nq, 128, 0, s>>>(cand, cnt, cap, n_rows, row_cnt, rows, row_cap); }
+}
+
+void launch_tail(const TailRows& t, const uint8_t* q_codes, const int32_t* thr, const int32_t* label, const int32_t* slot0,
+                 const int32_t* n_slots, int n_runs, Candidate* cand, uint32_t* cnt, uint32_t cap, int ld, cudaStream_t s)
+{
+  if (t.n_tail <= 0 || n_runs <= 0) { return; }
+  const auto grid = static_cast<unsigned>(std::min<int64_t>((static_cast<int64_t>(t.n_tail) + 7) / 8, 148 * 8));
+  auto kernel     = t.kind == 2 ? tail_kernel<2> : t.kind == 1 ? tail_kernel<1> : tail_kernel<0>;
+  kernel<<<grid, 256, 0, s>>>(t, q_codes, thr, label, slot0, n_slots, n_runs, cand, cnt, cap, ld);
 }
 
 void launch_chain_max(const int32_t* init, int64_t c0, int64_t n, int32_t* cmax, bool is_float, cudaStream_t s)

@@ -74,7 +74,8 @@ void launch_sort_batch(const int32_t* e, int64_t n, int32_t id0, int64_t row0, c
 
 /// What a screen kept: cand [nq, ld] chains per query (see Candidate in screen_i8.cuh; ld a power of two, at least cap), cnt
 /// [nq] how many (more than cap: the list overflowed), and what turns a row of a chain into an id and the value the thresholds are made of: perm [n_rows]
-/// the id of a code row, init [n_rows] its e (int32, or float bits with fp16 codes; never: a removed row, or no row). fp16
+/// the id of a code row, init [n_rows] its e (int32, or float bits with fp16 codes; never: a removed row, or no row).
+/// Code rows n_rows + t, t < n_tail, stand for the ids tail_id0 + t; their entries hold the value itself (launch_tail). fp16
 /// codes also, indexed like the queries: shift (see launch_encode_f16_queries) and, but for the L2 metric, qq (see
 /// launch_query_sqnorms).
 struct Candidate;
@@ -88,7 +89,27 @@ struct Candidates {
   const int32_t* init;
   const float* shift;
   const double* qq;
+  int32_t tail_id0;
+  int32_t n_tail;
 };
+
+/// The rows that were added after the label partition (ids tail_id0 .. tail_id0 + n_tail - 1), screened against the queries of
+/// their label: a row whose value reaches a query's threshold is appended to the query's candidates. Run r of n_runs holds the
+/// queries (slots) slot0[r] .. slot0[r] + n_slots[r] - 1, whose label is label[r] (ascending, no label twice).
+struct TailRows {
+  const int32_t* row_labels;   // [ids]
+  const uint8_t* removed;      // [ids]
+  const int32_t* inv;          // [ids] id -> code row
+  const uint8_t* codes;        // code rows of code_pitch bytes
+  const int32_t* init;         // e of the code rows
+  size_t code_pitch;
+  int kind;                    // 0 uint8, 1 int8, 2 fp16 codes
+  int32_t tail_id0;
+  int32_t n_tail;
+  int64_t n_rows;              // see Candidates
+};
+void launch_tail(const TailRows& t, const uint8_t* q_codes, const int32_t* thr, const int32_t* label, const int32_t* slot0,
+                 const int32_t* n_slots, int n_runs, Candidate* cand, uint32_t* cnt, uint32_t cap, int ld, cudaStream_t s);
 
 /// The rows of the candidate lists (row numbers below n_rows): row_cnt [nq] += how many, rows [nq, row_cap] the first of them.
 void launch_candidate_rows(const Candidate* cand, const uint32_t* cnt, uint32_t cap, int nq, int64_t n_rows, uint32_t* row_cnt,
