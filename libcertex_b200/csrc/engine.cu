@@ -19,6 +19,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <istream>
+#include <map>
+#include <mutex>
 #include <ostream>
 #include <vector>
 
@@ -43,28 +45,117 @@ inline int next_pow2(uint32_t v)
   return p;
 }
 
+// ------------------------------------------------------------------ memory of the indexes
+// The arrays of an index come from a memory pool of their device, so that a program which makes and drops indexes (one per
+// prompt, one per deduplicated block) does not pay the driver for mapping and unmapping memory each time: fifteen cudaMalloc
+// and as many cudaFree were most of such a call (a cache of 8 x 32 768 keys built, asked and dropped: 7.15 -> 1.70 ms; an index of
+// 200 000 x 96 halves built, searched 5000 times and dropped: 4.27 -> 0.97 ms). The pool keeps at most kPoolKeep bytes that no index uses: what
+// lies above goes back to the driver at the next synchronisation, and all of it when an allocation fails.
+constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+
+cudaMemPool_t index_pool(int device)
+{
+  static std::mutex mutex;
+  static std::map<int, cudaMemPool_t> pools;
+  std::lock_guard<std::mutex> lock(mutex);
+  auto it = pools.find(device);
+  if (it != pools.end()) { return it->second; }
+  cudaMemPoolProps props{};
+  props.allocType     = cudaMemAllocationTypePinned;
+  props.handleTypes   = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id   = device;
+  cudaMemPool_t pool  = nullptr;
+  CERTEX_CUDA(cudaMemPoolCreate(&pool, &props));
+  uint64_t keep = kPoolKeep;
+  CERTEX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  pools[device] = pool;
+  return pool;
+}
+
+/// Gives back what the pools of the device keep and nobody uses (an allocation failed).
+void trim_pools(int device)
+{
+  cudaGetLastError();
+  cudaDeviceSynchronize();
+  cudaMemPool_t scratch = nullptr;
+  if (cudaDeviceGetDefaultMemPool(&scratch, device) == cudaSuccess) { cudaMemPoolTrimTo(scratch, 0); }
+  cudaMemPoolTrimTo(index_pool(device), 0);
+}
+
+/// An array of an index, for use on `stream`, and on others once the host has waited for it.
+template <typename T>
+void index_alloc(T** out, size_t bytes, int device, cudaStream_t stream)
+{
+  void* p       = nullptr;
+  bytes         = std::max<size_t>(bytes, 1);
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, index_pool(device), stream);
+  if (e == cudaErrorMemoryAllocation) {
+    trim_pools(device);
+    e = cudaMallocFromPoolAsync(&p, bytes, index_pool(device), stream);
+  }
+  CERTEX_CUDA(e);
+  *out = static_cast<T*>(p);
+}
+
+/// Arrays of an index that nobody will be given any more. Work that reads them may still be enqueued on any stream (a search
+/// that returned before the device was done): the device is waited for first, as cudaFree does.
+void index_free(int device, const std::vector<void*>& arrays)
+{
+  bool any = false;
+  for (void* p : arrays) { any |= p != nullptr; }
+  if (!any) { return; }
+  int current = device;
+  cudaGetDevice(&current);
+  if (current != device) { cudaSetDevice(device); }
+  cudaDeviceSynchronize();
+  for (void* p : arrays) {
+    if (p) { cudaFreeAsync(p, cudaStreamPerThread); }
+  }
+  if (current != device) { cudaSetDevice(current); }
+}
+
 // ------------------------------------------------------------------ stream-ordered scratch memory
+// Small pieces are cut from chunks: a search of few queries takes a dozen of them, and each call of the allocator costs as
+// much as a launch.
 struct Scratch {
+  static constexpr size_t kSmall = size_t(64) << 10, kChunk = size_t(256) << 10;
   cudaStream_t stream;
   std::vector<void*> ptrs;
+  uint8_t* chunk = nullptr;
+  size_t left    = 0;
   explicit Scratch(cudaStream_t s) : stream(s) {}
   ~Scratch()
   {
     for (void* p : ptrs) { cudaFreeAsync(p, stream); }
   }
-  template <typename T>
-  T* get(size_t count)
+  void* take(size_t bytes)
   {
-    void* p             = nullptr;
-    const size_t bytes  = std::max<size_t>(count, 1) * sizeof(T);
-    const cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    void* p       = nullptr;
+    cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    if (e == cudaErrorMemoryAllocation) {
+      int device = 0;
+      CERTEX_CUDA(cudaGetDevice(&device));
+      trim_pools(device);
+      e = cudaMallocAsync(&p, bytes, stream);
+    }
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();  // the failed allocation leaves nothing behind: the error is reported, not kept
       throw OutOfMemory("certex: out of device memory (" + std::to_string(bytes) + " bytes of scratch)");
     }
     CERTEX_CUDA(e);
     ptrs.push_back(p);
-    return static_cast<T*>(p);
+    return p;
+  }
+  template <typename T>
+  T* get(size_t count)
+  {
+    const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    if (bytes > kSmall) { return static_cast<T*>(take(bytes)); }
+    if (bytes > left) { chunk = static_cast<uint8_t*>(take(kChunk)), left = kChunk; }
+    T* p = reinterpret_cast<T*>(chunk);
+    chunk += bytes, left -= bytes;
+    return p;
   }
 };
 
@@ -270,6 +361,7 @@ Resources::~Resources()
   if (pinned_) { cudaFreeHost(pinned_); }
   if (staging_) { cudaFreeHost(staging_); }
   if (staging_done_) { cudaEventDestroy(staging_done_); }
+  if (side_) { cudaStreamDestroy(side_); }
 }
 
 size_t Resources::upload_bytes(const std::vector<std::pair<const void*, size_t>>& pieces)
@@ -305,6 +397,12 @@ void Resources::upload(const std::vector<std::pair<const void*, size_t>>& pieces
 
 void Resources::sync() const { CERTEX_CUDA(cudaStreamSynchronize(stream)); }
 
+cudaStream_t Resources::side_stream() const
+{
+  if (!side_) { CERTEX_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking)); }
+  return side_;
+}
+
 void* Resources::pinned_block(int slot) const
 {
   if (!pinned_) { CERTEX_CUDA(cudaHostAlloc(&pinned_, 256 * kPinnedSlots, cudaHostAllocDefault)); }
@@ -337,7 +435,7 @@ Index::Index(const Resources& res, const IndexParams& params, int dtype, int64_t
   }
   kb_ = static_cast<int>(code_pitch_ / 128);
   if (screen_kind_ == 2) {
-    CERTEX_CUDA(cudaMalloc(&maxima_, 4 * sizeof(unsigned int)));
+    index_alloc(&maxima_, 4 * sizeof(unsigned int), device_, res.stream);
     CERTEX_CUDA(cudaMemsetAsync(maxima_, 0, 4 * sizeof(unsigned int), res.stream));
     res.sync();
   }
@@ -346,7 +444,7 @@ Index::Index(const Resources& res, const IndexParams& params, int dtype, int64_t
 namespace {
 /// The vectors of an index: device memory, or page-locked host memory mapped into the device's address space (with
 /// unified addressing the same pointer serves host and device).
-void* alloc_vectors(size_t bytes, bool on_host)
+void* alloc_vectors(size_t bytes, bool on_host, int device, cudaStream_t stream)
 {
   void* p = nullptr;
   if (on_host) {
@@ -357,38 +455,22 @@ void* alloc_vectors(size_t bytes, bool on_host)
     }
     CERTEX_CUDA(e);
   } else {
-    CERTEX_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 1)));
+    index_alloc(&p, bytes, device, stream);
   }
   return p;
-}
-void free_vectors(void* p, bool on_host)
-{
-  if (on_host) {
-    cudaFreeHost(p);
-  } else {
-    cudaFree(p);
-  }
 }
 }  // namespace
 
 Index::~Index()
 {
-  free_vectors(vectors_, host_vectors_);
-  cudaFree(removed_);
-  cudaFree(labels_);
-  cudaFree(part_ids_);
-  cudaFree(lcodes_), cudaFree(linit_), cudaFree(lcmax_), cudaFree(lperm_), cudaFree(linv_);
-  cudaFree(codes_);
-  cudaFree(perm_);
-  cudaFree(inv_);
-  cudaFree(init_);
-  cudaFree(cmax_);
-  cudaFree(maxima_);
-  cudaFree(sqnorm_);
-  for (auto& kv : plans_) { cudaFree(kv.second.segs), cudaFree(kv.second.begin); }
+  std::vector<void*> arrays{host_vectors_ ? nullptr : vectors_, removed_, labels_, part_ids_, lcodes_, linit_, lcmax_, lperm_, linv_,
+                            codes_, perm_, inv_, init_, cmax_, maxima_, sqnorm_};
+  for (auto& kv : plans_) { arrays.push_back(kv.second.segs); }
+  index_free(device_, arrays);
+  if (host_vectors_) { cudaFreeHost(vectors_); }
 }
 
-Index::DevicePlan Index::device_plan(int nqt, int nt, int panel_tiles, int grid, int chunk_tiles) const
+Index::DevicePlan Index::device_plan(const Resources& res, int nqt, int nt, int panel_tiles, int grid, int chunk_tiles) const
 {
   const std::array<int, 5> key{nqt, nt, panel_tiles, grid, chunk_tiles};
   std::lock_guard<std::mutex> lock(plans_mutex_);
@@ -397,18 +479,20 @@ Index::DevicePlan Index::device_plan(int nqt, int nt, int panel_tiles, int grid,
   DevicePlan d;
   if (plans_.size() >= kMaxPlans) { return d; }  // shapes keep changing (an index that grows between searches): not kept
   const ChunkedPlan plan = plan_chunked(nqt, nt, panel_tiles, grid, chunk_tiles);
-  CERTEX_CUDA(cudaMalloc(&d.segs, std::max<size_t>(plan.segs.size(), 1) * sizeof(ScreenSeg)));
-  if (cudaMalloc(&d.begin, plan.begin.size() * sizeof(int)) != cudaSuccess) {
-    cudaFree(d.segs);
-    throw Error("certex: out of device memory for a work split");
-  }
-  // blocking copies: the plan is complete before any stream of any thread can be given it
-  cudaError_t e = cudaMemcpy(d.segs, plan.segs.data(), plan.segs.size() * sizeof(ScreenSeg), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) { e = cudaMemcpy(d.begin, plan.begin.data(), plan.begin.size() * sizeof(int), cudaMemcpyHostToDevice); }
+  const size_t seg_bytes = (plan.segs.size() * sizeof(ScreenSeg) + 255) / 256 * 256;
+  uint8_t* both          = nullptr;
+  const cudaStream_t st  = res.side_stream();
+  index_alloc(&both, seg_bytes + plan.begin.size() * sizeof(int), device_, st);
+  // the host waits for the copies: the plan is complete before any stream of any thread can be given it
+  cudaError_t e = cudaMemcpyAsync(both, plan.segs.data(), plan.segs.size() * sizeof(ScreenSeg), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) { e = cudaMemcpyAsync(both + seg_bytes, plan.begin.data(), plan.begin.size() * sizeof(int), cudaMemcpyHostToDevice, st); }
+  if (e == cudaSuccess) { e = cudaStreamSynchronize(st); }
   if (e != cudaSuccess) {
-    cudaFree(d.segs), cudaFree(d.begin);
+    cudaFreeAsync(both, st);
     CERTEX_CUDA(e);
   }
+  d.segs  = both;
+  d.begin = reinterpret_cast<int*>(both + seg_bytes);
   plans_[key] = d;
   return d;
 }
@@ -424,23 +508,23 @@ void Index::reserve(const Resources& res, int64_t n)
   int32_t *pe = nullptr, *iv = nullptr, *in = nullptr, *cm = nullptr;
   double* sq  = nullptr;
   const int64_t pad_old = round_up(size_, kTile), pad_new = round_up(cap, kTile);
-  v = alloc_vectors(static_cast<size_t>(cap) * pitch_, host_vectors_);
-  CERTEX_CUDA(cudaMalloc(&r, static_cast<size_t>(round_up(cap, 4))));
+  v = alloc_vectors(static_cast<size_t>(cap) * pitch_, host_vectors_, device_, res.stream);
+  index_alloc(&r, static_cast<size_t>(round_up(cap, 4)), device_, res.stream);
   CERTEX_CUDA(cudaMemsetAsync(r, 0, static_cast<size_t>(round_up(cap, 4)), res.stream));
   if (labels_) {
-    CERTEX_CUDA(cudaMalloc(&l, static_cast<size_t>(cap) * 4));
+    index_alloc(&l, static_cast<size_t>(cap) * 4, device_, res.stream);
     CERTEX_CUDA(cudaMemsetAsync(l, 0xff, static_cast<size_t>(cap) * 4, res.stream));
   }
   // the squared norms the cosine verification would otherwise sum again for every candidate
   const bool keep_sqnorm = params_.metric == kCos && !host_vectors_ && (dtype_ == kF32 || dtype_ == kF16);
-  if (keep_sqnorm) { CERTEX_CUDA(cudaMalloc(&sq, static_cast<size_t>(cap) * 8)); }
+  if (keep_sqnorm) { index_alloc(&sq, static_cast<size_t>(cap) * 8, device_, res.stream); }
   if (screen_kind_) {
     const int32_t never = screen_kind_ == 2 ? static_cast<int32_t>(0xff800000u) : kNeverInit;  // -inf or -2^30
-    CERTEX_CUDA(cudaMalloc(&co, static_cast<size_t>(cap) * code_pitch_));
-    CERTEX_CUDA(cudaMalloc(&pe, static_cast<size_t>(cap) * 4));
-    CERTEX_CUDA(cudaMalloc(&iv, static_cast<size_t>(cap) * 4));
-    CERTEX_CUDA(cudaMalloc(&in, static_cast<size_t>(pad_new) * 4));
-    CERTEX_CUDA(cudaMalloc(&cm, static_cast<size_t>(pad_new / kChainRows) * 4));
+    index_alloc(&co, static_cast<size_t>(cap) * code_pitch_, device_, res.stream);
+    index_alloc(&pe, static_cast<size_t>(cap) * 4, device_, res.stream);
+    index_alloc(&iv, static_cast<size_t>(cap) * 4, device_, res.stream);
+    index_alloc(&in, static_cast<size_t>(pad_new) * 4, device_, res.stream);
+    index_alloc(&cm, static_cast<size_t>(pad_new / kChainRows) * 4, device_, res.stream);
     launch_fill_i32(in, pad_new, never, res.stream);
     launch_fill_i32(cm, pad_new / kChainRows, never, res.stream);
     CERTEX_CUDA(cudaGetLastError());
@@ -471,10 +555,11 @@ void Index::reserve(const Resources& res, int64_t n)
     if (sq) { sqnorm_ = sq; }
     capacity_ = cap;
   }
-  if (sq) { cudaFree(old_sq); }
-  free_vectors(old[0], host_vectors_);
-  for (int i = 1; i < 8; ++i) {
-    if (i != 2 || l) { cudaFree(old[i]); }
+  index_free(device_, {host_vectors_ ? nullptr : old[0], old[1], l ? old[2] : nullptr, old[3], old[4], old[5], old[6], old[7],
+                       sq ? old_sq : nullptr});
+  if (host_vectors_) {
+    cudaDeviceSynchronize();
+    cudaFreeHost(old[0]);
   }
 }
 
@@ -585,7 +670,7 @@ void Index::set_labels(const Resources& res, const int32_t* labels_device, int64
   CERTEX_EXPECTS(first >= 0 && n >= 0 && first + n <= size_, "certex: labels beyond the vectors of the index");
   if (!labels_) {
     int32_t* l = nullptr;
-    CERTEX_CUDA(cudaMalloc(&l, static_cast<size_t>(std::max<int64_t>(capacity_, 1)) * 4));
+    index_alloc(&l, static_cast<size_t>(std::max<int64_t>(capacity_, 1)) * 4, device_, res.stream);
     CERTEX_CUDA(cudaMemsetAsync(l, 0xff, static_cast<size_t>(std::max<int64_t>(capacity_, 1)) * 4, res.stream));
     res.sync();
     std::unique_lock<ReaderGate> lock(rw_);
@@ -607,7 +692,7 @@ void Index::partition_by_labels(const Resources& res)
   const int64_t n = size_;
   if (n == 0) { return; }
   int32_t* ids = nullptr;
-  CERTEX_CUDA(cudaMalloc(&ids, static_cast<size_t>(n) * 4));
+  index_alloc(&ids, static_cast<size_t>(n) * 4, device_, res.stream);
   std::vector<int32_t> distinct, counts;
   try {
     Scratch scratch(res.stream);
@@ -629,7 +714,7 @@ void Index::partition_by_labels(const Resources& res)
     CERTEX_CUDA(cudaMemcpyAsync(counts.data(), d_counts, counts.size() * 4, cudaMemcpyDeviceToHost, res.stream));
     res.sync();
   } catch (...) {
-    cudaFree(ids);
+    index_free(device_, {ids});
     throw;
   }
   std::vector<int64_t> offsets(distinct.size() + 1, 0);
@@ -652,11 +737,11 @@ void Index::partition_by_labels(const Resources& res)
     try {
       const bool f16      = screen_kind_ == 2;
       const int32_t never = f16 ? static_cast<int32_t>(0xff800000u) : kNeverInit;
-      CERTEX_CUDA(cudaMalloc(&lcodes, static_cast<size_t>(n_lrows) * code_pitch_));
-      CERTEX_CUDA(cudaMalloc(&linit, static_cast<size_t>(n_lrows) * 4));
-      CERTEX_CUDA(cudaMalloc(&lcmax, static_cast<size_t>(n_lrows / kChainRows) * 4));
-      CERTEX_CUDA(cudaMalloc(&lperm, static_cast<size_t>(n_lrows) * 4));
-      CERTEX_CUDA(cudaMalloc(&linv, static_cast<size_t>(n) * 4));
+      index_alloc(&lcodes, static_cast<size_t>(n_lrows) * code_pitch_, device_, res.stream);
+      index_alloc(&linit, static_cast<size_t>(n_lrows) * 4, device_, res.stream);
+      index_alloc(&lcmax, static_cast<size_t>(n_lrows / kChainRows) * 4, device_, res.stream);
+      index_alloc(&lperm, static_cast<size_t>(n_lrows) * 4, device_, res.stream);
+      index_alloc(&linv, static_cast<size_t>(n) * 4, device_, res.stream);
       Scratch scratch(res.stream);
       int32_t* lsrc   = scratch.get<int32_t>(static_cast<size_t>(n_lrows));
       int64_t* d_off  = scratch.get<int64_t>(offsets.size());
@@ -681,7 +766,7 @@ void Index::partition_by_labels(const Resources& res)
       CERTEX_CUDA(cudaGetLastError());
       res.sync();
     } catch (...) {
-      cudaFree(ids), cudaFree(lcodes), cudaFree(linit), cudaFree(lcmax), cudaFree(lperm), cudaFree(linv);
+      index_free(device_, {ids, lcodes, linit, lcmax, lperm, linv});
       throw;
     }
   }
@@ -697,7 +782,7 @@ void Index::partition_by_labels(const Resources& res)
     lcodes_ = lcodes, linit_ = linit, lcmax_ = lcmax, lperm_ = lperm, linv_ = linv;
     n_lrows_ = n_lrows;
   }
-  for (void* p : old) { cudaFree(p); }
+  index_free(device_, {old[0], old[1], old[2], old[3], old[4], old[5]});
 }
 
 // -------------------------------------------------------------------------------------------- search
@@ -742,7 +827,7 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   const int ld_cand    = next_pow2(cap);
   Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(nq) * ld_cand);
   int32_t* kept        = scratch.get<int32_t>(static_cast<size_t>(nq));
-  const DevicePlan plan = device_plan(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
+  const DevicePlan plan = device_plan(res, nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
   auto* d_segs          = static_cast<ScreenSeg*>(plan.segs);
   int* d_seg_begin      = plan.begin;
   if (!d_segs) { upload_plan(scratch, plan_chunked(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_)), d_segs, d_seg_begin); }
@@ -818,7 +903,7 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
   int32_t* gmax        = scratch.get<int32_t>(static_cast<size_t>(nq) * ld_g);
   int32_t* thr         = scratch.get<int32_t>(static_cast<size_t>(nq));
   // an anchor tile is 256 rows spread over the whole set: chunks by bytes of anchor rows, as for the screen
-  const DevicePlan plan_a = device_plan(nqt, nt_anchor, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
+  const DevicePlan plan_a = device_plan(res, nqt, nt_anchor, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
   auto* d_segs            = static_cast<ScreenSeg*>(plan_a.segs);
   int* d_seg_begin        = plan_a.begin;
   if (!d_segs) { upload_plan(scratch, plan_chunked(nqt, nt_anchor, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_)), d_segs, d_seg_begin); }

@@ -65,6 +65,8 @@ struct Resources {
   /// searches in flight are copied to; made on first use.
   static constexpr int kPinnedSlots = 4;
   void* pinned_block(int slot) const;
+  /// A stream of its own for what must be on the device before anything is enqueued behind it (work splits); made on first use.
+  cudaStream_t side_stream() const;
   /// Sends small host arrays to the device in one copy: `pieces` (pointer, bytes) are packed, 256-byte aligned, into
   /// page-locked memory and copied to `device` (at least upload_bytes(pieces) bytes) on the stream; offsets[i] is where
   /// piece i starts. A copy from pageable memory would make the host wait for the stream once per array.
@@ -76,6 +78,7 @@ struct Resources {
   mutable void* staging_        = nullptr;  // page-locked, grows; reused once the copy out of it has finished
   mutable size_t staging_bytes_ = 0;
   mutable cudaEvent_t staging_done_ = nullptr;
+  mutable cudaStream_t side_       = nullptr;
   friend class Index;
   mutable int searches_in_flight_ = 0;
   mutable unsigned next_slot_     = 0;
@@ -345,7 +348,7 @@ class Index {
     void* segs = nullptr;  // ScreenSeg[]
     int* begin = nullptr;  // [grid + 1]
   };
-  DevicePlan device_plan(int nqt, int nt, int panel_tiles, int grid, int chunk_tiles) const;  // empty: not kept, upload it
+  DevicePlan device_plan(const Resources& res, int nqt, int nt, int panel_tiles, int grid, int chunk_tiles) const;  // empty: not kept, upload it
   mutable std::mutex plans_mutex_;
   mutable std::map<std::array<int, 5>, DevicePlan> plans_;
   static constexpr size_t kMaxPlans = 64;
