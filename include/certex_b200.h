@@ -312,6 +312,11 @@ CERTEX_B200_EXPORT cuvsError_t certexB200ScreenTrace(void* trace, int32_t units)
 CERTEX_B200_EXPORT cuvsError_t certexB200PlanSegments(int32_t n_query_tiles, int32_t n_base_tiles, int32_t panel_tiles,
                                                       int32_t grid, int32_t* out);
 
+/** dst [n] = src [n] rounded to float16 (kind 0: src is float32, 1: float16, 2: bfloat16; device memory, dst may be null: only
+ *  the check); *finite = 1 when every value is finite in float16. Waits for the resources' stream. */
+CERTEX_B200_EXPORT cuvsError_t certexB200ToHalf(cuvsResources_t res, const void* src, int32_t kind, int64_t n, void* dst,
+                                                int32_t* finite);
+
 /** Filter words of a mask of n bytes in device memory (non-zero: keep): bit j of words[i] = entry 32 i + j, (n + 31) / 32
  *  words, bits beyond n are 0. Enqueued on the resources' stream. */
 CERTEX_B200_EXPORT cuvsError_t certexB200PackMask(cuvsResources_t res, const uint8_t* mask, int64_t n, uint32_t* words);

@@ -116,7 +116,7 @@ SYMBOLS = [
     "certexB200CommGetUniqueId", "certexB200CommInitRank", "certexB200CommAdopt", "certexB200CommDestroy",
     "certexB200DistributedSearch", "certexB200ScreenTrace", "certexB200PlanChunked",
     "certexB200DistributedSearchBegin", "certexB200DistributedSearchEnd", "certexB200OrderByLabel",
-    "certexB200PackMask",
+    "certexB200PackMask", "certexB200ToHalf",
 ]
 
 # void hook(void* ctx, int32_t* keys, int64_t n, cudaStream_t stream)
@@ -198,6 +198,7 @@ def lib():
                 L.certexB200DistributedSearchBegin.argtypes = [vp, vp, P(SearchParams), P(IndexHandle), mt, mt, mt, mt, i64,
                                                                ctypes.c_int32, P(vp)]
                 L.certexB200DistributedSearchEnd.argtypes = [vp]
+                L.certexB200ToHalf.argtypes = [vp, vp, ctypes.c_int32, i64, vp, P(ctypes.c_int32)]
                 L.certexB200PackMask.argtypes = [vp, vp, i64, vp]
                 L.certexB200ScreenTrace.argtypes = [vp, ctypes.c_int32]
                 L.certexB200OrderByLabel.argtypes = [P(ctypes.c_int32), i64, P(ctypes.c_int32)]

@@ -4,16 +4,29 @@ attention maps query head h to KV head h // (n_heads / n_kv_heads). Returns what
 but the k keys of every query are the exact top k by fp64 inner product, ties to the smaller key position.
 """
 
+import ctypes
+
 import torch
 
+from . import _lib as L
 from .index import Index, _need
+
+
+_HALF_KIND = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 
 def _as_half_or_float(x):
     """float16 on the GPU, or float32 where float16 would overflow (bf16 inputs can)."""
     x = torch.as_tensor(x, device="cuda")
-    h = x.to(torch.float16)
-    return h if bool(torch.isfinite(h).all()) else x.to(torch.float32)
+    if x.dtype not in _HALF_KIND or not x.is_contiguous() or (x.requires_grad and torch.is_grad_enabled()):
+        h = x.to(torch.float16)
+        return h if bool(torch.isfinite(h).all()) else x.to(torch.float32)
+    # rounding and check in one pass
+    h = x if x.dtype == torch.float16 else torch.empty_like(x, dtype=torch.float16)
+    finite = ctypes.c_int32()
+    L.check(L.lib().certexB200ToHalf(L.resources(), x.data_ptr(), _HALF_KIND[x.dtype], x.numel(),
+                                     None if h is x else h.data_ptr(), ctypes.byref(finite)))
+    return h if finite.value else x.to(torch.float32)
 
 
 class GrowingMap:

@@ -569,6 +569,21 @@ cuvsError_t certexB200ScreenRaw(cuvsResources_t res, const void* q_codes, int64_
   });
 }
 
+cuvsError_t certexB200ToHalf(cuvsResources_t res, const void* src, int32_t kind, int64_t n, void* dst, int32_t* finite)
+{
+  return translate([=] {
+    CERTEX_EXPECTS(n >= 0 && finite != nullptr && (n == 0 || src != nullptr), "certex: null argument");
+    CERTEX_EXPECTS(kind >= 0 && kind <= 2, "certex: the kind is 0 (float32), 1 (float16) or 2 (bfloat16)");
+    Resources& r = as_res(res);
+    auto* bad    = static_cast<int*>(r.pinned_block(Resources::kFlagBlock));
+    *bad         = 0;
+    launch_to_half(src, kind, n, dst, bad, r.stream);
+    CERTEX_CUDA(cudaGetLastError());
+    r.sync();
+    *finite = *static_cast<volatile int*>(bad) == 0 ? 1 : 0;
+  });
+}
+
 cuvsError_t certexB200PackMask(cuvsResources_t res, const uint8_t* mask, int64_t n, uint32_t* words)
 {
   return translate([=] {

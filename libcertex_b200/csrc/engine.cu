@@ -405,8 +405,8 @@ cudaStream_t Resources::side_stream() const
 
 void* Resources::pinned_block(int slot) const
 {
-  if (!pinned_) { CERTEX_CUDA(cudaHostAlloc(&pinned_, 256 * kPinnedSlots, cudaHostAllocDefault)); }
-  return static_cast<unsigned char*>(pinned_) + 256 * (slot % kPinnedSlots);
+  if (!pinned_) { CERTEX_CUDA(cudaHostAlloc(&pinned_, 256 * (kPinnedSlots + 1), cudaHostAllocDefault)); }
+  return static_cast<unsigned char*>(pinned_) + 256 * (slot == kFlagBlock ? kFlagBlock : slot % kPinnedSlots);
 }
 
 // ============================================================================================ Index

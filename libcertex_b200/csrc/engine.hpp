@@ -65,6 +65,7 @@ struct Resources {
   /// searches in flight are copied to; made on first use.
   static constexpr int kPinnedSlots = 4;
   void* pinned_block(int slot) const;
+  static constexpr int kFlagBlock = kPinnedSlots;  // one more block, for a flag that a kernel raises
   /// A stream of its own for what must be on the device before anything is enqueued behind it (work splits); made on first use.
   cudaStream_t side_stream() const;
   /// Sends small host arrays to the device in one copy: `pieces` (pointer, bytes) are packed, 256-byte aligned, into

@@ -158,6 +158,9 @@ struct Refine {
 /// entry: a zero row); rows n .. n_pad - 1 are zeros.
 void launch_gather_rows(const void* in, size_t in_pitch, const int32_t* sel, int64_t n, int64_t n_pad, void* out,
                         size_t out_pitch, size_t row_bytes, cudaStream_t s);
+/// dst [n] = src [n] (kind 0 float32, 1 float16, 2 bfloat16) rounded to fp16; *bad, page-locked host memory, becomes 1 when a
+/// value is not finite in fp16. dst null: only the check.
+void launch_to_half(const void* src, int kind, int64_t n, void* dst, int* bad, cudaStream_t s);
 /// words [(n + 31) / 32]: bit j of word i = entry 32 i + j of the byte mask (non-zero: set); bits beyond n are 0.
 void launch_pack_mask(const uint8_t* mask, int64_t n, uint32_t* words, cudaStream_t s);
 /// best_s / best_row rows sel[i] = rows i of s2 / row2, i < n (negative sel[i]: skipped).
