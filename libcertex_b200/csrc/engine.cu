@@ -815,7 +815,8 @@ void Index::search_dense(const Resources& res, const void* q, size_t qpitch, con
 void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32_t* thr, const void* queries,
                         size_t row_bytes, int q0, int nq, int k, double* best_s, int32_t* best_row, int32_t* ovf_list,
                         unsigned int* ovf_count, unsigned long long* stats, int* err, int64_t n, int32_t* thr2,
-                        const float* shift, const double* qq, const Admit& adm, std::vector<cudaEvent_t>* events) const
+                        const float* shift, const double* qq, const Admit& adm, std::vector<cudaEvent_t>* events,
+                        uint32_t* cnt) const
 {
   Scratch scratch(res.stream);
   const int grid          = res.sm_count;
@@ -823,7 +824,8 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   const ScreenShape shape = shape_for(kb_, nqt);
   const int nt_all        = static_cast<int>((n + kTile - 1) / kTile);
   const uint32_t cap      = test_mode_ == 2 ? static_cast<uint32_t>(test_cap_) : static_cast<uint32_t>(std::max(2048, 2 * k));
-  uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(nq));
+  const bool fresh     = cnt == nullptr;  // else [nq] zeros
+  if (fresh) { cnt = scratch.get<uint32_t>(static_cast<size_t>(nq)); }
   const int ld_cand    = next_pow2(cap);
   Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(nq) * ld_cand);
   int32_t* kept        = scratch.get<int32_t>(static_cast<size_t>(nq));
@@ -831,7 +833,7 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   auto* d_segs          = static_cast<ScreenSeg*>(plan.segs);
   int* d_seg_begin      = plan.begin;
   if (!d_segs) { upload_plan(scratch, plan_chunked(nqt, nt_all, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_)), d_segs, d_seg_begin); }
-  CERTEX_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * nq, res.stream));
+  if (fresh) { CERTEX_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * nq, res.stream)); }
   const size_t cp        = code_pitch_;
   const CUtensorMap tm_q = make_code_map(qcodes, cp, static_cast<uint64_t>(round_up(nq, kQTile)), cp, kQueryTile);
   const CUtensorMap tm_x = make_code_map(codes_, cp, static_cast<uint64_t>(n), cp, kBaseTile);
@@ -902,6 +904,7 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
                                                       : static_cast<size_t>(nt_anchor) * kTile);
   int32_t* gmax        = scratch.get<int32_t>(static_cast<size_t>(nq) * ld_g);
   int32_t* thr         = scratch.get<int32_t>(static_cast<size_t>(nq));
+  uint32_t* cnt        = scratch.get<uint32_t>(static_cast<size_t>(nq));  // the screen's counters of kept chains
   // an anchor tile is 256 rows spread over the whole set: chunks by bytes of anchor rows, as for the screen
   const DevicePlan plan_a = device_plan(res, nqt, nt_anchor, shape.panel_tiles, grid, chunk_tiles_for(code_pitch_));
   auto* d_segs            = static_cast<ScreenSeg*>(plan_a.segs);
@@ -957,23 +960,26 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
   // (with an exchange between row shards also the k largest group values of every query, in the same launch)
   const bool wide_exchange = topk_hook != nullptr && k <= kTopkExchangeMaxK;
   int32_t* topk            = wide_exchange ? scratch.get<int32_t>(static_cast<size_t>(nq) * k) : nullptr;
-  launch_kth_largest(gmax, ld_g, n_groups, k, nq, thr, res.stream, nullptr, 0x7fffffff, topk);
-  if (screen_kind_ == 2) {
+  // thr then holds, per query, (a key of) a score k rows of this index certainly reach, which other shards may tighten; on its
+  // own the index makes the screen's threshold in the same launch
+  const bool exchange = wide_exchange || threshold_hook != nullptr;
+  launch_kth_largest(gmax, ld_g, n_groups, k, nq, thr, res.stream, nullptr, 0x7fffffff, topk,
+                     screen_kind_ == 2 && !exchange ? shift + q0 : nullptr, cnt);
+  if (screen_kind_ == 2 && exchange) {
     launch_finish_thr_f16(thr, shift + q0, nq, 0, res.stream);
     if (wide_exchange) { launch_finish_thr_f16(topk, shift + q0, nq * k, 0, res.stream, k); }
   }
   CERTEX_CUDA(cudaGetLastError());
-  // thr now holds, per query, (a key of) a score k rows of this index certainly reach: other shards may tighten it
   if (wide_exchange) {
     topk_hook(threshold_hook_ctx, topk, thr, nq, k, res.stream);
   } else if (threshold_hook) {
     threshold_hook(threshold_hook_ctx, thr, nq, res.stream);
   }
-  if (screen_kind_ == 2) { launch_finish_thr_f16(thr, shift + q0, nq, 1, res.stream); }
+  if (screen_kind_ == 2 && exchange) { launch_finish_thr_f16(thr, shift + q0, nq, 1, res.stream); }
   CERTEX_CUDA(cudaGetLastError());
   // 3 screen over all rows, 4 exact scores of the candidates and the k best
   screen_pass(res, qb, thr, queries, row_bytes, q0, nq, k, best_s, best_row, ovf_list, ovf_count, stats, err, n, thr2, shift, qq,
-              adm, events);
+              adm, events, cnt);
 }
 
 namespace {
@@ -1204,14 +1210,13 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     int32_t* ovf_list    = scratch.get<int32_t>(static_cast<size_t>(ns));
     unsigned int* d_flag = scratch.get<unsigned int>(4);  // [0] overflowed slots, [1] error code, [2] fp16 overflow
     auto* d_stats        = scratch.get<unsigned long long>(2);
-    CERTEX_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * ns, res.stream));
     CERTEX_CUDA(cudaMemsetAsync(d_flag, 0, 4 * sizeof(unsigned int), res.stream));
     CERTEX_CUDA(cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned long long), res.stream));
     // queries in slot order (8-bit vectors: zero padded to code rows, which the verification reads as well)
     const size_t q_rows_pitch = f16 ? qpitch : cp;
     launch_gather_rows(q, qpitch, d_slot_q, ns, ns, q_rows, q_rows_pitch, qpitch, res.stream);
     if (f16) {
-      launch_encode_f16_queries(q_rows, qpitch, dtype_, static_cast<int>(dim_), ns, q_codes, cp, n1max_, n2max_, emax_, shift,
+      launch_encode_f16_queries(q_rows, qpitch, dtype_, static_cast<int>(dim_), ns, ns, q_codes, cp, n1max_, n2max_, emax_, shift,
                                 d_flag + 2, res.stream);
       if (qq) { launch_query_sqnorms(q_rows, qpitch, dtype_, static_cast<int>(dim_), ns, qq, res.stream); }
     }
@@ -1252,11 +1257,7 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
     mark();
     launch_kth_largest(gmax, ld_g, n_groups, k, ns, thr, res.stream, d_slot_ng,
-                       f16 ? static_cast<int32_t>(0x7f800000) : static_cast<int32_t>(0x7fffffff));
-    if (f16) {
-      launch_finish_thr_f16(thr, shift, ns, 0, res.stream);
-      launch_finish_thr_f16(thr, shift, ns, 1, res.stream);
-    }
+                       f16 ? static_cast<int32_t>(0x7f800000) : static_cast<int32_t>(0x7fffffff), nullptr, shift, cnt);
     CERTEX_CUDA(cudaGetLastError());
     // 3 screen over all tiles of every label, 4 exact scores of the candidates
     a.mode      = kModeScreen;
@@ -1288,7 +1289,7 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
                          ovf_list, d_flag, d_stats, Refine{}, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
     launch_scatter_best(slot_s, slot_row, d_slot_q, ns, k, best_s, best_row, res.stream);
     CERTEX_CUDA(cudaGetLastError());
-    st->launches += f16 ? (qq ? 10 : 9) : 7;
+    st->launches += f16 ? (qq ? 8 : 7) : 7;
     unsigned int h_flag[4]        = {0, 0, 0, 0};
     unsigned long long h_stats[2] = {0, 0};
     std::vector<int32_t> h_ovf;
@@ -1598,15 +1599,12 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
     if (screen_kind_ == 2) {
       shift = scratch.get<float>(static_cast<size_t>(nq));
       P.qq  = params_.metric != kL2 ? scratch.get<double>(static_cast<size_t>(nq)) : nullptr;
-      CERTEX_CUDA(cudaMemsetAsync(qbuf + static_cast<size_t>(nq) * code_pitch_, 0, static_cast<size_t>(nq_pad - nq) * code_pitch_, res.stream));
-      launch_encode_f16_queries(queries, row_bytes, dtype_, d, nq, qbuf, code_pitch_, n1max_, n2max_, emax_, shift, q_ovf, res.stream);
+      launch_encode_f16_queries(queries, row_bytes, dtype_, d, nq, nq_pad, qbuf, code_pitch_, n1max_, n2max_, emax_, shift, q_ovf, res.stream);
       if (P.qq) { launch_query_sqnorms(queries, row_bytes, dtype_, d, nq, P.qq, res.stream); }
       CERTEX_CUDA(cudaGetLastError());
     } else {
-      if (row_bytes != code_pitch_ || nq_pad != nq) {
-        CERTEX_CUDA(cudaMemsetAsync(qbuf, 0, static_cast<size_t>(nq_pad) * code_pitch_, res.stream));
-      }
-      CERTEX_CUDA(cudaMemcpy2DAsync(qbuf, code_pitch_, queries, row_bytes, row_bytes, static_cast<size_t>(nq), cudaMemcpyDeviceToDevice, res.stream));
+      launch_gather_rows(queries, row_bytes, nullptr, nq, nq_pad, qbuf, code_pitch_, row_bytes, res.stream);
+      CERTEX_CUDA(cudaGetLastError());
     }
     int32_t* ovf_list      = scratch.get<int32_t>(static_cast<size_t>(nq));
     int32_t* thr2          = scratch.get<int32_t>(static_cast<size_t>(nq));  // tighter thresholds of the queries in ovf_list
@@ -1617,7 +1615,7 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
       const int nb = static_cast<int>(std::min<int64_t>(batch, nq - q0));
       search_screened(res, qbuf, shift, P.qq, queries, row_bytes, static_cast<int>(q0), nb, k, best_s, best_row, ovf_list, d_count,
                       d_stats, reinterpret_cast<int*>(d_count + 1), stride, n, thr2, adm, stats_sink ? &P.events : nullptr);
-      local.launches += screen_kind_ == 2 ? 6 : 5;  // gather_init, GROUPMAX, kth_largest (+ thresholds), SCREEN, verify
+      local.launches += 5;  // gather_init, GROUPMAX, kth_largest, SCREEN, verify
     }
     // The outputs are written now, as if no list had overflowed; the counters follow them to the host and search_end
     // looks at them once the caller has enqueued what it wanted behind the search.
@@ -1716,7 +1714,7 @@ bool Index::search_end(Pending* raw, bool refinish) const
         const int nb = std::min<int>(static_cast<int>(P.batch), n_ovf - b0);
         screen_pass(res, qcodes2 + static_cast<size_t>(b0) * code_pitch_, P.thr2 + b0, queries2, P.row_bytes, b0, nb, k, best2_s,
                     best2_row, ovf2, P.d_count + 2, P.d_stats, reinterpret_cast<int*>(P.d_count + 1), n, nullptr,
-                    P.shift ? shift2 : nullptr, P.qq ? qq2 : nullptr, P.adm, stats_sink ? &P.events : nullptr);
+                    P.shift ? shift2 : nullptr, P.qq ? qq2 : nullptr, P.adm, stats_sink ? &P.events : nullptr, nullptr);
         local.launches += 2;
       }
       launch_scatter_best(best2_s, best2_row, P.ovf_list, n_ovf, k, P.best_s, P.best_row, res.stream);

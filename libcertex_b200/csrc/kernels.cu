@@ -552,16 +552,20 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_f16_rows_kernel(const u
 // The anchors give a value every one of k rows certainly reaches (their group maximum minus E + slack); a row is
 // kept unless its value certainly lies below that (its maximum plus E + slack): hence twice.
 template <typename T>
-__global__ void encode_f16_queries_kernel(const uint8_t* queries, size_t qpitch, int d, int64_t nq, uint8_t* codes,
+__global__ void encode_f16_queries_kernel(const uint8_t* queries, size_t qpitch, int d, int64_t nq, int64_t nq_pad, uint8_t* codes,
                                           size_t code_pitch, float n1max, float n2max, float emax, float* shift,
                                           unsigned int* overflow)
 {
   const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane    = threadIdx.x & 31;
-  if (row >= nq) { return; }
+  if (row >= nq_pad) { return; }
   const uint8_t* src = queries + static_cast<size_t>(row) * qpitch;
   __half* dst        = reinterpret_cast<__half*>(codes + static_cast<size_t>(row) * code_pitch);
   const int d_pad    = static_cast<int>(code_pitch / 2);
+  if (row >= nq) {  // rows that fill the last query tile
+    for (int t = lane; t < d_pad; t += 32) { dst[t] = __float2half_rn(0.f); }
+    return;
+  }
   double qq = 0, hh = 0, rr = 0;
   bool bad = false;
   for (int t = lane; t < d_pad; t += 32) {
@@ -629,19 +633,21 @@ __global__ void __launch_bounds__(32) query_sqnorm_kernel(const uint8_t* queries
   if (lane < n) { qq[q0 + lane] = a; }
 }
 
+/// The float of a key of the screen kernel's float_key, and a value less half a query's allowance, rounded down.
+__device__ __forceinline__ float float_of_key(int32_t key) { return __int_as_float(key ^ ((key >> 31) & 0x7fffffff)); }
+__device__ __forceinline__ float lowered(float v, float shift) { return __fadd_rd(v, -__fmul_ru(0.5f, shift)); }
+__device__ __forceinline__ int32_t lowered_bits(float v, float shift) { return __float_as_int(lowered(v, shift)); }
+
 // fp16 codes, in two steps around the optional exchange of thresholds between shards. Step 0: thr[q] = the key of the
 // k-th largest group maximum (see float_key in the screen kernel) -> the key of value - shift[q] / 2, a score that k
 // rows of this index certainly reach in exact arithmetic. Step 1: such a key -> float bits of the screen's
-// threshold, bound - shift[q] / 2. Both subtractions round down.
+// threshold, bound - shift[q] / 2. Both subtractions round down. (Without an exchange kth_largest_kernel makes both.)
 __global__ void finish_thr_f16_kernel(int32_t* thr, const float* shift, int nq, int step, int per)
 {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) { return; }
-  const int32_t key = thr[q];
-  const float v     = __int_as_float(key ^ ((key >> 31) & 0x7fffffff));
-  const float r     = __fadd_rd(v, -__fmul_ru(0.5f, shift[q / per]));
-  const int32_t b   = __float_as_int(r);
-  thr[q]            = step == 0 ? (b ^ ((b >> 31) & 0x7fffffff)) : b;
+  const int32_t b = lowered_bits(float_of_key(thr[q]), shift[q / per]);
+  thr[q]          = step == 0 ? (b ^ ((b >> 31) & 0x7fffffff)) : b;
 }
 
 __global__ void chain_max_f32_kernel(const float* init, int64_t c0, int64_t n, float* cmax)
@@ -778,19 +784,29 @@ __device__ void emit_topk(const int32_t* row, int ng, int32_t t, int k, int32_t*
   for (int i = static_cast<int>(min(*counter, static_cast<uint32_t>(k))) + threadIdx.x; i < k; i += blockDim.x) { out[i] = t; }
 }
 
-// With topk [nq, k] the k largest values of every row are written there as well (emit_topk).
+// With topk [nq, k] the k largest values of every row are written there as well (emit_topk). With shift [nq] (fp16 codes) the
+// threshold is lowered by it and leaves as float bits (both steps of finish_thr_f16_kernel); zero [nq] is set to 0: what follows
+// counts in it.
 __global__ void __launch_bounds__(512, 4) kth_largest_kernel(const int32_t* gmax, int64_t ld, int ng, int k, int32_t* thr,
-                                                              int in_smem, const int32_t* ng_rows, int32_t never, int32_t* topk)
+                                                              int in_smem, const int32_t* ng_rows, int32_t never, int32_t* topk,
+                                                              const float* shift, uint32_t* zero)
 {
   extern __shared__ int32_t row_smem[];
   __shared__ uint32_t hist[256];
   __shared__ uint32_t s_prefix, s_remaining;
+  // the k-th largest value of the row -> its threshold
+  auto answer = [&](int32_t t) {
+    if (threadIdx.x != 0) { return; }
+    if (shift) { t = lowered_bits(lowered(float_of_key(t), shift[blockIdx.x]), shift[blockIdx.x]); }
+    thr[blockIdx.x] = t;
+    if (zero) { zero[blockIdx.x] = 0; }
+  };
   const int32_t* row = gmax + static_cast<int64_t>(blockIdx.x) * ld;
   int32_t* topk_row  = topk ? topk + static_cast<int64_t>(blockIdx.x) * k : nullptr;
   if (ng_rows) {
     ng = ng_rows[blockIdx.x];
     if (ng < 0) {
-      if (threadIdx.x == 0) { thr[blockIdx.x] = never; }
+      answer(never);
       if (topk_row) {
         for (int i = threadIdx.x; i < k; i += blockDim.x) { topk_row[i] = never; }
       }
@@ -798,7 +814,7 @@ __global__ void __launch_bounds__(512, 4) kth_largest_kernel(const int32_t* gmax
     }
   }
   if (ng < k) {
-    if (threadIdx.x == 0) { thr[blockIdx.x] = static_cast<int32_t>(0x80000000u); }
+    answer(static_cast<int32_t>(0x80000000u));
     if (topk_row) {
       for (int i = threadIdx.x; i < k; i += blockDim.x) { topk_row[i] = static_cast<int32_t>(0x80000000u); }
     }
@@ -886,7 +902,7 @@ __global__ void __launch_bounds__(512, 4) kth_largest_kernel(const int32_t* gmax
       }
       __syncthreads();
       const int32_t t = static_cast<int32_t>(s_answer ^ 0x80000000u);
-      if (threadIdx.x == 0) { thr[blockIdx.x] = t; }
+      answer(t);
       if (topk_row) { emit_topk(row, ng, t, k, topk_row, &s_count); }
       return;
     }
@@ -947,7 +963,7 @@ __global__ void __launch_bounds__(512, 4) kth_largest_kernel(const int32_t* gmax
     mask |= 0xffu << shift;
   }
   const int32_t t = static_cast<int32_t>((prefix + base) ^ 0x80000000u);
-  if (threadIdx.x == 0) { thr[blockIdx.x] = t; }
+  answer(t);
   if (topk_row) { emit_topk(row, ng, t, k, topk_row, &s_count); }
 }
 
@@ -2347,17 +2363,17 @@ void launch_encode_f16_rows(const void* vectors, size_t pitch, int dtype, int d,
   });
 }
 
-void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, void* codes,
+void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, int64_t nq_pad, void* codes,
                                size_t code_pitch, float n1max, float n2max, float emax, float* shift,
                                unsigned int* overflow, cudaStream_t s)
 {
   if (nq <= 0) { return; }
-  const auto grid = static_cast<unsigned>((nq * 32 + 255) / 256);
+  const auto grid = static_cast<unsigned>((nq_pad * 32 + 255) / 256);
   if (dtype == kF32) {
-    encode_f16_queries_kernel<float><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq,
+    encode_f16_queries_kernel<float><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq, nq_pad,
                                                           static_cast<uint8_t*>(codes), code_pitch, n1max, n2max, emax, shift, overflow);
   } else {
-    encode_f16_queries_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq,
+    encode_f16_queries_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(queries), qpitch, d, nq, nq_pad,
                                                            static_cast<uint8_t*>(codes), code_pitch, n1max, n2max, emax, shift, overflow);
   }
 }
@@ -2429,7 +2445,7 @@ void launch_sort_batch(const int32_t* e, int64_t n, int32_t id0, int64_t row0, c
 }
 
 void launch_kth_largest(const int32_t* gmax, int64_t ld, int ng, int k, int nq, int32_t* thr, cudaStream_t s,
-                        const int32_t* ng_rows, int32_t never, int32_t* topk)
+                        const int32_t* ng_rows, int32_t never, int32_t* topk, const float* shift, uint32_t* zero)
 {
   if (nq <= 0) { return; }
   const size_t bytes = static_cast<size_t>(ng) * 4;
@@ -2437,7 +2453,7 @@ void launch_kth_largest(const int32_t* gmax, int64_t ld, int ng, int k, int nq, 
   if (in_smem) { allow_smem(kth_largest_kernel, bytes); }
   // short rows: smaller blocks, more of them per SM (the kernel is a chain of block-wide barriers)
   const int threads = ng > 4096 ? 512 : 2 * k <= 128 ? 128 : 2 * k <= 256 ? 256 : 512;
-  kth_largest_kernel<<<nq, threads, in_smem ? bytes : 0, s>>>(gmax, ld, ng, k, thr, in_smem, ng_rows, never, topk);
+  kth_largest_kernel<<<nq, threads, in_smem ? bytes : 0, s>>>(gmax, ld, ng, k, thr, in_smem, ng_rows, never, topk, shift, zero);
 }
 
 void launch_remove(const int64_t* ids, int64_t n_ids, int64_t size, uint8_t* removed, int32_t* init, const int32_t* inv,

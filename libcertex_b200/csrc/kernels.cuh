@@ -48,8 +48,9 @@ void launch_encode_f16_rows(const void* vectors, size_t pitch, int dtype, int d,
                             size_t code_pitch, float* e, unsigned int* maxima, cudaStream_t s);
 
 /// fp16 codes of the queries and shift [nq], the per-query allowance for rounding that separates the anchors' k-th
-/// group maximum from the screen's threshold; *overflow is raised when a query coordinate does not fit fp16.
-void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, void* codes,
+/// group maximum from the screen's threshold; *overflow is raised when a query coordinate does not fit fp16. Code rows
+/// nq .. nq_pad - 1 are zeros.
+void launch_encode_f16_queries(const void* queries, size_t qpitch, int dtype, int d, int64_t nq, int64_t nq_pad, void* codes,
                                size_t code_pitch, float n1max, float n2max, float emax, float* shift,
                                unsigned int* overflow, cudaStream_t s);
 
@@ -117,9 +118,11 @@ void launch_candidate_rows(const Candidate* cand, const uint32_t* cnt, uint32_t 
 
 /// thr[q] = k-th largest of gmax[q, 0:ng]  (INT_MIN when ng < k). With ng_rows [nq] every row has its own length
 /// (at most ng); a negative length gives thr[q] = never. With topk [nq, k] the k largest values of every row are
-/// written there too (any order: the values above the k-th, then copies of it), in the same launch.
+/// written there too (any order: the values above the k-th, then copies of it), in the same launch. With shift [nq] (fp16 codes, no exchange of
+/// thresholds) thr[q] = the float bits of the value less shift[q]; zero [nq] is set to 0.
 void launch_kth_largest(const int32_t* gmax, int64_t ld, int ng, int k, int nq, int32_t* thr, cudaStream_t s,
-                        const int32_t* ng_rows = nullptr, int32_t never = 0x7fffffff, int32_t* topk = nullptr);
+                        const int32_t* ng_rows = nullptr, int32_t never = 0x7fffffff, int32_t* topk = nullptr,
+                        const float* shift = nullptr, uint32_t* zero = nullptr);
 
 /// thr[q] = the k-th largest of the union of parts[p, q, 0:k], p < n_parts (lists of the k largest keys of every row
 /// shard: every key is reached by a row of its own, so the k-th largest of all of them is reached by k rows of the
