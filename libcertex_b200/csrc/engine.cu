@@ -16,6 +16,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <istream>
@@ -1466,19 +1467,33 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   return pairs;
 }
 
-int Index::anchor_stride_for(int64_t n, int k) const
+int Index::anchor_stride_for(int64_t n, int k, int64_t nq) const
 {
   // anchors: every stride-th row in whole tiles of 256, and at least 2k groups of 64 anchors, or the threshold would be
   // useless. The k-th largest group maximum is roughly the (stride * k)-th best row: for larger k the anchors are taken
   // denser, so that the candidate lists stay a small multiple of k (the anchor pass costs 1 / stride of a screen pass).
-  const int64_t by_k = std::max<int64_t>(1, static_cast<int64_t>(params_.anchor_stride) * 32 / k);
+  int64_t by_k = std::max<int64_t>(1, static_cast<int64_t>(params_.anchor_stride) * 32 / k);
+  // Many queries on rows of at most two K blocks: a unit's MMAs are short, and what holds the screen up is the epilogue's path
+  // for the pairs it keeps, about 1.3 stride k / n of all. The anchor pass costs 1 / stride of a pass without it, so the best
+  // stride grows with the root of n / k. Measured, us a call at strides 16 / 8 / 6 / 4 / 3 / 2:
+  //   100 000 x 128 float, 1000 queries, k = 10        206 / 187 / 181 / 169 / 168 / 166
+  //   1 M x 128 uint8, 1000 queries, k = 10            289 / 277 / 268 / 278
+  //   1 M x 64 float, 2000 queries, k = 10             495 / 469 / 467 / 492
+  //   1.2 M x 100 int8, 777 queries, k = 33, masked    433 (15) / 398 / 402 / 405 / 410
+  //   300 000 x 128 half, 2000 queries, k = 100        445 (5) / 431 (3) / 437 / 487 (1)
+  //   10 M x 128 uint8, 10 000 queries, k = 10         10 183 / 10 961 (12)
+  // Few queries are bound by reading the rows (1 M x 128 uint8, one query: 149 / 153 / - / 154), longer rows have MMAs enough to
+  // hide that path (300 000 x 256 float: 441 / 438 / - / 453), and shards that share their thresholds keep few pairs each.
+  if (kb_ <= 2 && nq > 4 * kQTile && threshold_hook == nullptr && topk_hook == nullptr) {
+    by_k = std::min(by_k, std::max<int64_t>(3, static_cast<int64_t>(std::sqrt(static_cast<double>(n) / k) / 50.0)));
+  }
   return static_cast<int>(std::min<int64_t>({params_.anchor_stride, by_k, n / (kTile * ((2 * k + 3) / 4))}));
 }
 
 bool Index::will_screen(int k) const
 {
   std::shared_lock<ReaderGate> lock(rw_);
-  return screen_kind_ != 0 && !code_overflow_ && test_mode_ != 1 && k >= 1 && anchor_stride_for(size_, k) >= 1;
+  return screen_kind_ != 0 && !code_overflow_ && test_mode_ != 1 && k >= 1 && anchor_stride_for(size_, k, 1) >= 1;
 }
 
 /// Counters of a screened search as the device leaves them, copied to page-locked host memory behind the search.
@@ -1574,7 +1589,7 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
   // 39-62). A bitmap (a row of bits per query) and label searches without a partition score every vector.
   const bool filtered = (filter.words != nullptr && filter.bitmap_cols > 0) || filter.query_labels != nullptr;
 
-  const int stride    = anchor_stride_for(n, k);
+  const int stride    = anchor_stride_for(n, k, nq);
   const bool screened = screen_kind_ != 0 && !code_overflow_ && !filtered && stride >= 1 && test_mode_ != 1;
 
   SearchStats& local = P.local;
