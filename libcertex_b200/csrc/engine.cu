@@ -877,7 +877,7 @@ void Index::screen_pass(const Resources& res, const uint8_t* qcodes, const int32
   // 8-bit vectors kept in host memory: the exact stage reads the candidates' code rows, which are the vectors
   const bool from_codes = host_vectors_ && screen_kind_ == 1;
   launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, queries, row_bytes,
-                       nq, q0, Candidates{cand, cnt, cap, ld_cand, n, perm_, init_, shift, qq, 0, 0}, k, adm, best_s, best_row, ovf_list, ovf_count,
+                       nq, q0, Candidates{cand, cnt, cap, ld_cand, n, perm_, init_, shift, qq, 0, 0, nullptr}, k, adm, best_s, best_row, ovf_list, ovf_count,
                        stats, rf, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
   CERTEX_CUDA(cudaGetLastError());
 }
@@ -1206,8 +1206,6 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     const int ld_cand    = next_pow2(cap);
     Candidate* cand      = scratch.get<Candidate>(static_cast<size_t>(ns) * ld_cand);
     int32_t* kept        = scratch.get<int32_t>(static_cast<size_t>(ns));
-    double* slot_s       = scratch.get<double>(static_cast<size_t>(ns) * k);
-    int32_t* slot_row    = scratch.get<int32_t>(static_cast<size_t>(ns) * k);
     int32_t* ovf_list    = scratch.get<int32_t>(static_cast<size_t>(ns));
     unsigned int* d_flag = scratch.get<unsigned int>(4);  // [0] overflowed slots, [1] error code, [2] fp16 overflow
     auto* d_stats        = scratch.get<unsigned long long>(2);
@@ -1286,11 +1284,10 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     plain.removed = removed_;
     const bool from_codes = host_vectors_ && screen_kind_ == 1;
     launch_verify_select(from_codes ? codes_ : vectors_, pitch_, dtype_, static_cast<int>(dim_), params_.metric, q_rows,
-                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq, static_cast<int32_t>(n_part_), static_cast<int32_t>(n_tail)}, k, plain, slot_s, slot_row,
+                         q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq, static_cast<int32_t>(n_part_), static_cast<int32_t>(n_tail), d_slot_q}, k, plain, best_s, best_row,
                          ovf_list, d_flag, d_stats, Refine{}, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
-    launch_scatter_best(slot_s, slot_row, d_slot_q, ns, k, best_s, best_row, res.stream);
     CERTEX_CUDA(cudaGetLastError());
-    st->launches += f16 ? (qq ? 8 : 7) : 7;
+    st->launches += f16 ? (qq ? 7 : 6) : 5;
     unsigned int h_flag[4]        = {0, 0, 0, 0};
     unsigned long long h_stats[2] = {0, 0};
     std::vector<int32_t> h_ovf;

@@ -1341,7 +1341,7 @@ enum : int { kFused = 0, kRank = 1, kScore = 2 };
 constexpr int kSplitK    = 256;
 constexpr int kScoreRows = 128;  // rows a block of the scoring step takes
 template <typename T, int METRIC, bool STORED_XX, int PART>
-__global__ void __launch_bounds__(kByteRows<T> ? 1024 : 256, kByteRows<T> ? 1 : 3)
+__global__ void __launch_bounds__(PART == kRank || kByteRows<T> ? 1024 : 256, PART == kRank || kByteRows<T> ? 1 : 3)
 verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* queries, size_t qpitch, int q0, Candidates cd,
                      int n2max, int k, Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
                      unsigned long long* stats, Refine rf, const int32_t* where, const double* sqnorm, int32_t* kept)
@@ -1354,6 +1354,11 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
   constexpr bool kBytes = kByteRows<T>;
   const int qb          = PART == kScore ? blockIdx.y : blockIdx.x;  // the query's number in its batch
   const int q           = q0 + qb;                                   // and in the call
+  const int out         = cd.sel ? __ldg(cd.sel + q) : q;            // and its list of answers
+  if (out < 0) {
+    if (PART == kRank && threadIdx.x == 0) { kept[qb] = -1; }
+    return;
+  }
   const Candidate* mine = cd.cand + static_cast<size_t>(qb) * cd.ld;
   // split: the query's list and scores in the memory of its candidates (ld = n2max entries of 16 bytes)
   double* far_s    = reinterpret_cast<double*>(const_cast<Candidate*>(mine));
@@ -1365,8 +1370,8 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
   int m        = 0;
   auto nothing = [&] {  // no candidate (a slot without a query, or nothing that the query may return)
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
-      best_s[static_cast<size_t>(q) * k + t]   = CUDART_INF;
-      best_row[static_cast<size_t>(q) * k + t] = -1;
+      best_s[static_cast<size_t>(out) * k + t]   = CUDART_INF;
+      best_row[static_cast<size_t>(out) * k + t] = -1;
     }
   };
   auto give_up = [&] {
@@ -1561,8 +1566,8 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
       const bool have                          = t < m;
       const unsigned long long key             = have ? keys[t] : 0ull;
-      best_s[static_cast<size_t>(q) * k + t]   = have ? __ll2double_rn(static_cast<long long>(key >> 32) - 2147483648ll) : CUDART_INF;
-      best_row[static_cast<size_t>(q) * k + t] = have ? static_cast<int32_t>(key & 0xffffffffull) : -1;
+      best_s[static_cast<size_t>(out) * k + t]   = have ? __ll2double_rn(static_cast<long long>(key >> 32) - 2147483648ll) : CUDART_INF;
+      best_row[static_cast<size_t>(out) * k + t] = have ? static_cast<int32_t>(key & 0xffffffffull) : -1;
     }
   } else {
     {
@@ -1641,8 +1646,8 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
     }
     for (int t = threadIdx.x; t < k; t += blockDim.x) {
       const bool have                         = t < m;
-      best_s[static_cast<size_t>(q) * k + t]   = have ? sc[t] : CUDART_INF;
-      best_row[static_cast<size_t>(q) * k + t] = have ? ids[t] : -1;
+      best_s[static_cast<size_t>(out) * k + t]   = have ? sc[t] : CUDART_INF;
+      best_row[static_cast<size_t>(out) * k + t] = have ? ids[t] : -1;
     }
   }
 }
@@ -1668,6 +1673,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
   int32_t* id         = reinterpret_cast<int32_t*>(s + n2max);
   int32_t* start      = reinterpret_cast<int32_t*>(stage_of(id + n2max));  // 16-byte aligned
   const int qb        = blockIdx.x, q = q0 + qb;
+  const int out       = cd.sel ? __ldg(cd.sel + q) : q;
   const int lane      = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t w     = kept[qb];
   if (w < 0) { return; }  // given up
@@ -1766,8 +1772,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
         for (int j = first; j < last; ++j) { place += pair_less(s[j], id[j], x[i], xi[i]) ? 1 : 0; }
       }
       if (place < k && !over) {
-        best_s[static_cast<size_t>(q) * k + place]   = x[i];
-        best_row[static_cast<size_t>(q) * k + place] = xi[i];
+        best_s[static_cast<size_t>(out) * k + place]   = x[i];
+        best_row[static_cast<size_t>(out) * k + place] = xi[i];
       }
       if (place == k - 1 && over) {
         report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, METRIC == kL2 && !kByteRows<T> ? 0.0 : query_sqnorm<T>(cd, queries, qpitch, d, q), x[i], ovf_list, ovf_count);
@@ -1781,8 +1787,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
     return;
   }
   for (int t = m + threadIdx.x; t < k; t += kSortThreads) {
-    best_s[static_cast<size_t>(q) * k + t]   = CUDART_INF;
-    best_row[static_cast<size_t>(q) * k + t] = -1;
+    best_s[static_cast<size_t>(out) * k + t]   = CUDART_INF;
+    best_row[static_cast<size_t>(out) * k + t] = -1;
   }
 }
 
@@ -2495,7 +2501,7 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
         go(verify_select_kernel<T, M, S, kFused>, dim3(nq), threads, q_bytes + pairs + tiles(threads));
         return;
       }
-      go(verify_select_kernel<T, M, S, kRank>, dim3(nq), 256, pairs);
+      go(verify_select_kernel<T, M, S, kRank>, dim3(nq), 1024, pairs);
       // (a batch has at most 32 768 queries: the second grid dimension takes them)
       go(verify_select_kernel<T, M, S, kScore>, dim3((n2max + kScoreRows - 1) / kScoreRows, nq), 128, q_bytes + tiles(128));
       const size_t smem = pairs + (kBuckets + 8) * sizeof(int32_t);
@@ -2750,6 +2756,11 @@ void launch_label_partition(const int32_t* labels, int64_t n, int32_t* labels_so
   cub::DeviceRunLengthEncode::Encode(temp, temp_bytes, labels_sorted, distinct, counts, n_distinct, n, s);
 }
 
+namespace {
+/// A thread per answer, as far as a block goes: with 64 threads the lists of 2048 took 32 turns, 23 us however few there were.
+int finish_threads(int k) { return std::min(1024, std::max(64, (k + 31) / 32 * 32)); }
+}  // namespace
+
 void launch_finish(const double* best_s, const int32_t* best_row, int64_t id_base, const void* queries, size_t qpitch,
                    int dtype, int d, int metric, int nq, int k, int64_t* neighbors, float* distances, double* scores_out,
                    cudaStream_t s)
@@ -2757,7 +2768,7 @@ void launch_finish(const double* best_s, const int32_t* best_row, int64_t id_bas
   if (nq <= 0) { return; }
   by_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
-    finish_kernel<T><<<nq, 64, 0, s>>>(best_s, best_row, nullptr, id_base, queries, qpitch, d, metric, k, neighbors, distances, scores_out);
+    finish_kernel<T><<<nq, finish_threads(k), 0, s>>>(best_s, best_row, nullptr, id_base, queries, qpitch, d, metric, k, neighbors, distances, scores_out);
   });
 }
 
@@ -2786,7 +2797,7 @@ void launch_merge(const double* in_s, const int64_t* in_id, int parts, int nq, i
   if (!finish) { return; }
   by_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
-    finish_kernel<T><<<nq, 64, 0, s>>>(scores_out, nullptr, neighbors, 0, queries, qpitch, d, metric, k, neighbors, distances, scores_out);
+    finish_kernel<T><<<nq, finish_threads(k), 0, s>>>(scores_out, nullptr, neighbors, 0, queries, qpitch, d, metric, k, neighbors, distances, scores_out);
   });
 }
 

@@ -76,6 +76,7 @@ void launch_sort_batch(const int32_t* e, int64_t n, int32_t id0, int64_t row0, c
 /// What a screen kept: cand [nq, ld] chains per query (see Candidate in screen_i8.cuh; ld a power of two, at least cap), cnt
 /// [nq] how many (more than cap: the list overflowed), and what turns a row of a chain into an id and the value the thresholds are made of: perm [n_rows]
 /// the id of a code row, init [n_rows] its e (int32, or float bits with fp16 codes; never: a removed row, or no row).
+/// sel (optional): the answers of query i go to list sel[i] (negative: there is no query i).
 /// Code rows n_rows + t, t < n_tail, stand for the ids tail_id0 + t; their entries hold the value itself (launch_tail). fp16
 /// codes also, indexed like the queries: shift (see launch_encode_f16_queries) and, but for the L2 metric, qq (see
 /// launch_query_sqnorms).
@@ -92,6 +93,7 @@ struct Candidates {
   const double* qq;
   int32_t tail_id0;
   int32_t n_tail;
+  const int32_t* sel;
 };
 
 /// The rows that were added after the label partition (ids tail_id0 .. tail_id0 + n_tail - 1), screened against the queries of
