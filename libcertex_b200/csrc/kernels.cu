@@ -1652,29 +1652,116 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
   }
 }
 
-// The third step of a split verification, block per query: its k best by (score, id). The scores are spread over kBuckets
-// equal intervals between the smallest and the largest, the buckets are laid out one after the other in shared memory, and a
-// row's place is the beginning of its bucket plus the rows of the bucket that come before it. A bitonic sort of 4096 pairs
-// moves 12 bytes a row 78 times through shared memory, which bounds it: 217 us for 512 lists of 2400 rows; this one takes
-// 44 us. (With most scores in one interval a row is compared with all others, which is as slow as the bitonic sort.)
+// Every thread of a block of NT: the m entries (score, id) that the threads hold (HELD each: entry threadIdx.x + i NT) in the
+// order of (score, id): emit(place, score, id) for the first k places. The scores are spread over 4 NT intervals, the buckets
+// are laid out one after the other in shared memory, and an entry's place is the beginning of its bucket plus the entries of
+// the bucket that come before it. The intervals grow with the distance from the worst score (NT / 4 per octave, 16 octaves):
+// the k best of a large set crowd at that end, the more so when a few are far better than the rest. A bitonic sort of 4096
+// pairs moves 12 bytes an entry 78 times through shared memory, which bounds it: 217 us for 512 lists of 2400 entries; this one
+// takes 44 us. (With most scores in one interval an entry is compared with all others, which is as slow as the bitonic
+// sort.) Shared memory: s [m] | id [m] | start [4 NT + 1], start 16-byte aligned.
+template <int NT, int HELD, typename Emit>
+__device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], int m, int k, double* s, int32_t* id, int32_t* start,
+                           Emit&& emit)
+{
+  constexpr int B      = 4 * NT;
+  constexpr int kShift = B == 4096 ? 15 : 17;  // of a float's bits: B / 16 intervals per octave
+  static_assert(B == 4096 || B == 1024, "16 octaves");
+  constexpr int W = NT / 32;
+  __shared__ double s_lo[W], s_hi[W];
+  __shared__ int s_sum[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double lo = CUDART_INF, hi = -CUDART_INF;
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    if (static_cast<int>(threadIdx.x) + i * NT < m) {
+      lo = fmin(lo, x[i]);
+      hi = fmax(hi, x[i]);
+    }
+  }
+  for (int i = threadIdx.x; i <= B; i += NT) { start[i] = 0; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) { s_lo[warp] = lo, s_hi[warp] = hi; }
+  __syncthreads();
+  lo = s_lo[lane & (W - 1)], hi = s_hi[lane & (W - 1)];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  // a larger score never has a smaller bucket: the difference, the product and the conversion round monotonically
+  const double scale = hi > lo ? 1.0 / (hi - lo) : 0.0;
+  auto bucket        = [&](double v) {
+    const int far = static_cast<int>(__float_as_uint(__double2float_rn((hi - v) * scale)) >> kShift) - ((127 - 16) << (23 - kShift));
+    return B - 1 - min(max(far, 0), B - 1);
+  };
+  int b[HELD], nth[HELD];
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    b[i] = -1;
+    if (static_cast<int>(threadIdx.x) + i * NT < m) {
+      b[i]   = bucket(x[i]);
+      nth[i] = atomicAdd(&start[b[i]], 1);
+    }
+  }
+  __syncthreads();
+  // counts -> first places: four buckets per thread
+  int4 c        = reinterpret_cast<int4*>(start)[threadIdx.x];
+  const int sum = c.x + c.y + c.z + c.w;
+  int incl      = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) { incl += v; }
+  }
+  if (lane == 31) { s_sum[warp] = incl; }
+  __syncthreads();
+  int before = incl - sum;
+  for (int w = 0; w < warp; ++w) { before += s_sum[w]; }
+  reinterpret_cast<int4*>(start)[threadIdx.x] = make_int4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
+  if (threadIdx.x == 0) { start[B] = m; }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    if (b[i] >= 0) {
+      const int at = start[b[i]] + nth[i];
+      s[at]        = x[i];
+      id[at]       = xi[i];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    if (b[i] >= 0) {
+      const int first = start[b[i]], last = start[b[i] + 1];
+      int place       = first;
+      if (first < k) {
+        for (int j = first; j < last; ++j) { place += pair_less(s[j], id[j], x[i], xi[i]) ? 1 : 0; }
+        if (place < k) { emit(place, x[i], xi[i]); }
+      }
+    }
+  }
+}
+
+// The third step of a split verification, block per query: its k best by (score, id).
 constexpr int kSortThreads = 1024;
 constexpr int kSortHeld    = 4;     // rows a thread holds: lists of at most 4096 rows
-constexpr int kBuckets     = 4096;
 template <typename T, int METRIC>
 __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
                                                                   int n2max, int k, double* best_s, int32_t* best_row,
                                                                   int32_t* ovf_list, unsigned int* ovf_count, Refine rf,
                                                                   const int32_t* kept)
 {
-  extern __shared__ double sh[];  // s [n2max] | id [n2max] | start [kBuckets + 1]
-  __shared__ double s_lo[32], s_hi[32];
-  __shared__ int s_sum[32];
+  extern __shared__ double sh[];  // s [n2max] | id [n2max] | start [4 kSortThreads + 1]
   double* s           = sh;
   int32_t* id         = reinterpret_cast<int32_t*>(s + n2max);
   int32_t* start      = reinterpret_cast<int32_t*>(stage_of(id + n2max));  // 16-byte aligned
   const int qb        = blockIdx.x, q = q0 + qb;
   const int out       = cd.sel ? __ldg(cd.sel + q) : q;
-  const int lane      = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t w     = kept[qb];
   if (w < 0) { return; }  // given up
   const bool over     = (w >> 30) != 0;
@@ -1682,7 +1769,6 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
   const double* far_s = reinterpret_cast<const double*>(cd.cand + static_cast<size_t>(qb) * cd.ld);
   double x[kSortHeld];
   int32_t xi[kSortHeld];
-  double lo = CUDART_INF, hi = -CUDART_INF;
 #pragma unroll
   for (int i = 0; i < kSortHeld; ++i) {
     const int at = threadIdx.x + i * kSortThreads;
@@ -1697,89 +1783,17 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
         x[i]  = far_s[at];
         xi[i] = reinterpret_cast<const int32_t*>(far_s + n2max)[at];
       }
-      lo = fmin(lo, x[i]);
-      hi = fmax(hi, x[i]);
     }
   }
-  for (int i = threadIdx.x; i <= kBuckets; i += kSortThreads) { start[i] = 0; }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  if (lane == 0) { s_lo[warp] = lo, s_hi[warp] = hi; }
-  __syncthreads();
-  lo = s_lo[lane], hi = s_hi[lane];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  // a larger score never has a smaller bucket: the difference and the product round monotonically
-  const double scale = hi > lo ? kBuckets / (hi - lo) : 0.0;
-  auto bucket        = [&](double v) { return min(max(static_cast<int>((v - lo) * scale), 0), kBuckets - 1); };
-  int b[kSortHeld], nth[kSortHeld];
-#pragma unroll
-  for (int i = 0; i < kSortHeld; ++i) {
-    b[i] = -1;
-    if (threadIdx.x + i * kSortThreads < m) {
-      b[i]   = bucket(x[i]);
-      nth[i] = atomicAdd(&start[b[i]], 1);
+  sort_block<kSortThreads, kSortHeld>(x, xi, m, k, s, id, start, [&](int place, double v, int32_t row) {
+    if (!over) {
+      best_s[static_cast<size_t>(out) * k + place]   = v;
+      best_row[static_cast<size_t>(out) * k + place] = row;
+    } else if (place == k - 1) {
+      const double qq = METRIC == kL2 && !kByteRows<T> ? 0.0 : query_sqnorm<T>(cd, queries, qpitch, d, q);
+      report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, qq, v, ovf_list, ovf_count);
     }
-  }
-  __syncthreads();
-  // counts -> first places: four buckets per thread
-  static_assert(kBuckets == 4 * kSortThreads, "one scan step");
-  int4 c        = reinterpret_cast<int4*>(start)[threadIdx.x];
-  const int sum = c.x + c.y + c.z + c.w;
-  int incl      = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) { incl += v; }
-  }
-  if (lane == 31) { s_sum[warp] = incl; }
-  __syncthreads();
-  if (warp == 0) {
-    int t = s_sum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) { t += v; }
-    }
-    s_sum[lane] = t;
-  }
-  __syncthreads();
-  const int before = incl - sum + (warp > 0 ? s_sum[warp - 1] : 0);
-  reinterpret_cast<int4*>(start)[threadIdx.x] = make_int4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
-  if (threadIdx.x == 0) { start[kBuckets] = m; }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kSortHeld; ++i) {
-    if (b[i] >= 0) {
-      const int at = start[b[i]] + nth[i];
-      s[at]        = x[i];
-      id[at]       = xi[i];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kSortHeld; ++i) {
-    if (b[i] >= 0) {
-      const int first = start[b[i]], last = start[b[i] + 1];
-      int place       = first;
-      if (first < k) {
-        for (int j = first; j < last; ++j) { place += pair_less(s[j], id[j], x[i], xi[i]) ? 1 : 0; }
-      }
-      if (place < k && !over) {
-        best_s[static_cast<size_t>(out) * k + place]   = x[i];
-        best_row[static_cast<size_t>(out) * k + place] = xi[i];
-      }
-      if (place == k - 1 && over) {
-        report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, METRIC == kL2 && !kByteRows<T> ? 0.0 : query_sqnorm<T>(cd, queries, qpitch, d, q), x[i], ovf_list, ovf_count);
-      }
-    }
-  }
+  });
   if (over) {
     if (threadIdx.x == 0 && m < k) {
       report_overflow<T, METRIC>(rf, q, qb, queries, qpitch, d, 0.0, CUDART_INF, ovf_list, ovf_count);
@@ -2015,117 +2029,184 @@ __global__ void group_columns_to_ids_kernel(int32_t* best_row, int k, const int3
   }
 }
 
-// Block per query: radix walk to the k-th smallest score, then the winners (ties: smallest rows) are gathered, sorted
-// and written. Shared memory: sel_s [k2] doubles | sel_id [k2] int32.
+// Block per query: the k smallest (score, row) of a row of scores (+inf and NaN: rows that do not count), sorted and written.
+// Bound by reading the row: once for its smallest and largest key, once for a histogram of 2048 intervals between them, once to
+// take the winners and the rows of the interval that holds the k-th, whose last places are given by counting. (A walk over fixed
+// 8-bit digits reads the row nine times, and its counters wait for one another: in the upper digits the scores of a row
+// are alike. 352 rows of 14 775 scores on average, k = 2048: 368 us; this one 99 us.) When the interval holds more than kPool rows
+// it is divided again; scores that are all equal go to the smallest rows.
+// Shared memory: sel_s [kk] doubles | sel_id [kk] int32 | pool_s [kPool] doubles | pool_id [kPool] int32 | bins, and after them
+// the sort's buckets; kk = k rounded up to a multiple of 4.
 // With `row_off` the score rows are ragged: row blockIdx.x starts at scores + row_off[blockIdx.x] and has row_n[] columns.
-__global__ void select_topk_kernel(const double* scores, int64_t ld, int64_t n_all, int k, const int32_t* qsel, int q0,
-                                   double* best_s, int32_t* best_row, int64_t chunk, double* part_s, int32_t* part_row,
-                                   const int64_t* row_off, const int32_t* row_n)
+constexpr int kPool = 1024, kBins = 2048;
+template <int NT>
+constexpr size_t select_smem(int k)
 {
+  return 12 * (static_cast<size_t>((k + 3) / 4 * 4) + kPool) + 4 * static_cast<size_t>(kBins > 4 * NT + 4 ? kBins : 4 * NT + 4);
+}
+template <int NT>
+__global__ void __launch_bounds__(NT) select_topk_kernel(const double* scores, int64_t ld, int64_t n_all, int k, const int32_t* qsel, int q0,
+                                                         double* best_s, int32_t* best_row, int64_t chunk, double* part_s,
+                                                         int32_t* part_row, const int64_t* row_off, const int32_t* row_n)
+{
+  using u64 = unsigned long long;
+  constexpr int W = NT / 32, kHeld = 2048 / NT;
   extern __shared__ double sh[];
-  __shared__ uint32_t hist[256];
-  __shared__ unsigned long long s_prefix;
-  __shared__ uint32_t s_remaining, s_less, s_eq_base;
-  const int k2        = max(next_pow2(k), 2);
-  double* sel_s       = sh;
-  int32_t* sel_id     = reinterpret_cast<int32_t*>(sh + k2);
+  __shared__ u64 s_min[W], s_max[W];
+  __shared__ int s_cnt[W], s_less, s_pool, s_bin, s_before, s_in_bin, s_eq;
+  const int kk    = (k + 3) / 4 * 4;
+  double* sel_s   = sh;
+  double* pool_s  = sel_s + kk;
+  int32_t* sel_id = reinterpret_cast<int32_t*>(pool_s + kPool);
+  int32_t* pool_id = sel_id + kk;
+  int32_t* bins   = pool_id + kPool;  // 16-byte aligned: everything before is a multiple of 16 bytes
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // blockIdx.y selects a chunk of columns [col0, col0 + n); with several chunks the winners go to part_* and are merged
-  const int64_t col0  = static_cast<int64_t>(blockIdx.y) * chunk;
+  const int64_t col0 = static_cast<int64_t>(blockIdx.y) * chunk;
   if (row_off) { n_all = row_n[blockIdx.x]; }
-  const int64_t n     = max(static_cast<int64_t>(0), min(chunk, n_all - col0));
-  const double* row   = scores + (row_off ? row_off[blockIdx.x] : static_cast<int64_t>(blockIdx.x) * ld) + col0;
-  const int64_t qout  = qsel ? qsel[blockIdx.x] : q0 + static_cast<int>(blockIdx.x);
-  const uint32_t want = static_cast<uint32_t>(min(static_cast<int64_t>(k), n));
+  const int64_t n    = max(static_cast<int64_t>(0), min(chunk, n_all - col0));
+  const double* row  = scores + (row_off ? row_off[blockIdx.x] : static_cast<int64_t>(blockIdx.x) * ld) + col0;
+  const int64_t qout = qsel ? qsel[blockIdx.x] : q0 + static_cast<int>(blockIdx.x);
 
-  for (int i = threadIdx.x; i < k2; i += blockDim.x) {
-    sel_s[i]  = CUDART_INF;
-    sel_id[i] = 0x7fffffff;
-  }
-  unsigned long long prefix = 0, mask = 0;
-  uint32_t remaining = want;
-  if (want > 0) {
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      for (int i = threadIdx.x; i < 256; i += blockDim.x) { hist[i] = 0; }
-      __syncthreads();
-      for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned long long key = ordered_key(row[i]);
-        if ((key & mask) == prefix) { atomicAdd(&hist[(key >> shift) & 255ull], 1u); }
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t cum = 0;
-        int b        = 0;
-        for (; b < 255; ++b) {
-          if (cum + hist[b] >= remaining) { break; }
-          cum += hist[b];
-        }
-        s_prefix    = prefix | (static_cast<unsigned long long>(b) << shift);
-        s_remaining = remaining - cum;
-      }
-      __syncthreads();
-      prefix    = s_prefix;
-      remaining = s_remaining;
-      mask |= 0xffull << shift;
-      __syncthreads();
+  u64 lo = ~0ull, hi = 0;
+  int counted = 0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += NT) {
+    const double v = row[i];
+    if (v < CUDART_INF) {
+      const u64 key = ordered_key(v);
+      lo = key < lo ? key : lo, hi = key > hi ? key : hi;
+      ++counted;
     }
-    // `prefix` is the key of the k-th smallest score; `remaining` of the rows that tie with it are wanted (smallest
-    // rows first), all rows below it are wanted.
-    const uint32_t n_less = want - remaining;
-    if (threadIdx.x == 0) {
-      s_less    = 0;
-      s_eq_base = 0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const u64 a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
+    lo = a < lo ? a : lo, hi = b > hi ? b : hi;
+  }
+  counted = __reduce_add_sync(0xffffffffu, counted);
+  if (lane == 0) { s_min[warp] = lo, s_max[warp] = hi, s_cnt[warp] = counted; }
+  if (threadIdx.x == 0) { s_less = 0, s_pool = 0, s_eq = 0; }
+  __syncthreads();
+  counted = 0;
+  for (int w = 0; w < W; ++w) {
+    lo = s_min[w] < lo ? s_min[w] : lo, hi = s_max[w] > hi ? s_max[w] : hi;
+    counted += s_cnt[w];
+  }
+  const int want = min(k, counted);
+  if (want > 0) {
+    // the interval [prefix << shift, (prefix + 1) << shift) of key - lo that holds the last winner
+    int above = 64 - __clzll(static_cast<long long>(hi - lo));  // bits of key - lo above which nothing differs
+    int shift = max(above - 11, 0), in_bin = 0, remaining = want;
+    u64 prefix = 0;
+    while (true) {
+      const u64 inside = (1ull << (above - shift)) - 1;  // 11 bits, or what is left
+      for (int i = threadIdx.x; i < kBins; i += NT) { bins[i] = 0; }
+      __syncthreads();
+#pragma unroll 4
+      for (int64_t i = threadIdx.x; i < n; i += NT) {
+        const double v = row[i];
+        if (v < CUDART_INF) {
+          const u64 d = ordered_key(v) - lo;
+          if (above == 64 || (d >> above) == prefix) { atomicAdd(&bins[(d >> shift) & inside], 1); }
+        }
+      }
+      __syncthreads();
+      // bins per thread in order, their running sum: the bin where it reaches `remaining`
+      constexpr int P = kBins / NT;
+      int c[P], sum = 0;
+#pragma unroll
+      for (int i = 0; i < P; ++i) { c[i] = bins[threadIdx.x * P + i], sum += c[i]; }
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) { incl += v; }
+      }
+      if (lane == 31) { s_cnt[warp] = incl; }
+      __syncthreads();
+      int before = incl - sum;
+      for (int w = 0; w < warp; ++w) { before += s_cnt[w]; }
+      if (before < remaining && before + sum >= remaining) {
+        int i = 0;
+        while (before + c[i] < remaining) { before += c[i++]; }
+        s_bin = threadIdx.x * P + i, s_before = before, s_in_bin = c[i];
+      }
+      __syncthreads();
+      prefix = (prefix << (above - shift)) + static_cast<u64>(s_bin);
+      remaining -= s_before;
+      in_bin = s_in_bin;
+      if (in_bin <= kPool || shift == 0) { break; }
+      above = shift;
+      shift = max(shift - 11, 0);
+    }
+    const int n_less = want - remaining;
+    const bool pooled = in_bin <= kPool;
+    for (int64_t i0 = 0; i0 < n; i0 += NT) {
+      const int64_t i = i0 + threadIdx.x;
+      const double v  = i < n ? row[i] : CUDART_INF;
+      const u64 d     = v < CUDART_INF ? (ordered_key(v) - lo) >> shift : ~0ull;
+      const bool less = v < CUDART_INF && d < prefix, eq = v < CUDART_INF && d == prefix;
+      const uint32_t bl = __ballot_sync(0xffffffffu, less), be = __ballot_sync(0xffffffffu, eq);
+      const uint32_t lt = (1u << lane) - 1u;
+      if (bl) {
+        int at = 0;
+        if (lane == 0) { at = atomicAdd(&s_less, __popc(bl)); }
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bl & lt);
+        if (less) { sel_s[at] = v, sel_id[at] = static_cast<int32_t>(col0 + i); }
+      }
+      if (pooled) {
+        if (be) {
+          int at = 0;
+          if (lane == 0) { at = atomicAdd(&s_pool, __popc(be)); }
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(be & lt);
+          if (eq) { pool_s[at] = v, pool_id[at] = static_cast<int32_t>(col0 + i); }
+        }
+      } else if (__syncthreads_or(eq)) {  // equal scores: the smallest rows, in the order of the row
+        if (lane == 0) { s_cnt[warp] = __popc(be); }
+        __syncthreads();
+        int at = s_eq + __popc(be & lt), total = 0;
+        for (int w = 0; w < W; ++w) {
+          at += w < warp ? s_cnt[w] : 0;
+          total += s_cnt[w];
+        }
+        if (eq && at < remaining) { sel_s[n_less + at] = v, sel_id[n_less + at] = static_cast<int32_t>(col0 + i); }
+        __syncthreads();
+        if (threadIdx.x == 0) { s_eq += total; }
+        __syncthreads();
+      }
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    __shared__ uint32_t warp_cnt[32];
-    for (int64_t c0 = 0; c0 < n; c0 += blockDim.x) {
-      const int64_t j = c0 + threadIdx.x;
-      double v        = 0;
-      bool eq         = false;
-      if (j < n) {
-        v                            = row[j];
-        const unsigned long long key = ordered_key(v);
-        if (key < prefix) {
-          const uint32_t pos = atomicAdd(&s_less, 1u);
-          sel_s[pos]         = v;
-          sel_id[pos]        = static_cast<int32_t>(col0 + j);
-        }
-        eq = key == prefix;
+    if (pooled) {
+      for (int i = threadIdx.x; i < in_bin; i += NT) {
+        const double v   = pool_s[i];
+        const int32_t vi = pool_id[i];
+        int place        = 0;
+        for (int j = 0; j < in_bin; ++j) { place += pair_less(pool_s[j], pool_id[j], v, vi) ? 1 : 0; }
+        if (place < remaining) { sel_s[n_less + place] = v, sel_id[n_less + place] = vi; }
       }
-      const int any = __syncthreads_count(eq);
-      if (any) {
-        const uint32_t ball = __ballot_sync(0xffffffffu, eq);
-        if (lane == 0) { warp_cnt[wid] = __popc(ball); }
-        __syncthreads();
-        uint32_t before = s_eq_base;
-        for (int w = 0; w < wid; ++w) { before += warp_cnt[w]; }
-        const uint32_t rank = before + __popc(ball & ((1u << lane) - 1u));
-        if (eq && rank < remaining) {
-          sel_s[n_less + rank]  = v;
-          sel_id[n_less + rank] = static_cast<int32_t>(col0 + j);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          uint32_t tot = 0;
-          for (int w = 0; w < nw; ++w) { tot += warp_cnt[w]; }
-          s_eq_base += tot;
-        }
-        __syncthreads();
-      }
+      __syncthreads();
     }
   }
+  double x[kHeld];
+  int32_t xi[kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int at = threadIdx.x + i * NT;
+    x[i]         = at < want ? sel_s[at] : CUDART_INF;
+    xi[i]        = at < want ? sel_id[at] : 0;
+  }
+  const size_t out = part_s ? (static_cast<size_t>(blockIdx.x) * gridDim.y + blockIdx.y) * k : static_cast<size_t>(qout) * k;
+  double* out_s    = part_s ? part_s : best_s;
+  int32_t* out_row = part_s ? part_row : best_row;
   __syncthreads();
-  bitonic_sort(sel_s, sel_id, k2);
-  for (int t = threadIdx.x; t < k; t += blockDim.x) {
-    const bool have = sel_s[t] < CUDART_INF;
-    if (part_s) {
-      const size_t o = (static_cast<size_t>(blockIdx.x) * gridDim.y + blockIdx.y) * k + t;
-      part_s[o]      = have ? sel_s[t] : CUDART_INF;
-      part_row[o]    = have ? sel_id[t] : 0x7fffffff;
-    } else {
-      best_s[static_cast<size_t>(qout) * k + t]   = have ? sel_s[t] : CUDART_INF;
-      best_row[static_cast<size_t>(qout) * k + t] = have ? sel_id[t] : -1;
-    }
+  sort_block<NT, kHeld>(x, xi, want, k, sel_s, sel_id, bins, [&](int place, double v, int32_t r) {
+    out_s[out + place]   = v;
+    out_row[out + place] = r;
+  });
+  for (int t = want + threadIdx.x; t < k; t += NT) {
+    out_s[out + t]   = CUDART_INF;
+    out_row[out + t] = part_s ? 0x7fffffff : -1;
   }
 }
 
@@ -2504,7 +2585,7 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
       go(verify_select_kernel<T, M, S, kRank>, dim3(nq), 1024, pairs);
       // (a batch has at most 32 768 queries: the second grid dimension takes them)
       go(verify_select_kernel<T, M, S, kScore>, dim3((n2max + kScoreRows - 1) / kScoreRows, nq), 128, q_bytes + tiles(128));
-      const size_t smem = pairs + (kBuckets + 8) * sizeof(int32_t);
+      const size_t smem = pairs + (4 * kSortThreads + 8) * sizeof(int32_t);
       allow_smem(sort_lists_kernel<T, M>, smem);
       sort_lists_kernel<T, M><<<nq, kSortThreads, smem, s>>>(queries, qpitch, d, q0, cd, n2max, k, best_s, best_row, ovf_list,
                                                              ovf_count, rf, kept);
@@ -2610,6 +2691,26 @@ void launch_dense_scores(const void* vectors, size_t pitch, int dtype, int d, in
   });
 }
 
+namespace {
+/// Rows of up to 8192 scores take blocks of 256 threads (many of them per SM), longer ones blocks of 1024.
+template <typename... Args>
+void launch_select(dim3 grid, int64_t n, const double* scores, int64_t ld, int64_t n_all, int k, Args... rest)
+{
+  auto go = [&](auto nt, const int32_t* qsel, int q0, double* best_s, int32_t* best_row, int64_t chunk, double* part_s, int32_t* part_row,
+                const int64_t* row_off, const int32_t* row_n, cudaStream_t s) {
+    constexpr int NT  = decltype(nt)::value;
+    const size_t smem = select_smem<NT>(k);
+    allow_smem(select_topk_kernel<NT>, smem);
+    select_topk_kernel<NT><<<grid, NT, smem, s>>>(scores, ld, n_all, k, qsel, q0, best_s, best_row, chunk, part_s, part_row, row_off, row_n);
+  };
+  if (n <= 8192) {
+    go(std::integral_constant<int, 256>{}, rest...);
+  } else {
+    go(std::integral_constant<int, 1024>{}, rest...);
+  }
+}
+}  // namespace
+
 int select_topk_parts(int64_t n, int k)
 {
   // long rows are cut into chunks that separate blocks select from; at most 8192 partial winners per query
@@ -2622,15 +2723,13 @@ void launch_select_topk(const double* scores, int64_t ld, int64_t n, int k, cons
                         double* best_s, int32_t* best_row, double* part_s, int32_t* part_row, cudaStream_t s)
 {
   if (nqb <= 0) { return; }
-  const int k2      = next_pow2(k) < 2 ? 2 : next_pow2(k);
-  const size_t smem = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(k2);
   const int parts   = select_topk_parts(n, k);
   if (parts == 1) {
-    select_topk_kernel<<<nqb, 256, smem, s>>>(scores, ld, n, k, qsel, q0, best_s, best_row, n, nullptr, nullptr, nullptr, nullptr);
+    launch_select(dim3(nqb), n, scores, ld, n, k, qsel, q0, best_s, best_row, n, nullptr, nullptr, nullptr, nullptr, s);
     return;
   }
   const int64_t chunk = (n + parts - 1) / parts;
-  select_topk_kernel<<<dim3(nqb, parts), 256, smem, s>>>(scores, ld, n, k, qsel, q0, best_s, best_row, chunk, part_s, part_row, nullptr, nullptr);
+  launch_select(dim3(nqb, parts), chunk, scores, ld, n, k, qsel, q0, best_s, best_row, chunk, part_s, part_row, nullptr, nullptr, s);
   const int n2       = next_pow2(parts * k);
   const size_t smem2 = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2);
   allow_smem(merge_partials_kernel, smem2);
@@ -2642,17 +2741,14 @@ void launch_select_topk_ragged(const double* scores, const int64_t* row_off, con
                                int32_t* part_row, cudaStream_t s)
 {
   if (nqb <= 0) { return; }
-  const int k2      = next_pow2(k) < 2 ? 2 : next_pow2(k);
-  const size_t smem = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(k2);
   const int parts   = select_topk_parts(n_max, k);
   if (parts == 1) {
-    select_topk_kernel<<<nqb, 256, smem, s>>>(scores, 0, 0, k, qsel, 0, best_s, best_row, std::max<int64_t>(n_max, 1), nullptr,
-                                              nullptr, row_off, row_n);
+    launch_select(dim3(nqb), n_max, scores, 0, 0, k, qsel, 0, best_s, best_row, std::max<int64_t>(n_max, 1), nullptr, nullptr, row_off,
+                  row_n, s);
     return;
   }
   const int64_t chunk = (n_max + parts - 1) / parts;
-  select_topk_kernel<<<dim3(nqb, parts), 256, smem, s>>>(scores, 0, 0, k, qsel, 0, best_s, best_row, chunk, part_s, part_row,
-                                                         row_off, row_n);
+  launch_select(dim3(nqb, parts), chunk, scores, 0, 0, k, qsel, 0, best_s, best_row, chunk, part_s, part_row, row_off, row_n, s);
   const int n2       = next_pow2(parts * k);
   const size_t smem2 = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2);
   allow_smem(merge_partials_kernel, smem2);
