@@ -1132,6 +1132,17 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
       const int64_t nt     = (h.n_in_part + kTile - 1) / kTile;
       const int64_t enough = (2 * static_cast<int64_t>(k) + per_tile - 1) / per_tile;
       const int64_t by_cap = (24 * static_cast<int64_t>(k) * nt + 10 * cap - 1) / (10 * static_cast<int64_t>(cap));
+      if (kb_ > 2) {
+        // Rows of more than two K blocks: a tile costs what its MMAs cost in either pass, and the pairs a looser threshold keeps
+        // cost little beside them (the epilogue's path for them hides behind the MMAs, the candidates are ranked before a row is
+        // read). So a quarter of the label will do, with chains of 16 rows as groups: 64 labels of 15 600 rows, 768 halves,
+        // 10 000 queries, k = 100: the pass 322 -> 118 us,
+        // 153 -> 413 rows kept and 129 -> 159 scored a query, the call 2356 -> 2289 us.
+        const int64_t least = std::max({(24 * static_cast<int64_t>(k) + 10 * per_tile - 1) / (10 * per_tile), enough, (nt + 3) / 4, by_cap});
+        steps[r]            = static_cast<int>(std::max<int64_t>(1, nt / least));
+        h.n_in_part         = (nt + steps[r] - 1) / steps[r] * kTile;  // tiles tile0, tile0 + step, ... to the label's end
+        continue;
+      }
       const int64_t take   = std::min(nt, std::max({int64_t(1024), enough, (nt + 15) / 16, by_cap}));
       if (take < nt) {
         steps[r]    = static_cast<int>(nt / take);  // tiles tile0, tile0 + step, ... stay inside the label
@@ -1367,9 +1378,9 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
     }
     run.queries.assign(order.begin() + i, order.begin() + j);
     // a threshold worth the passes needs about 2k groups: the k-th largest of them then sits near the best 1 % of the
-    // label. Groups are 64 rows, or single chains of 16 rows for labels too small for that.
+    // label. Groups are 64 rows, or single chains of 16 rows for labels too small for that and for a sample of long rows.
     const int64_t need = 2 * static_cast<int64_t>(k);
-    if (can_route && run.n_in_part / kGroupRows >= need) {
+    if (can_route && kb_ <= 2 && run.n_in_part / kGroupRows >= need) {
       routed.push_back(std::move(run));
     } else if (can_route && run.n_in_part / kChainRows >= need) {
       routed_fine.push_back(std::move(run));
