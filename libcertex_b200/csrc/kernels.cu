@@ -1388,15 +1388,19 @@ __device__ void report_overflow(const Refine& rf, int q, int qb, const void* que
   rf.thr2[pos] = t;
 }
 
-// The three steps (rank, score, sort) are one launch when a block's warps can score a query's rows side by side. With
-// longer lists (k > kSplitK) they are three: then scoring takes a block as many turns as lists are long, the blocks of a few
-// hundred queries fill the GPU unevenly (1.15 waves of them for 512 queries) and those of a few queries leave it idle, so the
-// rows to score are dealt out over the whole grid, 128 to a block, and the lists are sorted by blocks of 1024 threads
-// (sort_lists_kernel). The list of a query and its scores then lie in the memory of its candidates, which are no longer needed.
+// The three steps (rank, score, sort) are one launch when the lists are short and the rows too. With longer lists (k > 256)
+// scoring takes a block as many turns as lists are long, the blocks of a few hundred queries fill the GPU unevenly (1.15 waves
+// of them for 512 queries) and those of a few queries leave it idle; with long rows (kLongRow bytes and more than 32 answers) a
+// block holds the SM's shared memory through the steps in which it reads little, and the warps without 32 rows of their own
+// wait for the others'. So there the steps are launches of their own: the rows to score are dealt out over the whole grid, and the
+// lists are sorted by score intervals. The list of a query and its scores then lie in the memory of its candidates, which are
+// no longer needed.
 // 512 queries, k = 2048, 1 M x 128 halves (2402 rows a query): one launch 341 us; rank 38, score 97, sort 44 us.
+// 10 000 queries, k = 100, 768 floats, 159 rows a query (labels): rank 108, score 945, sort 85 us, the call 2304 -> 2063 us;
+// 220 rows a query: one launch 2316 us; rank 154, score 1516, sort 222 us.
 enum : int { kFused = 0, kRank = 1, kScore = 2 };
-constexpr int kSplitK    = 256;
-constexpr int kScoreRows = 128;  // rows a block of the scoring step takes
+constexpr int kSplitK  = 256;
+constexpr int kLongRow = 1024;
 template <typename T, int METRIC, bool STORED_XX, int PART>
 __global__ void __launch_bounds__(PART == kRank || kByteRows<T> ? 1024 : 256, PART == kRank || kByteRows<T> ? 1 : 3)
 verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* queries, size_t qpitch, int q0, Candidates cd,
@@ -1439,8 +1443,11 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
   };
   if constexpr (PART == kScore) {
     const int32_t w = kept[qb];  // how many rows are scored; negative: the query was given up; bit 30: its list overflowed
-    const int at    = static_cast<int>(blockIdx.x) * kScoreRows;
-    m               = min(kScoreRows, (w < 0 ? 0 : w & 0x3fffffff) - at);
+    const int all   = w < 0 ? 0 : w & 0x3fffffff;
+    // the rows in equal pieces of whole warps, but no fewer than the block's warps take at once
+    const int each  = max(static_cast<int>(blockDim.x), ((all + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + 31) / 32 * 32);
+    const int at    = static_cast<int>(blockIdx.x) * each;
+    m               = min(each, all - at);
     if (m <= 0) { return; }
     sc  = far_s + at;
     ids = far_ids + at;
@@ -1805,15 +1812,13 @@ __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], i
 }
 
 // The third step of a split verification, block per query: its k best by (score, id).
-constexpr int kSortThreads = 1024;
-constexpr int kSortHeld    = 4;     // rows a thread holds: lists of at most 4096 rows
-template <typename T, int METRIC>
-__global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
+template <typename T, int METRIC, int NT, int HELD>  // lists of at most NT HELD rows
+__global__ void __launch_bounds__(NT) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
                                                                   int n2max, int k, double* best_s, int32_t* best_row,
                                                                   int32_t* ovf_list, unsigned int* ovf_count, Refine rf,
                                                                   const int32_t* kept)
 {
-  extern __shared__ double sh[];  // s [n2max] | id [n2max] | start [4 kSortThreads + 1]
+  extern __shared__ double sh[];  // s [n2max] | id [n2max] | start [4 NT + 1]
   double* s           = sh;
   int32_t* id         = reinterpret_cast<int32_t*>(s + n2max);
   int32_t* start      = reinterpret_cast<int32_t*>(stage_of(id + n2max));  // 16-byte aligned
@@ -1824,11 +1829,11 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
   const bool over     = (w >> 30) != 0;
   const int m         = w & 0x3fffffff;
   const double* far_s = reinterpret_cast<const double*>(cd.cand + static_cast<size_t>(qb) * cd.ld);
-  double x[kSortHeld];
-  int32_t xi[kSortHeld];
+  double x[HELD];
+  int32_t xi[HELD];
 #pragma unroll
-  for (int i = 0; i < kSortHeld; ++i) {
-    const int at = threadIdx.x + i * kSortThreads;
+  for (int i = 0; i < HELD; ++i) {
+    const int at = threadIdx.x + i * NT;
     x[i]         = CUDART_INF;
     xi[i]        = 0x7fffffff;
     if (at < m) {
@@ -1842,7 +1847,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
       }
     }
   }
-  sort_block<kSortThreads, kSortHeld>(x, xi, m, k, s, id, start, [&](int place, double v, int32_t row) {
+  sort_block<NT, HELD>(x, xi, m, k, s, id, start, [&](int place, double v, int32_t row) {
     if (!over) {
       best_s[static_cast<size_t>(out) * k + place]   = v;
       best_row[static_cast<size_t>(out) * k + place] = row;
@@ -1857,7 +1862,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_lists_kernel(const void* qu
     }
     return;
   }
-  for (int t = m + threadIdx.x; t < k; t += kSortThreads) {
+  for (int t = m + threadIdx.x; t < k; t += NT) {
     best_s[static_cast<size_t>(out) * k + t]   = CUDART_INF;
     best_row[static_cast<size_t>(out) * k + t] = -1;
   }
@@ -2622,7 +2627,7 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
   if (nq <= 0) { return; }
   const int n2max  = cd.ld;
   const bool bytes = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys
-  const bool split = k > kSplitK;
+  const bool split = k > kSplitK || (!bytes && k > 32 && static_cast<size_t>(d) * dtype_size(dtype) >= kLongRow);
   const size_t q_bytes = bytes ? static_cast<size_t>((d + 15) / 16 * 16) : sizeof(double) * static_cast<size_t>(d);
   const size_t pairs   = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2max);
   // float rows: one staging tile per warp, + 16 bytes of alignment
@@ -2643,13 +2648,25 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
         go(verify_select_kernel<T, M, S, kFused>, dim3(nq), threads, q_bytes + pairs + tiles(threads));
         return;
       }
-      go(verify_select_kernel<T, M, S, kRank>, dim3(nq), 1024, pairs);
+      // blocks by the length of the lists: the candidates of a query are a few times k, the rows to score one to two k
+      const bool longer = k > kSplitK;
+      go(verify_select_kernel<T, M, S, kRank>, dim3(nq), longer ? 1024 : 128, pairs);
       // (a batch has at most 32 768 queries: the second grid dimension takes them)
-      go(verify_select_kernel<T, M, S, kScore>, dim3((n2max + kScoreRows - 1) / kScoreRows, nq), 128, q_bytes + tiles(128));
-      const size_t smem = pairs + (4 * kSortThreads + 8) * sizeof(int32_t);
-      allow_smem(sort_lists_kernel<T, M>, smem);
-      sort_lists_kernel<T, M><<<nq, kSortThreads, smem, s>>>(queries, qpitch, d, q0, cd, n2max, k, best_s, best_row, ovf_list,
-                                                             ovf_count, rf, kept);
+      const int threads = longer ? 128 : 64;
+      const int pieces  = longer ? (n2max + threads - 1) / threads : (2 * k + threads - 1) / threads;
+      go(verify_select_kernel<T, M, S, kScore>, dim3(pieces, nq), threads, q_bytes + tiles(threads));
+      auto sort = [&](auto nt, auto held) {
+        constexpr int NT = decltype(nt)::value, H = decltype(held)::value;
+        const size_t smem = pairs + (4 * NT + 8) * sizeof(int32_t);
+        allow_smem(sort_lists_kernel<T, M, NT, H>, smem);
+        sort_lists_kernel<T, M, NT, H><<<nq, NT, smem, s>>>(queries, qpitch, d, q0, cd, n2max, k, best_s, best_row, ovf_list, ovf_count,
+                                                            rf, kept);
+      };
+      if (n2max > 2048) {
+        sort(std::integral_constant<int, 1024>{}, std::integral_constant<int, 4>{});
+      } else {
+        sort(std::integral_constant<int, 256>{}, std::integral_constant<int, 8>{});
+      }
     };
     using std::integral_constant;
     if (metric == kL2) {
