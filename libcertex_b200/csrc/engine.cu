@@ -1475,7 +1475,7 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   return pairs;
 }
 
-int Index::anchor_stride_for(int64_t n, int k, int64_t nq) const
+int Index::anchor_stride_for(int64_t n, int k, int64_t nq, bool masked) const
 {
   // anchors: every stride-th row in whole tiles of 256, and at least 2k groups of 64 anchors, or the threshold would be
   // useless. The k-th largest group maximum is roughly the (stride * k)-th best row: for larger k the anchors are taken
@@ -1490,10 +1490,11 @@ int Index::anchor_stride_for(int64_t n, int k, int64_t nq) const
   //   1.2 M x 100 int8, 777 queries, k = 33, masked    433 (15) / 398 / 402 / 405 / 410
   //   300 000 x 128 half, 2000 queries, k = 100        445 (5) / 431 (3) / 437 / 487 (1)
   //   10 M x 128 uint8, 10 000 queries, k = 10         10 183 / 10 961 (12)
+  // (Anchors that are masked one by one cost an addition per element: half as many of them.)
   // Few queries are bound by reading the rows (1 M x 128 uint8, one query: 149 / 153 / - / 154), longer rows have MMAs enough to
   // hide that path (300 000 x 256 float: 441 / 438 / - / 453), and shards that share their thresholds keep few pairs each.
   if (kb_ <= 2 && nq > 4 * kQTile && threshold_hook == nullptr && topk_hook == nullptr) {
-    by_k = std::min(by_k, std::max<int64_t>(3, static_cast<int64_t>(std::sqrt(static_cast<double>(n) / k) / 50.0)));
+    by_k = std::min(by_k, std::max<int64_t>(3, static_cast<int64_t>(std::sqrt(static_cast<double>(n) / k) / (masked ? 25.0 : 50.0))));
   }
   return static_cast<int>(std::min<int64_t>({params_.anchor_stride, by_k, n / (kTile * ((2 * k + 3) / 4))}));
 }
@@ -1501,7 +1502,7 @@ int Index::anchor_stride_for(int64_t n, int k, int64_t nq) const
 bool Index::will_screen(int k) const
 {
   std::shared_lock<ReaderGate> lock(rw_);
-  return screen_kind_ != 0 && !code_overflow_ && test_mode_ != 1 && k >= 1 && anchor_stride_for(size_, k, 1) >= 1;
+  return screen_kind_ != 0 && !code_overflow_ && test_mode_ != 1 && k >= 1 && anchor_stride_for(size_, k, 1, false) >= 1;
 }
 
 /// Counters of a screened search as the device leaves them, copied to page-locked host memory behind the search.
@@ -1597,7 +1598,7 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
   // 39-62). A bitmap (a row of bits per query) and label searches without a partition score every vector.
   const bool filtered = (filter.words != nullptr && filter.bitmap_cols > 0) || filter.query_labels != nullptr;
 
-  const int stride    = anchor_stride_for(n, k, nq);
+  const int stride    = anchor_stride_for(n, k, nq, adm.bits != nullptr || n_removed_ * 64 > n);
   const bool screened = screen_kind_ != 0 && !code_overflow_ && !filtered && stride >= 1 && test_mode_ != 1;
 
   SearchStats& local = P.local;

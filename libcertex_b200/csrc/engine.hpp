@@ -282,7 +282,7 @@ class Index {
                    int q0, int nq, int k, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
                    unsigned long long* stats, int* err, int64_t n, int32_t* thr2, const float* shift, const double* qq, const Admit& adm,
                    std::vector<cudaEvent_t>* events, uint32_t* cnt) const;
-  int anchor_stride_for(int64_t n, int k, int64_t nq) const;
+  int anchor_stride_for(int64_t n, int k, int64_t nq, bool masked) const;
   void search_dense(const Resources& res, const void* q, size_t qpitch, const int32_t* qsel, int q0, int nqb, int k,
                     const Admit& adm, double* best_s, int32_t* best_row, int64_t n) const;
   /// Search by label over the label partition; returns the (query, row) pairs scored and counts its launches.
