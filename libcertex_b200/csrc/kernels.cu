@@ -2190,9 +2190,15 @@ __global__ void __launch_bounds__(NT) select_topk_kernel(const double* scores, i
       int before = incl - sum;
       for (int w = 0; w < warp; ++w) { before += s_cnt[w]; }
       if (before < remaining && before + sum >= remaining) {
-        int i = 0;
-        while (before + c[i] < remaining) { before += c[i++]; }
-        s_bin = threadIdx.x * P + i, s_before = before, s_in_bin = c[i];
+        bool found = false;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          if (!found && before + c[i] >= remaining) {
+            s_bin = threadIdx.x * P + i, s_before = before, s_in_bin = c[i];
+            found = true;
+          }
+          before += c[i];
+        }
       }
       __syncthreads();
       prefix = (prefix << (above - shift)) + static_cast<u64>(s_bin);
@@ -2788,6 +2794,14 @@ void launch_select(dim3 grid, int64_t n, const double* scores, int64_t ld, int64
   }
 }
 }  // namespace
+
+void load_select_topk()
+{
+  cudaFuncAttributes a;
+  cudaFuncGetAttributes(&a, select_topk_kernel<256>);
+  cudaFuncGetAttributes(&a, select_topk_kernel<1024>);
+  cudaFuncGetAttributes(&a, merge_partials_kernel);
+}
 
 int select_topk_parts(int64_t n, int k)
 {

@@ -208,6 +208,8 @@ void launch_dense_scores(const void* vectors, size_t pitch, int dtype, int d, in
 /// Long rows are selected from in select_topk_parts(n, k) chunks by separate blocks and merged; part_s / part_row are
 /// scratch of nqb * parts * k elements (unused when parts == 1).
 int select_topk_parts(int64_t n, int k);
+/// Loads the selection's kernels on the current device (a kernel is otherwise loaded at its first launch, which takes memory).
+void load_select_topk();
 void launch_select_topk(const double* scores, int64_t ld, int64_t n, int k, const int32_t* qsel, int q0, int nqb,
                         double* best_s, int32_t* best_row, double* part_s, int32_t* part_row, cudaStream_t s);
 

@@ -110,6 +110,7 @@ extern "C" cuvsError_t certexB200SearchStatic(cuvsResources_t res, cuvsDistanceT
       if (e != cudaSuccess || p == nullptr) {
         return fail(std::string("certex: cudaGetSymbolAddress of the static scratch failed: ") + cudaGetErrorString(e));
       }
+      load_select_topk();  // whichever of them this call needs: later calls of other sizes must not load anything
       g_scratch_address[device] = p;
     }
     scratch = static_cast<unsigned char*>(g_scratch_address[device]);
