@@ -204,7 +204,7 @@ struct ScreenShape {
 /// Shared memory of the resident-panel variant: panel_tiles * kb * 16 KB + n_stages * (kb * 32 KB + 1 KB) + the rest
 /// (screen_smem_bytes). The panel is what the call's query tiles split into evenly, at most 7 (kb = 1) or 2 (kb = 2) tiles;
 /// what it leaves goes to stages: a short panel is done with a stored tile soon, and the tiles in flight are what keeps
-/// the memory busy (one query over 1 M rows of 128 bytes: 27.6 us, 4.6 TB/s). Rows of more than two K blocks stream their K blocks
+/// the memory busy (one query over 1 M rows of 128 bytes, a call: 158 us with 2 stages, 157 with 3, 153 with 6). Rows of more than two K blocks stream their K blocks
 /// (two query tiles per segment, stages fixed by the kernel).
 ScreenShape shape_for(int kb, int nqt)
 {
@@ -2191,8 +2191,8 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   }
   CERTEX_CUDA(cudaGetLastError());
   // lists of chains, which become the caller's lists of rows
-  const uint32_t n_chains  = static_cast<uint32_t>((n + kChainRows - 1) / kChainRows);
-  const uint32_t chain_cap = mode == kModeScreen ? std::min(std::max<uint32_t>(cap, 2048), n_chains) : 0;
+  const uint32_t n_entries = static_cast<uint32_t>(kb > 2 ? n : (n + kChainRows - 1) / kChainRows);
+  const uint32_t chain_cap = mode == kModeScreen ? std::min(std::max<uint32_t>(cap, 2048), n_entries) : 0;
   Candidate* chains        = scratch.get<Candidate>(static_cast<size_t>(nq) * chain_cap);
   uint32_t* chain_cnt      = scratch.get<uint32_t>(static_cast<size_t>(nq));
   CERTEX_CUDA(cudaMemsetAsync(chain_cnt, 0, static_cast<size_t>(nq) * 4, res.stream));

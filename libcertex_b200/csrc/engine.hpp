@@ -346,7 +346,7 @@ class Index {
   /// chunk): a search then enqueues no copy from pageable host memory, which would make the host wait for the stream in
   /// the middle of the search.
   struct DevicePlan {
-    void* segs = nullptr;  // ScreenSeg[]
+    void* segs = nullptr;  // ScreenSeg[], and behind them in the same allocation
     int* begin = nullptr;  // [grid + 1]
   };
   DevicePlan device_plan(const Resources& res, int nqt, int nt, int panel_tiles, int grid, int chunk_tiles) const;  // empty: not kept, upload it

@@ -1365,7 +1365,6 @@ __device__ void report_overflow(const Refine& rf, int q, int qb, const void* que
   if (kth < CUDART_INF) {
     // the screen's value of a row as good as the k-th: <q, x> - |x|^2 / 2 (L2), <q, x> (inner product),
     // <q, x / |x|> (cosine)
-    
     if (!kByteRows<T> && METRIC == kL2) {  // the scores had no use for it
       const uint8_t* src = static_cast<const uint8_t*>(queries) + static_cast<size_t>(q) * qpitch;
       for (int i = 0; i < d; ++i) {

@@ -175,10 +175,10 @@ void launch_scatter_best(const double* s2, const int32_t* row2, const int32_t* s
 void launch_compose(int32_t* list, const unsigned int* n, int n_max, const int32_t* sel, cudaStream_t s);
 
 /**
- * The k best of every query's candidates by (exact fp64 score, id). One block per query: the candidates are ranked by the
- * screen's own values, and those that can belong to the k best are scored. A query with cnt > cap chains, or more than
- * ld rows in them, is appended to ovf_list and not answered. best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates exist). `where`
- * (8-bit rows only, optional): `vectors` is not in id order, row where[id] of it holds the vector with that id (the
+ * The k best of every query's candidates by (exact fp64 score, id): the candidates are ranked by the screen's own values, and
+ * those that can belong to the k best are scored. A query with cnt > cap entries, or more than ld rows in them, is appended
+ * to ovf_list and not answered. best_s / best_row [nq, k] (row -1, score +inf where fewer than k admitted candidates
+ * exist). `where` (8-bit rows only, optional): `vectors` is not in id order, row where[id] of it holds the vector with that id (the
  * norm-sorted code rows of an index whose vectors live in host memory). kept: scratch of nq ints; the candidates are
  * overwritten.
  */

@@ -36,7 +36,8 @@ struct ScreenSeg {
   int t1;
 };
 
-/// An entry of a query's candidate list: the rows of one chain that reached the query's threshold.
+/// An entry of a query's candidate list: the rows of one chain that reached the query's threshold (or, with rows of more than two
+/// K blocks, one of them).
 struct __align__(16) Candidate {
   uint32_t chain;   // rows 16 chain .. 16 chain + 15 of the code rows the pass read
   uint32_t mask;    // one bit per row of the chain
