@@ -895,12 +895,15 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
   const ScreenShape shape = shape_for(kb_, nqt);
   // anchors: sorted rows 0, stride, 2 stride, ...; only whole tiles of 256 anchors take part
   const int nt_anchor     = static_cast<int>(n / (static_cast<int64_t>(anchor_stride) * kTile));
-  const int n_groups      = nt_anchor * (kBaseTile / kGroupRows);
-  const int64_t ld_g      = round_up(n_groups, 8);
-
   // The threshold stage at the screen's price (chains of 16 adjacent anchors, e per chain: kModeGroupBound) unless
   // anchors are masked one by one: a bitset filter, or many removed rows (a chain with a masked anchor drops out whole).
   const bool chained   = adm.bits == nullptr && n_removed_ * 64 <= n && test_mode_ != 5;
+  // With far more groups than k, groups of 128 anchors do as well as groups of 64 (two of the k best anchors hardly share one:
+  // k^2 / groups pairs do) and leave half the values to write and to rank: 10 M x 128 bytes, 10 000 queries, k = 10:
+  // anchor pass 902 -> 825 us, the ranking of its values 136 -> 93 us, 161.4 pairs kept a query in either case.
+  const bool wide_groups = chained && static_cast<int64_t>(nt_anchor) * 2 >= 64 * static_cast<int64_t>(k);
+  const int n_groups     = nt_anchor * (wide_groups ? 2 : kBaseTile / kGroupRows);
+  const int64_t ld_g     = round_up(n_groups, 8);
   int32_t* anchor_init = scratch.get<int32_t>(chained ? static_cast<size_t>(nt_anchor) * (kTile / kChainRows)
                                                       : static_cast<size_t>(nt_anchor) * kTile);
   int32_t* gmax        = scratch.get<int32_t>(static_cast<size_t>(nq) * ld_g);
@@ -940,6 +943,7 @@ void Index::search_screened(const Resources& res, const uint8_t* qbuf, const flo
   a.err         = err;
   // 1 anchors: a value that some anchor of every group of 64 reaches (the group's maximum, or the chained bound)
   a.mode    = chained ? kModeGroupBound : kModeGroupMax;
+  a.wide_groups = wide_groups ? 1 : 0;
   a.init    = anchor_init;
   a.cmax    = anchor_init;
   a.gmax    = gmax;

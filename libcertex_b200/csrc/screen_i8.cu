@@ -696,6 +696,14 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
           // writes both values with one 8-byte store.
           int held = 0;  // kSplit: the value of the warp's first piece, until the second is known
           auto put = [&](int pc, int m) {
+            if (kSplit && MODE == kModeGroupBound && p.wide_groups) {  // both pieces of this warp are one group
+              if (pc == piece0) {
+                held = m;
+              } else if (q < p.nq) {
+                p.gmax[static_cast<size_t>(q) * p.ld_gmax + (t - col0) * 2 + (pc >> 1)] = max(held, m);  // (float keys order like ints)
+              }
+              return;
+            }
             int32_t* dst = p.gmax + static_cast<size_t>(q) * p.ld_gmax + (t - col0) * (kBaseTile / kGroupRows) + pc;
             if (!kSplit) {
               if (q < p.nq) { *dst = m; }

@@ -70,6 +70,7 @@ struct ScreenArgs {
   int wide;                       // 1: rows of more than two K blocks; a segment then has at most two query tiles
   int plain_tiles;                // GROUPMAX: tile t is rows [256 t, 256 t + 256) of a 2-D map (else the 3-D anchor map)
   int fine_groups;                // GROUPMAX: one maximum per 16 rows (16 columns of gmax per tile) instead of per 64 (4)
+  int wide_groups;                // GROUPBOUND: one value per 128 rows (2 columns of gmax per tile)
   int* err;                       // set to a non-zero code when a bounded wait gave up
   long long* trace;               // trace builds only (see screen_set_trace): [trace_units, 12] clock stamps of CTA 0
   int trace_units;
