@@ -780,7 +780,9 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
         // the tile is done: staged candidates go out once the buffer is half full (those beyond its end go straight to the
         // lists meanwhile), and the tile's e values are released (GROUPMAX)
         if (MODE == kModeScreen && __any_sync(0xffffffffu, kept)) {
-          const int staged = min(*rec_n, kRecBuf);
+          __syncwarp();  // a vote orders no memory: the entries were staged by single lanes, and flush reads those of all
+          // one lane's count decides for the warp, before any lane can stage an entry of the next tile
+          const int staged = __shfl_sync(0xffffffffu, min(*rec_n, kRecBuf), 0);
           if (staged > kRecBuf / 2) { flush(staged); }
         }
         if (kNeedE) {

@@ -127,6 +127,24 @@ def test_overflow_is_counted_and_written_entries_are_valid():
         assert keep[i, cand[i]].all() and len(set(cand[i].tolist())) == 8
 
 
+@pytest.mark.parametrize("cl", [128, 256, 384])
+@pytest.mark.parametrize("share", [1 / 500, 1 / 150, 1 / 40, 1 / 4, 1])
+def test_staged_candidates_arrive_whole_and_at_their_own_query(share, cl):
+    """A warp of the epilogue stages what its lanes keep in a tile (64 entries) and sends it to the lists once the buffer is
+    half full: shares of kept pairs that leave the buffer below that mark, send it in the middle, and run over it."""
+    nq, n = 300, 3072
+    q, x, init = _data(nq, n, cl, 0, seed=cl)
+    order = np.argsort(-init.astype(np.int64), kind="stable")
+    x, init = np.ascontiguousarray(x[order]), init[order]
+    acc = oracle.int_gram(q, x, init).astype(np.int64)
+    thr = np.quantile(acc, 1 - share, axis=1, method="lower").astype(np.int32) if share < 1 else np.full(nq, -(1 << 29), np.int32)
+    keep, _ = _kept(q, x, init, thr)
+    _, cnt, cand, _ = _run(0, q, x, init, thr=thr, cap=int(keep.sum(1).max()))
+    assert np.array_equal(cnt, keep.sum(1))
+    for i in range(nq):
+        assert np.array_equal(np.sort(cand[i, : cnt[i]]), np.nonzero(keep[i])[0])
+
+
 # ---------------------------------------------------------------------------------------------------- float16 codes
 def _run_f16(mode, hq, hx, e, thr=None, cap=64):
     """The pass on float16 code rows (code kind 2): e and thr are float32, passed as their bit patterns."""
