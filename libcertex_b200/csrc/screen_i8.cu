@@ -40,8 +40,8 @@
 // tiles and of one base tile (64 KB), the MMAs of both query tiles accumulate over the K blocks into the two TMEM slots,
 // and the e values of a tile travel through a small ring of their own.
 //
-// CTA = 18 warps: warps 0..15 are the epilogue (four warps per TMEM lane quarter, each owning one 64-column piece of
-// every unit), warp 16 lane 0 issues TMA loads (query panel once per segment, base tiles through a ring of stages),
+// CTA = 18 warps: warps 0..15 are the epilogue (two groups of 8, one per TMEM slot, each warp with two 64-column
+// pieces of a lane quarter), warp 16 lane 0 issues TMA loads (query panel once per segment, base tiles through a ring of stages),
 // warp 17 lane 0 issues tcgen05.mma. TMEM holds two accumulator slots of 256 columns: the MMAs of one unit run while the
 // epilogue reads the other; a slot goes back to the MMA warp as soon as its columns are in registers. No cluster
 // launch: each CTA loads its own tiles from its GPU's memory.
@@ -69,10 +69,6 @@ constexpr int kRecBuf     = 64;                // staged candidates per epilogue
 constexpr int kWideStage  = 2 * kQTileBytes + kBTileBytes;  // WIDE: one K block of two query tiles and a base tile
 constexpr int kWideStages = 3;
 constexpr int kERing      = 4;                 // WIDE: tiles whose e values may be in flight
-#ifndef CERTEX_SPLIT_EPILOGUE
-#define CERTEX_SPLIT_EPILOGUE 1
-#endif
-constexpr bool kSplit     = CERTEX_SPLIT_EPILOGUE != 0;  // two groups of 8 epilogue warps, one per TMEM slot
 
 #ifndef CERTEX_SCREEN_TRACE
 #define CERTEX_SCREEN_TRACE 0
@@ -271,7 +267,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
     }
     for (int i = 0; i < kSlots; ++i) {
       mbar_init(smem_u32(&ctl->tmem_full[i]), 1);
-      mbar_init(smem_u32(&ctl->tmem_empty[i]), kSplit ? kEpiWarps / 2 : kEpiWarps);
+      mbar_init(smem_u32(&ctl->tmem_empty[i]), kEpiWarps / 2);
     }
     mbar_init(smem_u32(&ctl->panel_full), 1);
     mbar_init(smem_u32(&ctl->panel_empty), 1);
@@ -513,7 +509,6 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
   } else if (MODE != kModeRate) {
     // ================================================================ epilogue (16 warps, one 64-column piece each)
     const int ew             = warp;
-    const int piece          = ew >> 2;   // which 64 columns of a unit
     const int quarter        = warp & 3;  // the TMEM lane quarter this warp may access
     const int row            = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
@@ -599,12 +594,12 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
 #if CERTEX_SCREEN_TRACE
     const bool tr_w = tr_cta && lane == 0 && ew == 0, tr_x = tr_cta && lane == 0 && ew == kEpiWarps - 1;
 #endif
-    // With kSplit the 16 warps form two groups of 8, one per TMEM slot: group g reads the units of slot g (every other
+    // The 16 warps form two groups of 8, one per TMEM slot: group g reads the units of slot g (every other
     // unit), each warp two 64-column pieces of it. A warp then has two unit times for the fixed latencies of a unit
     // (noticing its completion, tcgen05.ld, the release) and its comparisons run while the other group waits; the price
     // is a later release: the second piece can only be loaded into the registers the first has left.
-    const uint32_t grp = kSplit ? static_cast<uint32_t>(ew) >> 3 : 0u;
-    const int piece0   = kSplit ? ((ew >> 2) & 1) * 2 : piece;  // first (or only) 64-column piece of this warp
+    const uint32_t grp = static_cast<uint32_t>(ew) >> 3;
+    const int piece0   = ((ew >> 2) & 1) * 2;  // first 64-column piece of this warp
     const uint32_t taddr_w = tmem + lane_base + static_cast<uint32_t>(piece0 * kGroupRows);
     for (int s = 0; s < nseg && ok; ++s) {
       const ScreenSeg sg = segs[s];
@@ -617,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
         int4 ce0 = make_int4(0, 0, 0, 0), ce1 = ce0;
         if (kChainE) {
           ce0 = __ldg(cm);
-          if (kSplit) { ce1 = __ldg(cm + 1); }
+          ce1 = __ldg(cm + 1);
         }
         if (kNeedE) {
           // the tile's e values landed with (or, WIDE, ahead of) its code rows. Every warp waits for them, also one
@@ -632,7 +627,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
         int q              = q_first;
         for (int j = 0; j < nqt; ++j, ++gu, q += kQueryTile) {
           const uint32_t slot = gu & 1u;
-          if (kSplit && slot != grp) { continue; }
+          if (slot != grp) { continue; }
           int thr = never_thr;
           if (MODE == kModeScreen && q < p.nq) { thr = __ldg(p.thr + q); }
           TRACE_AT(tr_w, gu, 3);
@@ -694,9 +689,9 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
           // One group value per 64-column piece. Rows of gmax are far apart, so every 4-byte store of a thread is a memory
           // transaction of its own; with the two-group epilogue a thread holds two adjacent pieces of its row and
           // writes both values with one 8-byte store.
-          int held = 0;  // kSplit: the value of the warp's first piece, until the second is known
+          int held = 0;  // the value of the warp's first piece, until the second is known
           auto put = [&](int pc, int m) {
-            if (kSplit && MODE == kModeGroupBound && p.wide_groups) {  // both pieces of this warp are one group
+            if (MODE == kModeGroupBound && p.wide_groups) {  // both pieces of this warp are one group
               if (pc == piece0) {
                 held = m;
               } else if (q < p.nq) {
@@ -705,9 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
               return;
             }
             int32_t* dst = p.gmax + static_cast<size_t>(q) * p.ld_gmax + (t - col0) * (kBaseTile / kGroupRows) + pc;
-            if (!kSplit) {
-              if (q < p.nq) { *dst = m; }
-            } else if (pc == piece0) {
+            if (pc == piece0) {
               held = m;
             } else if (q < p.nq) {
               *reinterpret_cast<int2*>(dst - 1) = make_int2(held, m);
@@ -725,54 +718,39 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
               put(pc, F16 ? float_key(fmaxf(__int_as_float(m4.x), __int_as_float(m4.z))) : max(m4.x, m4.z));
             }
           };
-          if (!kSplit) {
-            release();
-            if (MODE == kModeScreen) {
-              screen32(a, ce0.x, ce0.y, row0);
-              screen32(b, ce0.z, ce0.w, row0 + 32);
-            } else if (MODE == kModeGroupBound) {
-              bound_store(bound32(a, ce0.x, ce0.y), bound32(b, ce0.z, ce0.w), piece0);
-            } else {
-              int4 m4 = make_int4(0, 0, 0, 0);
-              gmax32(a, e, m4.x, m4.y);
-              gmax32(b, e + 32, m4.z, m4.w);
-              gmax_store(m4, piece0);
-            }
+          // first piece; each half of the second piece is fetched as soon as its registers are free
+          int4 m4 = make_int4(0, 0, 0, 0);
+          int ma = 0, mb = 0;
+          if (MODE == kModeScreen) {
+            screen32(a, ce0.x, ce0.y, row0);
+          } else if (MODE == kModeGroupBound) {
+            ma = bound32(a, ce0.x, ce0.y);
           } else {
-            // first piece; each half of the second piece is fetched as soon as its registers are free
-            int4 m4 = make_int4(0, 0, 0, 0);
-            int ma = 0, mb = 0;
-            if (MODE == kModeScreen) {
-              screen32(a, ce0.x, ce0.y, row0);
-            } else if (MODE == kModeGroupBound) {
-              ma = bound32(a, ce0.x, ce0.y);
-            } else {
-              gmax32(a, e, m4.x, m4.y);
-            }
-            tmem_ld32(taddr + 64, a);
-            if (MODE == kModeScreen) {
-              screen32(b, ce0.z, ce0.w, row0 + 32);
-            } else if (MODE == kModeGroupBound) {
-              mb = bound32(b, ce0.z, ce0.w);
-            } else {
-              gmax32(b, e + 32, m4.z, m4.w);
-            }
-            tmem_ld32(taddr + 96, b);
-            if (MODE == kModeGroupBound) { bound_store(ma, mb, piece0); }
-            if (MODE == kModeGroupMax) { gmax_store(m4, piece0); }
-            tmem_wait_ld(a);
-            reg_fence32(b);
-            release();
-            if (MODE == kModeScreen) {
-              screen32(a, ce1.x, ce1.y, row0 + 64);
-              screen32(b, ce1.z, ce1.w, row0 + 96);
-            } else if (MODE == kModeGroupBound) {
-              bound_store(bound32(a, ce1.x, ce1.y), bound32(b, ce1.z, ce1.w), piece0 + 1);
-            } else {
-              gmax32(a, e + 64, m4.x, m4.y);
-              gmax32(b, e + 96, m4.z, m4.w);
-              gmax_store(m4, piece0 + 1);
-            }
+            gmax32(a, e, m4.x, m4.y);
+          }
+          tmem_ld32(taddr + 64, a);
+          if (MODE == kModeScreen) {
+            screen32(b, ce0.z, ce0.w, row0 + 32);
+          } else if (MODE == kModeGroupBound) {
+            mb = bound32(b, ce0.z, ce0.w);
+          } else {
+            gmax32(b, e + 32, m4.z, m4.w);
+          }
+          tmem_ld32(taddr + 96, b);
+          if (MODE == kModeGroupBound) { bound_store(ma, mb, piece0); }
+          if (MODE == kModeGroupMax) { gmax_store(m4, piece0); }
+          tmem_wait_ld(a);
+          reg_fence32(b);
+          release();
+          if (MODE == kModeScreen) {
+            screen32(a, ce1.x, ce1.y, row0 + 64);
+            screen32(b, ce1.z, ce1.w, row0 + 96);
+          } else if (MODE == kModeGroupBound) {
+            bound_store(bound32(a, ce1.x, ce1.y), bound32(b, ce1.z, ce1.w), piece0 + 1);
+          } else {
+            gmax32(a, e + 64, m4.x, m4.y);
+            gmax32(b, e + 96, m4.z, m4.w);
+            gmax_store(m4, piece0 + 1);
           }
           TRACE_AT(tr_w, gu, 7);
         }
