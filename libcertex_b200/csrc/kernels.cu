@@ -2000,6 +2000,7 @@ __global__ void compose_kernel(int32_t* list, const unsigned int* n, const int32
 
 // ------------------------------------------------------------------------------------------- dense path
 constexpr int kDenseQ = 4;  // queries per block that share one walk over a stored row
+constexpr size_t kDenseMost = kMaxSmem - 256;  // dynamic shared memory of a block of them, beside their own variables
 
 template <typename T, int METRIC>
 __global__ void dense_scores_kernel(const uint8_t* vectors, size_t pitch, int d, int64_t n, const void* queries,
@@ -2428,11 +2429,16 @@ void by_dtype(int dtype, F&& f)
   }
 }
 
+/// Opts in to the shared memory of a launch. The limit belongs to the function on its device, not to the calling thread: it is
+/// set to `most`, the largest that any launch of the kernel takes, so that a thread with a small call cannot lower it
+/// between another thread's call of this function and its launch. (Setting it each time serves every device and context.)
 template <typename Kernel>
-void allow_smem(Kernel kernel, size_t bytes)
+void allow_smem(Kernel kernel, size_t bytes, size_t most)
 {
   // the 48 KB that need no opt-in include the kernel's static shared memory: leave room for it
-  if (bytes > 32 * 1024) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)); }
+  if (bytes > 32 * 1024) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(std::max(bytes, most)));
+  }
 }
 
 }  // namespace
@@ -2607,8 +2613,9 @@ void launch_kth_largest(const int32_t* gmax, int64_t ld, int ng, int k, int nq, 
     return;
   }
   const size_t bytes = static_cast<size_t>(ng) * 4;
-  const int in_smem  = bytes <= 160 * 1024;
-  if (in_smem) { allow_smem(kth_largest_kernel, bytes); }
+  constexpr size_t kMost = 160 * 1024;
+  const int in_smem  = bytes <= kMost;
+  if (in_smem) { allow_smem(kth_largest_kernel, bytes, kMost); }
   // short rows: smaller blocks, more of them per SM (the kernel is a chain of block-wide barriers)
   const int threads = ng > 4096 ? 512 : 2 * k <= 128 ? 128 : 2 * k <= 256 ? 256 : 512;
   kth_largest_kernel<<<nq, threads, in_smem ? bytes : 0, s>>>(gmax, ld, ng, k, thr, in_smem, ng_rows, never, topk, shift, zero);
@@ -2640,7 +2647,9 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
   by_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
     auto go = [&](auto kernel, dim3 grid, int threads, size_t smem) {
-      allow_smem(kernel, smem);
+      // 2048 coordinates of a float query, lists of 4096, tiles of 8 warps
+      constexpr size_t kMost = 8 * 2048 + 12 * 4096 + 16 + 8 * 32 * kStageStride;
+      allow_smem(kernel, smem, kMost);
       kernel<<<grid, threads, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch, q0, cd, n2max, k, adm,
                                          best_s, best_row, ovf_list, ovf_count, stats, rf, where, sqnorm, kept);
     };
@@ -2663,7 +2672,7 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
       auto sort = [&](auto nt, auto held) {
         constexpr int NT = decltype(nt)::value, H = decltype(held)::value;
         const size_t smem = pairs + (4 * NT + 8) * sizeof(int32_t);
-        allow_smem(sort_lists_kernel<T, M, NT, H>, smem);
+        allow_smem(sort_lists_kernel<T, M, NT, H>, smem, 12 * NT * H + (4 * NT + 8) * sizeof(int32_t));
         sort_lists_kernel<T, M, NT, H><<<nq, NT, smem, s>>>(queries, qpitch, d, q0, cd, n2max, k, best_s, best_row, ovf_list, ovf_count,
                                                             rf, kept);
       };
@@ -2761,7 +2770,7 @@ void launch_dense_scores(const void* vectors, size_t pitch, int dtype, int d, in
   by_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
     auto go = [&](auto kernel) {
-      allow_smem(kernel, smem);
+      allow_smem(kernel, smem, kDenseMost);
       kernel<<<grid, 256, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, n, queries, qpitch, qsel, q0, nqb, adm, out, ld);
     };
     if (metric == kL2) {
@@ -2783,7 +2792,7 @@ void launch_select(dim3 grid, int64_t n, const double* scores, int64_t ld, int64
                 const int64_t* row_off, const int32_t* row_n, cudaStream_t s) {
     constexpr int NT  = decltype(nt)::value;
     const size_t smem = select_smem<NT>(k);
-    allow_smem(select_topk_kernel<NT>, smem);
+    allow_smem(select_topk_kernel<NT>, smem, select_smem<NT>(2048));
     select_topk_kernel<NT><<<grid, NT, smem, s>>>(scores, ld, n_all, k, qsel, q0, best_s, best_row, chunk, part_s, part_row, row_off, row_n);
   };
   if (n <= 8192) {
@@ -2823,7 +2832,7 @@ void launch_select_topk(const double* scores, int64_t ld, int64_t n, int k, cons
   launch_select(dim3(nqb, parts), chunk, scores, ld, n, k, qsel, q0, best_s, best_row, chunk, part_s, part_row, nullptr, nullptr, s);
   const int n2       = next_pow2(parts * k);
   const size_t smem2 = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2);
-  allow_smem(merge_partials_kernel, smem2);
+  allow_smem(merge_partials_kernel, smem2, (sizeof(double) + sizeof(int32_t)) * 8192);
   merge_partials_kernel<<<nqb, 256, smem2, s>>>(part_s, part_row, parts, k, n2, qsel, q0, best_s, best_row);
 }
 
@@ -2842,7 +2851,7 @@ void launch_select_topk_ragged(const double* scores, const int64_t* row_off, con
   launch_select(dim3(nqb, parts), chunk, scores, 0, 0, k, qsel, 0, best_s, best_row, chunk, part_s, part_row, row_off, row_n, s);
   const int n2       = next_pow2(parts * k);
   const size_t smem2 = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2);
-  allow_smem(merge_partials_kernel, smem2);
+  allow_smem(merge_partials_kernel, smem2, (sizeof(double) + sizeof(int32_t)) * 8192);
   merge_partials_kernel<<<nqb, 256, smem2, s>>>(part_s, part_row, parts, k, n2, qsel, 0, best_s, best_row);
 }
 
@@ -2856,7 +2865,7 @@ void launch_dense_scores_grouped(const void* vectors, size_t pitch, int dtype, i
   by_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
     auto go = [&](auto kernel) {
-      allow_smem(kernel, smem);
+      allow_smem(kernel, smem, kDenseMost);
       kernel<<<static_cast<unsigned>(n_blocks), 256, smem, s>>>(static_cast<const uint8_t*>(vectors), pitch, d, queries, qpitch,
                                                                  order, groups, n_groups, part_ids, tail0, n_tail, adm, out);
     };
@@ -2978,7 +2987,7 @@ void launch_merge(const double* in_s, const int64_t* in_id, int parts, int nq, i
   } else {
     const int n2      = next_pow2(parts * k) < 2 ? 2 : next_pow2(parts * k);
     const size_t smem = (sizeof(double) + sizeof(int64_t)) * static_cast<size_t>(n2);
-    allow_smem(merge_kernel, smem);
+    allow_smem(merge_kernel, smem, (sizeof(double) + sizeof(int64_t)) * 8192);
     merge_kernel<<<nq, 256, smem, s>>>(in_s, in_id, parts, nq, k, n2, scores_out, neighbors, part_stride);
   }
   if (!finish) { return; }

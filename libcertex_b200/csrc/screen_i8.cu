@@ -808,7 +808,6 @@ cudaError_t screen_i8_launch(const CUtensorMap& tm_q, const CUtensorMap& tm_x, c
   args.trace       = g_trace;
   args.trace_units = g_trace_units;
   const size_t smem = screen_smem_bytes(args.kb, args.panel_tiles, args.n_stages);
-  // opt-in to large dynamic shared memory (cheap; set on every launch so that every device of the process has it)
   if (!args.wide && args.kb != 1 && args.kb != 2) { return cudaErrorInvalidValue; }
   const bool kb2 = args.kb == 2;
   auto kernel    = kb2 ? screen_i8_kernel<kModeRate, false, false, 2> : screen_i8_kernel<kModeRate, false, false, 1>;
@@ -827,7 +826,10 @@ cudaError_t screen_i8_launch(const CUtensorMap& tm_q, const CUtensorMap& tm_x, c
              : args.f16 ? (kb2 ? screen_i8_kernel<kModeGroupMax, true, false, 2> : screen_i8_kernel<kModeGroupMax, true, false, 1>)
                         : (kb2 ? screen_i8_kernel<kModeGroupMax, false, false, 2> : screen_i8_kernel<kModeGroupMax, false, false, 1>);
   }
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  // Opt-in to large dynamic shared memory (cheap; set on every launch so that every device of the process has it). Launches of
+  // one kernel differ in `smem` (screen_smem_bytes), and the limit is the function's, not the thread's: always the most, or a
+  // search of another thread could lower it before this launch.
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem));
   if (e != cudaSuccess) { return e; }
   kernel<<<grid, kThreads, smem, stream>>>(tm_q, tm_x, args);
   return cudaGetLastError();
