@@ -325,6 +325,11 @@ CERTEX_B200_EXPORT cuvsError_t certexB200PackMask(cuvsResources_t res, const uin
  *  labels in ascending order. */
 CERTEX_B200_EXPORT cuvsError_t certexB200OrderByLabel(const int32_t* labels, int64_t n, int32_t* order);
 
+/** Test hook (host only): what gives the thresholds of a label of `rows` vectors in a search by labels, where a vector takes
+ *  k_blocks blocks of 128 bytes: out[0] rows of a group, out[1] every how many of the label's tiles of 256 rows, out[2] how many
+ *  of them. */
+CERTEX_B200_EXPORT cuvsError_t certexB200LabelSample(int32_t k_blocks, int64_t rows, int32_t k, int64_t* out);
+
 /** Test hook (host only): the split that searches use, with the base tiles taken in chunks of chunk_tiles (0: one
  *  chunk) so that a chunk's rows stay in L2 while every query panel passes over them. segs receives 4 ints per segment
  *  (as above), *n_segs their number (at most cap_segs), seg_begin [grid + 1] the range of every CTA. */

@@ -116,7 +116,7 @@ SYMBOLS = [
     "certexB200CommGetUniqueId", "certexB200CommInitRank", "certexB200CommAdopt", "certexB200CommDestroy",
     "certexB200DistributedSearch", "certexB200ScreenTrace", "certexB200PlanChunked",
     "certexB200DistributedSearchBegin", "certexB200DistributedSearchEnd", "certexB200OrderByLabel",
-    "certexB200PackMask", "certexB200ToHalf",
+    "certexB200PackMask", "certexB200ToHalf", "certexB200LabelSample",
 ]
 
 # void hook(void* ctx, int32_t* keys, int64_t n, cudaStream_t stream)
@@ -201,6 +201,7 @@ def lib():
                 L.certexB200ToHalf.argtypes = [vp, vp, ctypes.c_int32, i64, vp, P(ctypes.c_int32)]
                 L.certexB200PackMask.argtypes = [vp, vp, i64, vp]
                 L.certexB200ScreenTrace.argtypes = [vp, ctypes.c_int32]
+                L.certexB200LabelSample.argtypes = [ctypes.c_int32, i64, ctypes.c_int32, P(i64)]
                 L.certexB200OrderByLabel.argtypes = [P(ctypes.c_int32), i64, P(ctypes.c_int32)]
                 L.certexB200SearchStatic.argtypes = [vp, ctypes.c_int, DLDataType, vp, i64, vp, i64, i64, ctypes.c_int32, vp, vp]
                 _lib = L

@@ -625,6 +625,14 @@ cuvsError_t certexB200OrderByLabel(const int32_t* labels, int64_t n, int32_t* or
   });
 }
 
+cuvsError_t certexB200LabelSample(int32_t k_blocks, int64_t rows, int32_t k, int64_t* out)
+{
+  return translate([=] {
+    CERTEX_EXPECTS(out != nullptr, "certex: null argument");
+    label_sample(k_blocks, rows, k, out);
+  });
+}
+
 cuvsError_t certexB200PlanRouted(int32_t n_runs, const int32_t* n_query_tiles, const int32_t* n_base_tiles,
                                  int32_t panel_tiles, int32_t grid, int32_t max_segs, int32_t* segs, int32_t cap_segs,
                                  int32_t* n_segs, int32_t* seg_begin, int32_t* runs_done)

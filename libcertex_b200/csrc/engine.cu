@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <istream>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <ostream>
@@ -1087,7 +1088,57 @@ size_t plan_routed(const std::vector<LabelRun>& runs, size_t r0, size_t r1, cons
   return done - r0;
 }
 
+/// The tiles of a label (nt tiles) that give its queries' thresholds: every step-th one from the first, `tiles` of them.
+struct LabelSample {
+  int step;
+  int64_t tiles;
+};
+
+/// The thresholds of a large label come from a strided sample of its tiles (its rows are sorted by norm, so the sample
+/// spans all norms; the group maxima of any subset of rows are valid): at least 1024 tiles (smaller labels take part
+/// whole: every tile left out costs survivors, and their exact scores cost more than the tile), enough tiles for
+/// 2k groups, for a sixteenth of the label, and for candidate lists that stay within half their capacity (about
+/// 1.2 k rows per sampled fraction).
+LabelSample sample_label(int kb, int64_t nt, int k, bool fine)
+{
+  const int per_tile   = fine ? kBaseTile / kChainRows : kBaseTile / kGroupRows;
+  const int64_t cap    = std::max(2048, 2 * k);
+  const int64_t enough = (2 * static_cast<int64_t>(k) + per_tile - 1) / per_tile;
+  const int64_t by_cap = (24 * static_cast<int64_t>(k) * nt + 10 * cap - 1) / (10 * cap);
+  const int64_t take   = std::min(nt, std::max({int64_t(1024), enough, (nt + 15) / 16, by_cap}));
+  if (kb > 2) {
+    // Rows of more than two K blocks: a tile costs what its MMAs cost in either pass, and the pairs a looser threshold keeps
+    // cost little beside them (the epilogue's path for them hides behind the MMAs, the candidates are ranked before a row is
+    // read). So a quarter of the label will do where that is less than the rule above asks for: 64 labels of 15 600 rows, 768
+    // halves, chains of 16 rows as groups, 10 000 queries, k = 100: the pass 322 -> 118 us,
+    // 153 -> 413 rows kept and 129 -> 159 scored a query, the call 2356 -> 2289 us.
+    const int64_t least = std::max({(24 * static_cast<int64_t>(k) + 10 * per_tile - 1) / (10 * per_tile), enough, (nt + 3) / 4, by_cap});
+    const int64_t step  = std::max<int64_t>(1, nt / std::min(least, take));
+    return LabelSample{static_cast<int>(step), (nt + step - 1) / step};  // to the label's end
+  }
+  return LabelSample{take < nt ? static_cast<int>(nt / take) : 1, take};  // the sample stays inside the label
+}
+
+/// Whether thresholds come from chains of 16 rows or from groups of 64, by the rows of the largest label: from chains where it has
+/// too few groups of 64 (2k make a threshold worth the passes), and for long rows, whose sample is a part of the label, as long as a
+/// query has no more values than the 1024 tiles of a large label give in groups of 64. Beyond that chains add more to what is
+/// written and ranked than they save: a label of 2 M rows of 300 bytes, 3000 queries, k = 10, with 31 252 values a query (chains, a
+/// quarter of the tiles) 3.73 ms, with 4468 values 2.57; eight labels of 250 000 rows of 256 halves, k = 100, 2.73 either way.
+bool fine_groups(int kb, int64_t rows, int k)
+{
+  if (rows / kGroupRows < 2 * static_cast<int64_t>(k)) { return true; }
+  return kb > 2 && sample_label(kb, (rows + kTile - 1) / kTile, k, true).tiles * (kBaseTile / kChainRows) <= 4096;
+}
+
 }  // namespace
+
+void label_sample(int kb, int64_t rows, int k, int64_t* out)
+{
+  CERTEX_EXPECTS(kb >= 1 && rows >= 1 && k >= 1, "certex: sizes must be positive");
+  const bool fine     = fine_groups(kb, rows, k);
+  const LabelSample s = sample_label(kb, (rows + kTile - 1) / kTile, k, fine);
+  out[0] = fine ? kChainRows : kGroupRows, out[1] = s.step, out[2] = s.tiles;
+}
 
 // One class of routed runs (groups of 64 rows, or with `fine` of 16): passes of at most 32 768 query slots. Returns the
 // pairs the screens kept; runs' queries whose candidate list overflowed are appended to `dense`.
@@ -1124,35 +1175,15 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
     std::vector<int> col0, seg_begin;
     r1 = r0 + plan_routed(routed, r0, r1, q_tile0, shape.panel_tiles, grid, 64, segs, col0, seg_begin);
     CERTEX_EXPECTS(r1 > r0, "certex: internal error: a label's queries do not fit one routed pass");
-    // The thresholds of a large label come from a strided sample of its tiles (its rows are sorted by norm, so the sample
-    // spans all norms; the group maxima of any subset of rows are valid): at least 1024 tiles (smaller labels take part
-    // whole: every tile left out costs survivors, and their exact scores cost more than the tile), enough tiles for
-    // 2k groups, for a sixteenth of the label, and for candidate lists that stay within half their capacity (about
-    // 1.2 k rows per sampled fraction).
     const uint32_t cap = static_cast<uint32_t>(std::max(2048, 2 * k));
     std::vector<LabelRun> heads(routed.begin() + static_cast<std::ptrdiff_t>(r0), routed.begin() + static_cast<std::ptrdiff_t>(r1));
     std::vector<int> steps(heads.size(), 1);  // the sample of a large label: every steps[r]-th tile
     for (size_t r = 0; r < heads.size(); ++r) {
-      LabelRun& h          = heads[r];
-      const int64_t nt     = (h.n_in_part + kTile - 1) / kTile;
-      const int64_t enough = (2 * static_cast<int64_t>(k) + per_tile - 1) / per_tile;
-      const int64_t by_cap = (24 * static_cast<int64_t>(k) * nt + 10 * cap - 1) / (10 * static_cast<int64_t>(cap));
-      if (kb_ > 2) {
-        // Rows of more than two K blocks: a tile costs what its MMAs cost in either pass, and the pairs a looser threshold keeps
-        // cost little beside them (the epilogue's path for them hides behind the MMAs, the candidates are ranked before a row is
-        // read). So a quarter of the label will do, with chains of 16 rows as groups: 64 labels of 15 600 rows, 768 halves,
-        // 10 000 queries, k = 100: the pass 322 -> 118 us,
-        // 153 -> 413 rows kept and 129 -> 159 scored a query, the call 2356 -> 2289 us.
-        const int64_t least = std::max({(24 * static_cast<int64_t>(k) + 10 * per_tile - 1) / (10 * per_tile), enough, (nt + 3) / 4, by_cap});
-        steps[r]            = static_cast<int>(std::max<int64_t>(1, nt / least));
-        h.n_in_part         = (nt + steps[r] - 1) / steps[r] * kTile;  // tiles tile0, tile0 + step, ... to the label's end
-        continue;
-      }
-      const int64_t take   = std::min(nt, std::max({int64_t(1024), enough, (nt + 15) / 16, by_cap}));
-      if (take < nt) {
-        steps[r]    = static_cast<int>(nt / take);  // tiles tile0, tile0 + step, ... stay inside the label
-        h.n_in_part = take * kTile;
-      }
+      LabelRun& h               = heads[r];
+      const int64_t nt          = (h.n_in_part + kTile - 1) / kTile;
+      const LabelSample sampled = sample_label(kb_, nt, k, fine);
+      steps[r]                  = sampled.step;
+      if (sampled.tiles < nt) { h.n_in_part = sampled.tiles * kTile; }
     }
     std::vector<ScreenSeg> segs_g;
     std::vector<int> col0_g, seg_begin_g;
@@ -1368,6 +1399,7 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
   // thresholds of the partition's rows. With a tail longer than half the partition those would keep too much of it.
   const bool can_route = lcodes_ != nullptr && screen_kind_ != 0 && !code_overflow_ && 2 * n_tail <= n_part_ && test_mode_ != 3;
   std::vector<LabelRun> routed, routed_fine, dense;
+  int64_t largest = 0;  // rows of the largest label that is routed
   for (int i = 0; i < nq;) {
     const int32_t l = lab[order[static_cast<size_t>(i)]];
     int j           = i;
@@ -1384,15 +1416,21 @@ unsigned long long Index::search_by_labels(const Resources& res, const void* q, 
     run.queries.assign(order.begin() + i, order.begin() + j);
     // a threshold worth the passes needs about 2k groups: the k-th largest of them then sits near the best 1 % of the
     // label. Groups are 64 rows, or single chains of 16 rows for labels too small for that and for a sample of long rows.
-    const int64_t need = 2 * static_cast<int64_t>(k);
-    if (can_route && kb_ <= 2 && run.n_in_part / kGroupRows >= need) {
+    if (can_route && run.n_in_part / kChainRows >= 2 * static_cast<int64_t>(k)) {
+      largest = std::max(largest, run.n_in_part);
       routed.push_back(std::move(run));
-    } else if (can_route && run.n_in_part / kChainRows >= need) {
-      routed_fine.push_back(std::move(run));
     } else {
       dense.push_back(std::move(run));
     }
     i = j;
+  }
+  // one rule for all labels of the call as far as that goes: labels of two kinds take two sets of passes
+  if (!routed.empty()) {
+    const bool fine = fine_groups(kb_, largest, k);
+    auto is_coarse  = [&](const LabelRun& r) { return !fine && r.n_in_part / kGroupRows >= 2 * static_cast<int64_t>(k); };
+    const auto cut  = std::stable_partition(routed.begin(), routed.end(), is_coarse);
+    routed_fine.assign(std::make_move_iterator(cut), std::make_move_iterator(routed.end()));
+    routed.erase(cut, routed.end());
   }
   unsigned long long pairs = 0;
 
