@@ -24,6 +24,7 @@
 #include <map>
 #include <mutex>
 #include <ostream>
+#include <set>
 #include <vector>
 
 namespace certex_b200 {
@@ -52,16 +53,36 @@ inline int next_pow2(uint32_t v)
 // prompt, one per deduplicated block) does not pay the driver for mapping and unmapping memory each time: fifteen cudaMalloc
 // and as many cudaFree were most of such a call (a cache of 8 x 32 768 keys built, asked and dropped: 7.15 -> 1.70 ms; an index of
 // 200 000 x 96 halves built, searched 5000 times and dropped: 4.27 -> 0.97 ms). The pool keeps at most kPoolKeep bytes that no index uses: what
-// lies above goes back to the driver at the next synchronisation, and all of it when an allocation fails.
+// lies above is back with the driver when the index is gone, and all of it when an allocation fails. Mapping what it does not
+// keep costs a pool far more than it costs cudaMalloc, so arrays above kPoolMost go there. Building and dropping, ms, with all arrays
+// by cudaMalloc / all from the pool / the line at 64 / 256 / 512 MiB:
+//   10 M x 128 bytes                            9.2 / 16.1 / 7.7 / 7.9 / 7.3
+//   the same in ten additions                  31.4 / 77.2 / 15.3 / 11.5 / 23.4
+//   1 M x 768 floats, with a capacity          19.6 / 114 / 12.1 / 12.0 / 15.8
+//   the same with labels, removals, additions  27.8 / 138 / 52.4 / 16.8 / 17.3
+//   a cache of 8 x 131 072 keys, with room     13.0 / 13.9 / 19.5 / 3.5 / 15.6
+//   a cache of 8 x 32 768 keys                  4.4 / 1.0 / 1.0 / 1.0 / 1.0
+//   100 000 x 768 floats                        2.2 / 0.6 / 7.2 / 1.1 / 0.7
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+constexpr size_t kPoolMost   = size_t(256) << 20;
+
+struct IndexMemory {
+  std::mutex mutex;
+  std::map<int, cudaMemPool_t> pools;  // of the devices
+  std::set<void*> large;               // arrays by cudaMalloc
+};
+IndexMemory& index_memory()
+{
+  static IndexMemory* m = new IndexMemory;  // indexes may be dropped while the process ends
+  return *m;
+}
 
 cudaMemPool_t index_pool(int device)
 {
-  static std::mutex mutex;
-  static std::map<int, cudaMemPool_t> pools;
-  std::lock_guard<std::mutex> lock(mutex);
-  auto it = pools.find(device);
-  if (it != pools.end()) { return it->second; }
+  IndexMemory& m = index_memory();
+  std::lock_guard<std::mutex> lock(m.mutex);
+  auto it = m.pools.find(device);
+  if (it != m.pools.end()) { return it->second; }
   cudaMemPoolProps props{};
   props.allocType     = cudaMemAllocationTypePinned;
   props.handleTypes   = cudaMemHandleTypeNone;
@@ -71,7 +92,7 @@ cudaMemPool_t index_pool(int device)
   CERTEX_CUDA(cudaMemPoolCreate(&pool, &props));
   uint64_t keep = kPoolKeep;
   CERTEX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  pools[device] = pool;
+  m.pools[device] = pool;
   return pool;
 }
 
@@ -85,18 +106,25 @@ void trim_pools(int device)
   cudaMemPoolTrimTo(index_pool(device), 0);
 }
 
-/// An array of an index, for use on `stream`, and on others once the host has waited for it.
+/// An array of an index, for use on `stream`, and on others once the host has waited for it. (The index's device is current.)
 template <typename T>
 void index_alloc(T** out, size_t bytes, int device, cudaStream_t stream)
 {
-  void* p       = nullptr;
-  bytes         = std::max<size_t>(bytes, 1);
-  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, index_pool(device), stream);
+  void* p          = nullptr;
+  bytes            = std::max<size_t>(bytes, 1);
+  const bool large = bytes > kPoolMost;
+  auto take        = [&] { return large ? cudaMalloc(&p, bytes) : cudaMallocFromPoolAsync(&p, bytes, index_pool(device), stream); };
+  cudaError_t e    = take();
   if (e == cudaErrorMemoryAllocation) {
     trim_pools(device);
-    e = cudaMallocFromPoolAsync(&p, bytes, index_pool(device), stream);
+    e = take();
+    if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); }  // reported here, not by the next call
   }
   CERTEX_CUDA(e);
+  if (large) {
+    std::lock_guard<std::mutex> lock(index_memory().mutex);
+    index_memory().large.insert(p);
+  }
   *out = static_cast<T*>(p);
 }
 
@@ -112,8 +140,19 @@ void index_free(int device, const std::vector<void*>& arrays)
   if (current != device) { cudaSetDevice(device); }
   cudaDeviceSynchronize();
   for (void* p : arrays) {
-    if (p) { cudaFreeAsync(p, cudaStreamPerThread); }
+    if (!p) { continue; }
+    bool large = false;
+    {
+      std::lock_guard<std::mutex> lock(index_memory().mutex);
+      large = index_memory().large.erase(p) != 0;
+    }
+    if (large) {
+      cudaFree(p);
+    } else {
+      cudaFreeAsync(p, cudaStreamPerThread);
+    }
   }
+  cudaStreamSynchronize(cudaStreamPerThread);  // the pool gives back what it does not keep when it sees that the arrays are free
   if (current != device) { cudaSetDevice(current); }
 }
 
