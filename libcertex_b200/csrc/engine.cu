@@ -2275,9 +2275,10 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
     launch_chain_max(init_pad, 0, n_pad / kChainRows, cmax, f16, res.stream);
   }
   CERTEX_CUDA(cudaGetLastError());
-  // lists of chains, which become the caller's lists of rows
-  const uint32_t n_entries = static_cast<uint32_t>(kb > 2 ? n : (n + kChainRows - 1) / kChainRows);
-  const uint32_t chain_cap = mode == kModeScreen ? std::min(std::max<uint32_t>(cap, 2048), n_entries) : 0;
+  // lists of chains, which become the caller's lists of rows (long rows: an entry per row, the padding of the last chain included)
+  const uint32_t n_chains  = static_cast<uint32_t>((n + kChainRows - 1) / kChainRows);
+  const uint32_t n_entries = kb > 2 ? n_chains * kChainRows : n_chains;
+  uint32_t chain_cap       = mode == kModeScreen ? std::min(std::max<uint32_t>(cap, 2048), n_entries) : 0;
   Candidate* chains        = scratch.get<Candidate>(static_cast<size_t>(nq) * chain_cap);
   uint32_t* chain_cnt      = scratch.get<uint32_t>(static_cast<size_t>(nq));
   CERTEX_CUDA(cudaMemsetAsync(chain_cnt, 0, static_cast<size_t>(nq) * 4, res.stream));
@@ -2309,9 +2310,6 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   CERTEX_CUDA(cudaEventRecord(e0, res.stream));
   const cudaError_t le = screen_i8_launch(tm_q, tm_x, a, grid, res.stream);
   CERTEX_CUDA(cudaEventRecord(e1, res.stream));
-  if (mode == kModeScreen && le == cudaSuccess) {
-    launch_candidate_rows(chains, chain_cnt, chain_cap, static_cast<int>(nq), n, cnt, cand, cap, res.stream);
-  }
   int h_err = 0;
   std::vector<uint32_t> h_cnt(static_cast<size_t>(nq), 0u);
   CERTEX_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, res.stream));
@@ -2325,8 +2323,20 @@ void screen_raw(const Resources& res, const void* q_codes, int64_t nq, const voi
   CERTEX_CUDA(se);
   CERTEX_EXPECTS(h_err == 0, "certex: the screening pass gave up on a wait (code " + std::to_string(h_err) + ")");
   if (mode == kModeScreen) {
+    // The caller counts rows, so every chain must be listed: lists that ran over are made again at the length they have.
     const uint32_t most = *std::max_element(h_cnt.begin(), h_cnt.end());
-    CERTEX_EXPECTS(most <= chain_cap, "certex: a list of kept chains overflowed");
+    if (most > chain_cap) {
+      chain_cap = most;
+      a.cand    = scratch.get<Candidate>(static_cast<size_t>(nq) * chain_cap);
+      a.cap = a.ld_cand = chain_cap;
+      CERTEX_CUDA(cudaMemsetAsync(chain_cnt, 0, static_cast<size_t>(nq) * 4, res.stream));
+      CERTEX_CUDA(screen_i8_launch(tm_q, tm_x, a, grid, res.stream));
+      CERTEX_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, res.stream));
+    }
+    launch_candidate_rows(a.cand, chain_cnt, chain_cap, static_cast<int>(nq), n, cnt, cand, cap, res.stream);
+    CERTEX_CUDA(cudaGetLastError());
+    res.sync();
+    CERTEX_EXPECTS(h_err == 0, "certex: the screening pass gave up on a wait (code " + std::to_string(h_err) + ")");
   }
   if (elapsed_ms) { *elapsed_ms = ms; }
 }

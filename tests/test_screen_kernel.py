@@ -145,6 +145,17 @@ def test_staged_candidates_arrive_whole_and_at_their_own_query(share, cl):
         assert np.array_equal(np.sort(cand[i, : cnt[i]]), np.nonzero(keep[i])[0])
 
 
+@pytest.mark.parametrize("nq,n,cl", [(3, 40_007, 128), (130, 100, 384), (2, 5003, 512), (1, 9, 256)])
+def test_every_kept_row_is_counted_whatever_the_list_holds(nq, n, cl):
+    """Queries that keep all rows, with a list of the caller's that holds a few of them."""
+    q, x, init = _data(nq, n, cl, 0, seed=n)
+    init[init == NEVER] = -1
+    _, cnt, cand, _ = _run(0, q, x, init, thr=np.full(nq, -(1 << 29), np.int32), cap=5)
+    assert (cnt == n).all()
+    for i in range(nq):
+        assert len(set(cand[i].tolist())) == 5 and cand[i].min() >= 0 and cand[i].max() < n
+
+
 # ---------------------------------------------------------------------------------------------------- float16 codes
 def _run_f16(mode, hq, hx, e, thr=None, cap=64):
     """The pass on float16 code rows (code kind 2): e and thr are float32, passed as their bit patterns."""
