@@ -17,7 +17,7 @@ _HALF_KIND = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 def _as_half_or_float(x):
     """float16 on the GPU, or float32 where float16 would overflow (bf16 inputs can)."""
-    x = torch.as_tensor(x, device="cuda")
+    x = torch.as_tensor(x, device="cuda").resolve_neg()  # the kernel reads the memory as it lies there
     if x.dtype not in _HALF_KIND or not x.is_contiguous() or (x.requires_grad and torch.is_grad_enabled()):
         h = x.to(torch.float16)
         return h if bool(torch.isfinite(h).all()) else x.to(torch.float32)

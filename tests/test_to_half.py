@@ -26,3 +26,12 @@ def test_same_as_rounding_and_checking(n, offset, dtype):
     if n > 8:
         t = x[: n // 8 * 8].reshape(8, -1).t()
         assert torch.equal(_as_half_or_float(t), t.to(torch.float16))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_views_that_negate_when_they_are_read(dtype):
+    x = torch.randn((1000,), device="cuda").to(dtype)
+    v = torch._neg_view(x)
+    assert v.is_neg() and v.is_contiguous()
+    got = _as_half_or_float(v)
+    assert torch.equal(got, -x.to(torch.float16)) and not got.is_neg()
