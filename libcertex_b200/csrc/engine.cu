@@ -1373,7 +1373,7 @@ unsigned long long Index::search_routed(const Resources& res, const void* q, siz
                          q_rows_pitch, ns, 0, Candidates{cand, cnt, cap, ld_cand, n_lrows_, lperm_, linit_, shift, qq, static_cast<int32_t>(n_part_), static_cast<int32_t>(n_tail), d_slot_q}, k, plain, best_s, best_row,
                          ovf_list, d_flag, d_stats, Refine{}, res.stream, kept, from_codes ? inv_ : nullptr, sqnorm_);
     CERTEX_CUDA(cudaGetLastError());
-    st->launches += f16 ? (qq ? 7 : 6) : 5;
+    st->launches += (f16 ? (qq ? 6 : 5) : 4) + verify_launches(dtype_, static_cast<int>(dim_), k);  // queries, GROUPMAX, kth, SCREEN, verify
     unsigned int h_flag[4]        = {0, 0, 0, 0};
     unsigned long long h_stats[2] = {0, 0};
     std::vector<int32_t> h_ovf;
@@ -1715,6 +1715,7 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
       launch_gather_rows(queries, row_bytes, nullptr, nq, nq_pad, qbuf, code_pitch_, row_bytes, res.stream);
       CERTEX_CUDA(cudaGetLastError());
     }
+    local.launches += P.qq ? 2 : 1;
     int32_t* ovf_list      = scratch.get<int32_t>(static_cast<size_t>(nq));
     int32_t* thr2          = scratch.get<int32_t>(static_cast<size_t>(nq));  // tighter thresholds of the queries in ovf_list
     const int64_t batch = std::min<int64_t>(sp.batch_size, 32768);
@@ -1724,7 +1725,7 @@ Index::Pending* Index::search_begin(const Resources& res, const SearchParams& sp
       const int nb = static_cast<int>(std::min<int64_t>(batch, nq - q0));
       search_screened(res, qbuf, shift, P.qq, queries, row_bytes, static_cast<int>(q0), nb, k, best_s, best_row, ovf_list, d_count,
                       d_stats, reinterpret_cast<int*>(d_count + 1), stride, n, thr2, adm, stats_sink ? &P.events : nullptr);
-      local.launches += 5;  // gather_init, GROUPMAX, kth_largest, SCREEN, verify
+      local.launches += 4 + verify_launches(dtype_, d, k);  // gather_init, GROUPMAX, kth_largest, SCREEN, verify
     }
     // The outputs are written now, as if no list had overflowed; the counters follow them to the host and search_end
     // looks at them once the caller has enqueued what it wanted behind the search.
@@ -1824,7 +1825,7 @@ bool Index::search_end(Pending* raw, bool refinish) const
         screen_pass(res, qcodes2 + static_cast<size_t>(b0) * code_pitch_, P.thr2 + b0, queries2, P.row_bytes, b0, nb, k, best2_s,
                     best2_row, ovf2, P.d_count + 2, P.d_stats, reinterpret_cast<int*>(P.d_count + 1), n, nullptr,
                     P.shift ? shift2 : nullptr, P.qq ? qq2 : nullptr, P.adm, stats_sink ? &P.events : nullptr, nullptr);
-        local.launches += 2;
+        local.launches += 1 + verify_launches(dtype_, static_cast<int>(dim_), k);
       }
       launch_scatter_best(best2_s, best2_row, P.ovf_list, n_ovf, k, P.best_s, P.best_row, res.stream);
       launch_compose(ovf2, P.d_count + 2, n_ovf, P.ovf_list, res.stream);

@@ -2631,6 +2631,12 @@ void launch_remove(const int64_t* ids, int64_t n_ids, int64_t size, uint8_t* rem
   if (init && cmax) { chain_max_of_ids_kernel<<<grid, 256, 0, s>>>(ids, n_ids, size, inv, init, cmax, is_float ? 1 : 0); }
 }
 
+int verify_launches(int dtype, int d, int k)
+{
+  const bool bytes = dtype == kI8 || dtype == kU8;
+  return k > kSplitK || (!bytes && k > 32 && static_cast<size_t>(d) * dtype_size(dtype) >= kLongRow) ? 3 : 1;
+}
+
 void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, int metric, const void* queries,
                           size_t qpitch, int nq, int q0, const Candidates& cd, int k,
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
@@ -2639,7 +2645,7 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
   if (nq <= 0) { return; }
   const int n2max  = cd.ld;
   const bool bytes = dtype == kI8 || dtype == kU8;  // 8-bit rows rank 64-bit keys
-  const bool split = k > kSplitK || (!bytes && k > 32 && static_cast<size_t>(d) * dtype_size(dtype) >= kLongRow);
+  const bool split = verify_launches(dtype, d, k) > 1;
   const size_t q_bytes = bytes ? static_cast<size_t>((d + 15) / 16 * 16) : sizeof(double) * static_cast<size_t>(d);
   const size_t pairs   = (sizeof(double) + sizeof(int32_t)) * static_cast<size_t>(n2max);
   // float rows: one staging tile per warp, + 16 bytes of alignment

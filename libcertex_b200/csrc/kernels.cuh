@@ -187,6 +187,8 @@ void launch_verify_select(const void* vectors, size_t pitch, int dtype, int d, i
                           Admit adm, double* best_s, int32_t* best_row, int32_t* ovf_list, unsigned int* ovf_count,
                           unsigned long long* stats, Refine rf, cudaStream_t s, int32_t* kept, const int32_t* where = nullptr,
                           const double* sqnorm = nullptr);
+/// Its launches: one, or three.
+int verify_launches(int dtype, int d, int k);
 
 /// out[r] = |x_r|^2 of n float32 / float16 rows, summed over the coordinates in order in fp64 with every product and sum
 /// rounded on its own: the sum the cosine verification makes per candidate. With it (sqnorm of launch_verify_select,
