@@ -173,7 +173,8 @@ CERTEX_B200_EXPORT cuvsError_t cuvsCertexSetLabels(cuvsResources_t res, DLManage
                                                    cuvsCertexIndex_t index);
 /** certex.h:164: groups the ids by label and, when the index has a tensor-core screen, copies the code rows in label
  *  order, so that searches by label screen and score only the rows of the query's label. Speed only: results are the
- *  same with or without it. Vectors added later are found too (scored densely) until the next call. */
+ *  same with or without it. Vectors added later are found too until the next call: they are screened one by one against the queries of
+ *  their label, or, once they are more than half of what the partition holds, every label is scored densely. */
 CERTEX_B200_EXPORT cuvsError_t cuvsCertexPartitionByLabels(cuvsResources_t res, cuvsCertexIndex_t index);
 
 /** certex.h:184-190: exact k nearest neighbours, k = neighbors.shape[1]. queries [nq, dim] (device, index dtype),

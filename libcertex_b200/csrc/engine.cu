@@ -244,7 +244,7 @@ struct ScreenShape {
 /// Shared memory of the resident-panel variant: panel_tiles * kb * 16 KB + n_stages * (kb * 32 KB + 1 KB) + the rest
 /// (screen_smem_bytes). The panel is what the call's query tiles split into evenly, at most 7 (kb = 1) or 2 (kb = 2) tiles;
 /// what it leaves goes to stages: a short panel is done with a stored tile soon, and the tiles in flight are what keeps
-/// the memory busy (one query over 1 M rows of 128 bytes, a call: 158 us with 2 stages, 157 with 3, 153 with 6). Rows of more than two K blocks stream their K blocks
+/// the memory busy (one query over 1 M rows of 128 bytes, a call: 147 us with 2 stages, 143 with 3 to 5, which is what fits). Rows of more than two K blocks stream their K blocks
 /// (two query tiles per segment, stages fixed by the kernel).
 ScreenShape shape_for(int kb, int nqt)
 {

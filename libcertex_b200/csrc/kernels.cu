@@ -447,13 +447,15 @@ __global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v)
 // All sums are fp64. maxima[0..2] collect the largest |h|, |y - h| and |e| as float bits (non-negative floats order
 // like their bits); maxima[3] is raised when a coordinate does not fit fp16.
 //
-// Bound by memory (the row in, its code out). The blocks are as many as fit the GPU at once and walk the rows in a grid
-// stride, and a lane keeps the largest squared norms it has seen (a norm rounds up monotonically in its square), so that
+// Bound by memory (the row in, its code out). The blocks are few enough to walk the rows in a grid stride of many turns, and a lane keeps the largest squared norms it has seen (a norm rounds up monotonically in its square), so that
 // a block touches the three counters once: an atomic per row on the same three words held the whole pass at their rate
 // (262 144 rows of 128 halves: 534 us, 0.25 TB/s; now 43 us, 3.1 TB/s). 16-byte loads; a row is split over 8 lanes when that leaves a lane at
 // most four of them, so that short rows do not leave most of a warp without a coordinate, else over the whole warp.
 constexpr int kEncodeThreads = 256;
-constexpr int kEncodeBlocks  = 148 * 8;  // what is resident at once
+// Two turns of the blocks that an SM holds (4 of 58 registers a thread for halves, 5 of 48 for floats). Us at 4 / 5 / 8 / 10 blocks
+// an SM: 262 144 x 128 halves 44 / 55 / 44 / 46, 1 M x 768 halves 858 / 1042 / 850 / 877, 1 M x 768 floats (cosine) 1083 / 1039 /
+// 1026 / 1005, 1 M x 128 floats 199 / 181 / 201 / 180.
+constexpr int kEncodeBlocks  = 148 * 8;
 template <typename T, int G>
 __global__ void __launch_bounds__(kEncodeThreads) encode_f16_rows_kernel(const uint8_t* vectors, size_t pitch, int d, int metric,
                                                                          int64_t n, uint8_t* codes, size_t code_pitch, float* e,

@@ -229,7 +229,7 @@ class Index:
                 # The partition (ids grouped by label and a label-ordered copy of the screen's rows) is renewed with
                 # every labeled addition: it costs a sort of the labels and one copy of the code rows.
                 # partition_labels="lazy" keeps the reference's rule instead (certex/index.py:306-311): renew once an
-                # eighth of the vectors is newer than the partition; until then the newer vectors are scored densely.
+                # eighth of the vectors is newer than the partition; until then the newer vectors are screened one by one.
                 i = self.core.info()
                 lazy = self.partition_labels == "lazy"
                 if self.partition_labels and (not lazy or 8 * (int(i.size) - int(i.n_partitioned)) > int(i.size)):

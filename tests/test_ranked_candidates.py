@@ -1,6 +1,6 @@
 """The candidates of a screen are ranked by the products it leaves before any is scored exactly. Cases where the ranking is
 tight or worthless: many equal rows around the k-th place, chains of 16 rows that are kept whole, rows removed or filtered out
-inside kept chains, lists on both sides of the size that one warp ranks, and more kept rows than a list of rows holds."""
+inside kept chains, and lists on both sides of the size that one warp ranks."""
 
 import numpy as np
 import pytest
