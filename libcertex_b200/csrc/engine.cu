@@ -663,7 +663,7 @@ void Index::extend(const Resources& res, const void* rows, int64_t n, bool on_ho
     } else {
       launch_row_init(from, pitch_, dtype_, static_cast<int>(dim_), kL2, nullptr, 0, m, m, e, res.stream);
     }
-    if (a < size_ && n_removed_ > 0) { launch_mask_removed(e, removed_ + a, size_ - a, f16, res.stream); }
+    if (a < size_ && any_removed_) { launch_mask_removed(e, removed_ + a, size_ - a, f16, res.stream); }
     CERTEX_CUDA(cudaGetLastError());
     launch_sort_batch(e, m, static_cast<int32_t>(a), a, src, src_id0, code_pitch_, params_.metric, f16, keys_in, keys_out,
                       ids_in, ids_out, temp, tb, codes_, perm_, inv_, init_, res.stream);
@@ -703,6 +703,7 @@ void Index::remove(const Resources& res, const int64_t* ids_device, int64_t n_id
   res.sync();
   std::unique_lock<ReaderGate> lock(rw_);
   n_removed_ += static_cast<int64_t>(n_new);
+  any_removed_ |= n_new > 0;
 }
 
 void Index::set_labels(const Resources& res, const int32_t* labels_device, int64_t n, int64_t first)
@@ -2102,7 +2103,8 @@ std::unique_ptr<Index> Index::from_blocks(const Resources& res, const IndexParam
     CERTEX_CUDA(cudaMemcpyAsync(idx->removed_, host.data(), static_cast<size_t>(n), cudaMemcpyHostToDevice, res.stream));
     res.sync();
     idx->n_removed_ = n_rem;
-    if (idx->screen_kind_ && std::any_of(host.begin(), host.begin() + n, [](char f) { return f != 0; })) {
+    idx->any_removed_ = std::any_of(host.begin(), host.begin() + n, [](char f) { return f != 0; });
+    if (idx->screen_kind_ && idx->any_removed_) {
       // removed rows must never pass the screen
       Scratch scratch(res.stream);
       int64_t* ids     = scratch.get<int64_t>(static_cast<size_t>(n));

@@ -307,6 +307,7 @@ class Index {
   int64_t size_       = 0;
   int64_t capacity_   = 0;
   int64_t n_removed_  = 0;
+  bool any_removed_   = false;  // a removal flag is set, also where a file's count says 0 (saved while rows were being removed)
   bool has_labels_    = false;
   bool host_vectors_  = false;    // vectors_ is page-locked host memory that the GPU reads in place (index_params.host_vectors)
   void* vectors_      = nullptr;  // [capacity, pitch]

@@ -371,7 +371,7 @@ def test_removed_rows_exceeding_k_leave_missing_entries():
     assert (I[:, 4:] == -1).all() and (I[:, :4] >= 60).all() and np.isinf(D[:, 4:]).all()
 
 
-def _write_reference_file(path, x, metric_code, removed, labels, int8_rows, width=27, stride=16):
+def _write_reference_file(path, x, metric_code, removed, labels, int8_rows, width=27, stride=16, n_removed=None):
     """A file in the layout the reference's serialize writes (cpp/src/neighbors/certex/certex_serialize.cu:40-132):
     the 4-byte dtype prefix, then one .npy record per scalar and array, in its order. The projection, certificate rows
     and anchors hold filler values: they are the reference's own screening data."""
@@ -386,7 +386,8 @@ def _write_reference_file(path, x, metric_code, removed, labels, int8_rows, widt
 
         f.write(prefix)
         put(0x43455258, np.int32), put(1, np.int32), put(metric_code, np.int32), put(d, np.int64), put(width, np.int32)
-        put(stride, np.int32), put(0, np.int32), put(n, np.int64), put(int(removed.sum()), np.int64)
+        put(stride, np.int32), put(0, np.int32), put(n, np.int64)
+        put(int(removed.sum()) if n_removed is None else n_removed, np.int64)
         put(0 if labels is None else 1, np.int32), put(1 if int8_rows else 0, np.int32)
         for v in (0.5, 1.0, 2.0, 3.0, 4.0, 5.0):  # alpha and the certificate maxima
             put(v, np.float64)
@@ -425,3 +426,20 @@ def test_load_a_file_in_the_reference_layout(tmp_path, dtype, metric, int8_rows,
         f.write(np.int32(3).tobytes())
     with pytest.raises(Exception, match="lists"):
         certex.Index.load(path)
+
+
+@pytest.mark.parametrize("dtype", ["uint8", "float32"])
+def test_flags_count_where_a_file_says_that_nothing_was_removed(tmp_path, dtype):
+    """A file that was written while rows were being removed holds their flags and an older count. The rows stay away, also
+    once an addition has sorted them again together with the new ones."""
+    x, q = data(9000, 40, 50, dtype, seed=2)
+    removed = np.zeros(5000, dtype=bool)
+    removed[oracle.knn(x[:5000], q, 3, "l2")[0].ravel()] = True
+    path = tmp_path / "flags.bin"
+    _write_reference_file(path, x[:5000], 0, removed, None, False, n_removed=0)
+    index = certex.Index.load(path)
+    same(index, x[:5000], q, 5, keep_row=~removed)
+    index.add(x[5000:])
+    with certex.search_stats() as st:
+        same(index, x, q, 5, keep_row=np.concatenate([~removed, np.ones(4000, dtype=bool)]))
+    assert st.dense_queries == 0
