@@ -586,7 +586,10 @@ __global__ void __launch_bounds__(kThreads, 1) screen_i8_kernel(const __grid_con
     // until the slot is released, and the release follows tcgen05.wait::ld directly (it is warp-wide: when lane 0 is
     // past it, every lane's columns are in registers).
     const uint32_t tfull_bar0 = smem_u32(&ctl->tmem_full[0]), tempty_bar0 = smem_u32(&ctl->tmem_empty[0]);
-    const int never_thr       = F16 ? __float_as_int(CUDART_INF_F) : 0x7fffffff;  // float bits when F16
+    // The threshold of a lane without a query: 2^31 - 1, which no product reaches, or NaN, which no comparison holds for. (Not
+    // infinity: behind the queries of a batch that fills no tile lie the codes of the next batch, and a coordinate of theirs
+    // beyond the fp16 range makes infinite products. What they kept would be written past the end of the batch's lists.)
+    const int never_thr       = 0x7fffffff;
     constexpr int kERingOrNs  = WIDE ? kERing : 0;
     int est = 0;            // GROUPMAX: ring position of the tile's e values and its parity
     uint32_t est_par = 0;
