@@ -1717,14 +1717,27 @@ verify_select_kernel(const uint8_t* vectors, size_t pitch, int d, const void* qu
   }
 }
 
+// Sorts m entries in shared memory by (score, id): not inlined, it would cost the kernels registers that their usual path needs
+// (sort_lists_kernel 64 -> 74 and a block per SM less, select_topk_kernel 2 - 4 % slower on plain scores).
+constexpr int kSortCompares = 2048;
+__device__ __noinline__ void sort_crowded(double* s, int32_t* id, int m)
+{
+  const int n2 = next_pow2(m);
+  for (int i = m + threadIdx.x; i < n2; i += blockDim.x) { s[i] = CUDART_INF, id[i] = 0x7fffffff; }
+  bitonic_sort(s, id, n2);
+}
+
 // Every thread of a block of NT: the m entries (score, id) that the threads hold (HELD each: entry threadIdx.x + i NT) in the
 // order of (score, id): emit(place, score, id) for the first k places. The scores are spread over 4 NT intervals, the buckets
 // are laid out one after the other in shared memory, and an entry's place is the beginning of its bucket plus the entries of
 // the bucket that come before it. The intervals grow with the distance from the worst score (NT / 4 per octave, 16 octaves):
 // the k best of a large set crowd at that end, the more so when a few are far better than the rest. A bitonic sort of 4096
 // pairs moves 12 bytes an entry 78 times through shared memory, which bounds it: 217 us for 512 lists of 2400 entries; this one
-// takes 44 us. (With most scores in one interval an entry is compared with all others, which is as slow as the bitonic
-// sort.) Shared memory: s [m] | id [m] | start [4 NT + 1], start 16-byte aligned.
+// takes 44 us. An entry is compared with those of its interval, about 45 cycles each: where scores crowd (ties, or a spread
+// of more than 16 octaves) so that a thread would make more than kSortCompares of them, the bitonic sort is what is left (a search
+// of 200 queries that scores 5000 rows, k = 2048, all scores equal: 465 us by comparisons, 142 with this rule; all but five in one
+// far cluster 470 and 155).
+// Shared memory: s and id [next_pow2(m)] each | start [4 NT + 1], start 16-byte aligned.
 template <int NT, int HELD, typename Emit>
 __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], int m, int k, double* s, int32_t* id, int32_t* start,
                            Emit&& emit)
@@ -1734,7 +1747,7 @@ __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], i
   static_assert(B == 4096 || B == 1024, "16 octaves");
   constexpr int W = NT / 32;
   __shared__ double s_lo[W], s_hi[W];
-  __shared__ int s_sum[W];
+  __shared__ int s_sum[W], s_work[W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double lo = CUDART_INF, hi = -CUDART_INF;
 #pragma unroll
@@ -1783,7 +1796,8 @@ __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], i
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) { incl += v; }
   }
-  if (lane == 31) { s_sum[warp] = incl; }
+  const int work = __reduce_add_sync(0xffffffffu, c.x * c.x + c.y * c.y + c.z * c.z + c.w * c.w);  // at most m^2 in all
+  if (lane == 31) { s_sum[warp] = incl, s_work[warp] = work; }
   __syncthreads();
   int before = incl - sum;
   for (int w = 0; w < warp; ++w) { before += s_sum[w]; }
@@ -1799,6 +1813,13 @@ __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], i
     }
   }
   __syncthreads();
+  int compares = 0;
+  for (int w = 0; w < W; ++w) { compares += s_work[w]; }
+  if (compares > kSortCompares * NT) {
+    sort_crowded(s, id, m);
+    for (int i = threadIdx.x; i < min(m, k); i += NT) { emit(i, s[i], id[i]); }
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < HELD; ++i) {
     if (b[i] >= 0) {
@@ -1814,7 +1835,7 @@ __device__ void sort_block(const double (&x)[HELD], const int32_t (&xi)[HELD], i
 
 // The third step of a split verification, block per query: its k best by (score, id).
 template <typename T, int METRIC, int NT, int HELD>  // lists of at most NT HELD rows
-__global__ void __launch_bounds__(NT) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 1) sort_lists_kernel(const void* queries, size_t qpitch, int d, int q0, Candidates cd,
                                                                   int n2max, int k, double* best_s, int32_t* best_row,
                                                                   int32_t* ovf_list, unsigned int* ovf_count, Refine rf,
                                                                   const int32_t* kept)
@@ -2097,8 +2118,10 @@ __global__ void group_columns_to_ids_kernel(int32_t* best_row, int k, const int3
 // Bound by reading the row: once for its smallest and largest key, once for a histogram of 2048 intervals between them, once to
 // take the winners and the rows of the interval that holds the k-th, whose last places are given by counting. (A walk over fixed
 // 8-bit digits reads the row nine times, and its counters wait for one another: in the upper digits the scores of a row
-// are alike. 352 rows of 14 775 scores on average, k = 2048: 368 us; this one 99 us.) When the interval holds more than kPool rows
-// it is divided again; scores that are all equal go to the smallest rows.
+// are alike. 352 rows of 14 775 scores on average, k = 2048: 368 us; this one 99 us.) When the interval holds more than kPool rows,
+// or so many that counting their places takes longer than reading the row once more (200 rows of 5000 scores over 15 orders of
+// magnitude, k = 2048: 405 us a call with up to kPool in any case, 163 with both rules), it is divided again; scores that are all
+// equal go to the smallest rows.
 // Shared memory: sel_s [kk] doubles | sel_id [kk] int32 | pool_s [kPool] doubles | pool_id [kPool] int32 | bins, and after them
 // the sort's buckets; kk = k rounded up to a multiple of 4.
 // With `row_off` the score rows are ragged: row blockIdx.x starts at scores + row_off[blockIdx.x] and has row_n[] columns.
@@ -2162,6 +2185,7 @@ __global__ void __launch_bounds__(NT) select_topk_kernel(const double* scores, i
     // the interval [prefix << shift, (prefix + 1) << shift) of key - lo that holds the last winner
     int above = 64 - __clzll(static_cast<long long>(hi - lo));  // bits of key - lo above which nothing differs
     int shift = max(above - 11, 0), in_bin = 0, remaining = want;
+    bool pooled = false;
     u64 prefix = 0;
     while (true) {
       const u64 inside = (1ull << (above - shift)) - 1;  // 11 bits, or what is left
@@ -2206,12 +2230,12 @@ __global__ void __launch_bounds__(NT) select_topk_kernel(const double* scores, i
       prefix = (prefix << (above - shift)) + static_cast<u64>(s_bin);
       remaining -= s_before;
       in_bin = s_in_bin;
-      if (in_bin <= kPool || shift == 0) { break; }
+      pooled = in_bin <= kPool && static_cast<int64_t>(in_bin) * in_bin <= 4 * n + 64 * NT;
+      if (pooled || shift == 0) { break; }
       above = shift;
       shift = max(shift - 11, 0);
     }
     const int n_less = want - remaining;
-    const bool pooled = in_bin <= kPool;
     for (int64_t i0 = 0; i0 < n; i0 += NT) {
       const int64_t i = i0 + threadIdx.x;
       const double v  = i < n ? row[i] : CUDART_INF;
